@@ -15,17 +15,20 @@
 //                          4-byte offset) and the warp moves its bytes, 32 at
 //                          a time (copies whose source overlaps their output
 //                          go in steps of the offset);
-//   parquet_pages_kernel   one CTA per page: thread 0 skips (and checks) the
-//                          definition levels, walks byte-array lengths (data
-//                          and dictionary pages) and reads the dictionary
-//                          indices' run headers, up to 256 a round, and every
-//                          thread then decodes the round's indices, a
-//                          fixed-width column's straight into its values;
+//   parquet_pages_kernel   one CTA per 8,192 values of a page: thread 0 skips
+//                          (and checks) the definition levels, walks
+//                          byte-array lengths (data and dictionary pages) and
+//                          reads the dictionary indices' run headers, up to
+//                          256 a round, and every thread then decodes the
+//                          round's indices that lie in the CTA's part of the
+//                          page, a fixed-width column's straight into its
+//                          values;
 //   parquet_values_kernel  per plain data page and value: fixed-width values
 //                          copied into the output column; byte arrays (plain
 //                          or dictionary-encoded) get their source and
 //                          length;
 //   then per utf8 column a prefix sum of the lengths and a byte copy.
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -203,25 +206,45 @@ __device__ __forceinline__ void copy_value(const uint8_t* src, uint8_t* dst, int
 
 constexpr int kPqThreads = 256;
 constexpr int kPqRuns = 256;  // run headers read per round
+// Dictionary indices of a page that one CTA decodes: 32 per thread. One CTA
+// per page left most SMs without a warp (a 4M-row, 7-column file of
+// 131,072-row pages is 237 pages; the pass took 460 us at 12% occupancy) and
+// the longest page set its length; with parts, word-wide index reads and one
+// copy per span of chunks the whole read of that file went from 1,118 to 680 us.
+constexpr int kPqPart = 8192;
 
-// One CTA per page. Thread 0 does the sequential parts (definition levels,
-// byte-array lengths, run headers); the dictionary indices of each round of
-// up to kPqRuns runs are then decoded by every thread, a value finding its
-// run by binary search over the runs' first values. A fixed-width column's
+struct PagePart {
+  int32_t page;
+  int32_t first;  // the part's first value in the page
+};
+
+// One CTA per part of a page: kPqPart consecutive values where the page
+// holds dictionary indices, the whole of any other page. Thread 0
+// does the sequential parts (definition levels, byte-array lengths, run
+// headers, which every part of a page walks for itself up to its own end);
+// the dictionary indices of each round of up to kPqRuns runs that lie in the
+// part are then decoded by every thread, a value finding its run by binary
+// search over the runs' first values. A fixed-width column's
 // index is looked up in its dictionary page at once and the value written
 // to the output column (the dictionary page's body is read as the host laid
 // it out, not through fields another CTA of this launch sets); a byte-array
 // column's index is kept for parquet_values_kernel, which runs after the
 // dictionary pages' entries are known.
-__global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* pages, int32_t n_pages, DictArrays dicts,
-                                                                   DevStatus* st) {
+__global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* pages, int32_t n_pages,
+                                                                   const PagePart* __restrict__ items, int64_t n_items,
+                                                                   DictArrays dicts, DevStatus* st) {
   __shared__ int32_t s_first[kPqRuns + 1];  // the page value index each run starts at; then the round's end
   __shared__ int32_t s_start[kPqRuns];      // bit-packed runs: first byte; RLE runs: -1
   __shared__ uint32_t s_value[kPqRuns];     // RLE runs: the value
-  __shared__ int32_t s_n, s_ok, s_at, s_done, s_bw;
-  for (int64_t w = blockIdx.x; w < n_pages; w += gridDim.x) {
-    __syncthreads();  // the previous page's shared state is no longer read
+  __shared__ int32_t s_n, s_ok, s_at, s_done, s_bw, s_blen;
+  __shared__ const uint8_t* s_base;
+  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    __syncthreads();  // the previous part's shared state is no longer read
+    const int32_t w = items[item].page;
     PageDev& pg = pages[w];
+    const int32_t part_lo = items[item].first;
+    const int32_t num_values = pg.num_values;
+    const int32_t part_hi = num_values - part_lo < kPqPart ? num_values : part_lo + kPqPart;
     const uint8_t* base;
     int32_t blen;
     if (pg.snappy) {
@@ -274,11 +297,16 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
             blen -= 4 + len;
           }
         }
-        if (!ok) raise_status(st, GFPDB_EUNSUPPORTED, 200000 + static_cast<int32_t>(w));  // nulls, or bad levels
+        if (!ok) raise_status(st, GFPDB_EUNSUPPORTED, 200000 + w);  // nulls, or bad levels
       }
+      s_base = base;
+      s_blen = blen;
       if (ok) {
-        pg.values = base;
-        pg.values_len = blen;
+        if (part_lo == 0) {  // for parquet_values_kernel
+          pg.values = base;
+          pg.values_len = blen;
+        }
+        // (a page walked or checked here has one part)
         const bool bytes_walk = pg.width == 0 && (pg.type == parquet::PAGE_DICTIONARY || pg.encoding == parquet::ENC_PLAIN);
         if (bytes_walk) {  // byte arrays: each value's address and length
           const bool dict = pg.type == parquet::PAGE_DICTIONARY;
@@ -290,7 +318,7 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
               at += 4;
             }
             if (len < 0 || len > blen - at) {
-              raise_status(st, GFPDB_EINVAL, (dict ? 300000 : 400000) + static_cast<int32_t>(w));
+              raise_status(st, GFPDB_EINVAL, (dict ? 300000 : 400000) + w);
               ok = 0;
               break;
             }
@@ -305,14 +333,14 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
           }
         } else if (pg.width > 0 && (pg.type == parquet::PAGE_DICTIONARY || pg.encoding == parquet::ENC_PLAIN) &&
                    static_cast<int64_t>(pg.num_values) * pg.width > blen) {
-          raise_status(st, GFPDB_EINVAL, 400000 + static_cast<int32_t>(w));
+          raise_status(st, GFPDB_EINVAL, 400000 + w);
           ok = 0;
         }
       }
       const bool indices = ok && pg.type != parquet::PAGE_DICTIONARY && pg.encoding != parquet::ENC_PLAIN;
       s_bw = blen > 0 ? base[0] : 99;
       if (indices && (s_bw > 32 || pg.dict_page < 0 || pg.dict_page >= n_pages)) {
-        raise_status(st, GFPDB_EINVAL, 500000 + static_cast<int32_t>(w));
+        raise_status(st, GFPDB_EINVAL, 500000 + w);
         ok = 0;
       }
       s_ok = indices ? ok : 0;
@@ -322,16 +350,20 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
     __syncthreads();
     if (!s_ok) continue;
     // Dictionary indices: a bit-width byte, then RLE / bit-packed hybrid runs.
-    base = pg.values;
-    blen = pg.values_len;
+    base = s_base;
+    blen = s_blen;
     const int32_t bw = s_bw;
-    const uint64_t mask = bw == 32 ? 0xffffffffull : ((1ull << bw) - 1ull);
+    const uint32_t mask = bw == 32 ? 0xffffffffu : ((1u << bw) - 1u);
+    const int32_t width = pg.width;
+    const int64_t first_row = pg.first_row;
+    uint8_t* const fixed_out = pg.fixed_out;
+    int32_t* const idx_out = pg.idx;
     // a fixed-width column's dictionary: its page's values as laid out on
     // the host (dictionary pages carry no levels), its entry count and bytes
     const uint8_t* dvals = nullptr;
     int64_t dlen = 0;
     int32_t dn = 0;
-    if (pg.width > 0) {
+    if (width > 0) {
       const PageDev& dp = pages[pg.dict_page];
       dvals = dp.snappy ? dp.inflated : dp.body;
       dlen = dp.snappy ? dp.inflated_len : dp.body_len;
@@ -340,7 +372,7 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
     for (;;) {
       if (threadIdx.x == 0) {
         int32_t n = 0, at = s_at, done = s_done;
-        while (n < kPqRuns && done < pg.num_values) {
+        while (n < kPqRuns && done < part_hi) {
           uint32_t h;
           if (!run_header(base, blen, &at, &h)) {
             s_ok = 0;
@@ -374,19 +406,19 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
             break;
           }
           s_first[n] = done;
-          done += static_cast<int32_t>(count < pg.num_values - done ? count : pg.num_values - done);
-          ++n;
+          done += static_cast<int32_t>(count < num_values - done ? count : num_values - done);
+          if (done > part_lo) ++n;  // a run wholly before the part is passed over
         }
         s_first[n] = done;
         s_n = s_ok ? n : 0;
         s_at = at;
         s_done = done;
-        if (!s_ok) raise_status(st, GFPDB_EINVAL, 500000 + static_cast<int32_t>(w));
+        if (!s_ok) raise_status(st, GFPDB_EINVAL, 500000 + w);
       }
       __syncthreads();
       const int32_t n = s_n;
       if (n == 0) break;
-      const int32_t v0 = s_first[0], v1 = s_first[n];
+      const int32_t v0 = s_first[0] > part_lo ? s_first[0] : part_lo, v1 = s_first[n] < part_hi ? s_first[n] : part_hi;
       // unrolled so that several values' loads are in flight together
 #pragma unroll 4
       for (int32_t v = v0 + static_cast<int32_t>(threadIdx.x); v < v1; v += kPqThreads) {
@@ -400,30 +432,37 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
         if (s_start[lo] < 0) {
           idx = s_value[lo];
         } else {
+          // the value's bits from the two aligned words around them (32 bits
+          // at most; the buffers start 16-byte aligned and carry 16 bytes of
+          // tail padding)
           const int64_t bit = static_cast<int64_t>(v - s_first[lo]) * bw;
-          const uint8_t* q = base + s_start[lo] + (bit >> 3);
-          uint64_t x = 0;
-          const int nb = (static_cast<int>(bit & 7) + bw + 7) / 8;  // bytes the value spans (within the run)
-          for (int k = 0; k < nb; ++k) x |= static_cast<uint64_t>(__ldg(q + k)) << (8 * k);
-          idx = static_cast<uint32_t>((x >> (bit & 7)) & mask);
+          const uintptr_t q = reinterpret_cast<uintptr_t>(base + s_start[lo]) + static_cast<uintptr_t>(bit >> 3);
+          const uint32_t* al = reinterpret_cast<const uint32_t*>(q & ~uintptr_t{3});
+          const uint32_t sh = 8u * static_cast<uint32_t>(q & 3u) + static_cast<uint32_t>(bit & 7);
+          idx = __funnelshift_r(__ldg(al), __ldg(al + 1), sh) & mask;
         }
-        if (pg.width > 0) {
-          if (idx >= static_cast<uint32_t>(dn) || (static_cast<int64_t>(idx) + 1) * pg.width > dlen) {
-            raise_status(st, GFPDB_EINVAL, 600000 + static_cast<int32_t>(w));
+        if (width > 0) {
+          if (idx >= static_cast<uint32_t>(dn) || (static_cast<int64_t>(idx) + 1) * width > dlen) {
+            raise_status(st, GFPDB_EINVAL, 600000 + w);
             continue;
           }
           // the value's 4-byte words from the two aligned words around each
           // (the arena and the inflated buffer carry 16 bytes of tail padding)
-          const uint8_t* sp = dvals + static_cast<int64_t>(idx) * pg.width;
+          const uint8_t* sp = dvals + static_cast<int64_t>(idx) * width;
           const uint32_t* al = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(sp) & ~uintptr_t{3});
           const uint32_t sh = 8u * static_cast<uint32_t>(reinterpret_cast<uintptr_t>(sp) & 3u);
-          uint32_t* dw = reinterpret_cast<uint32_t*>(pg.fixed_out + (pg.first_row + v) * pg.width);
-          for (int k = 0; k < pg.width / 4; ++k) dw[k] = __funnelshift_r(__ldg(al + k), __ldg(al + k + 1), sh);
+          const uint32_t w0 = __ldg(al), w1 = __ldg(al + 1);
+          if (width == 4) {
+            reinterpret_cast<uint32_t*>(fixed_out)[first_row + v] = __funnelshift_r(w0, w1, sh);
+          } else {
+            const uint2 d = make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, __ldg(al + 2), sh));
+            reinterpret_cast<uint2*>(fixed_out)[first_row + v] = d;
+          }
         } else {
-          pg.idx[pg.first_row + v] = static_cast<int32_t>(idx);
+          idx_out[first_row + v] = static_cast<int32_t>(idx);
         }
       }
-      const bool more = s_done < pg.num_values;
+      const bool more = s_done < part_hi;
       __syncthreads();  // the runs are read before thread 0 rewrites them
       if (!more) break;
     }
@@ -478,6 +517,8 @@ __global__ void parquet_bytes_kernel(const uint64_t* __restrict__ ptr, const int
   }
 }
 
+constexpr int64_t kPqCopyGap = 64 * 1024;
+
 int grid_parquet(int64_t n) {
   int64_t b = (n + 255) / 256;
   const int64_t cap = static_cast<int64_t>(num_sms()) * 8;
@@ -494,16 +535,26 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   if (rows > INT32_MAX) fail(GFPDB_EUNSUPPORTED, "a Parquet read of more than 2^31 - 1 rows");
   const int nc = static_cast<int>(L.columns.size());
 
-  // the column chunks' bytes on the device, one copy each
+  // the column chunks' bytes on the device: chunks that follow each other in
+  // the file with at most kPqCopyGap bytes between them share one copy (a
+  // copy costs about 3 us besides its bytes)
+  struct Span {
+    int64_t begin, end, at;  // file bytes [begin, end) at byte `at` of the arena
+  };
+  std::vector<Span> spans;
   std::vector<int64_t> chunk_at(L.chunks.size());
   int64_t arena_bytes = 0;
   for (size_t c = 0; c < L.chunks.size(); ++c) {
-    chunk_at[c] = arena_bytes;
-    arena_bytes += (L.chunks[c].end - L.chunks[c].begin + 15) / 16 * 16;
+    const auto& ch = L.chunks[c];
+    if (!spans.empty() && ch.begin >= spans.back().end && ch.begin - spans.back().end <= kPqCopyGap)
+      spans.back().end = ch.end;
+    else
+      spans.push_back(Span{ch.begin, ch.end, arena_bytes});
+    chunk_at[c] = spans.back().at + (ch.begin - spans.back().begin);
+    arena_bytes = (chunk_at[c] + (ch.end - ch.begin) + 15) / 16 * 16;
   }
   auto arena = make_buffer(arena_bytes + 16, s);  // tail padding: 4-byte word reads past a value's end
-  for (size_t c = 0; c < L.chunks.size(); ++c)
-    copy_h2d(arena->as<uint8_t>() + chunk_at[c], file + L.chunks[c].begin, L.chunks[c].end - L.chunks[c].begin, s);
+  for (const Span& sp : spans) copy_h2d(arena->as<uint8_t>() + sp.at, file + sp.begin, sp.end - sp.begin, s);
 
   // per-column outputs and working arrays
   std::vector<BufferPtr> fixed(nc), row_ptr(nc), row_len(nc), idx(nc);
@@ -523,7 +574,7 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
 
   // page descriptors
   std::vector<PageDev> pd(L.pages.size());
-  std::vector<int32_t> snappy_list, data_list;
+  std::vector<int32_t> snappy_list, data_list, item_list;  // item_list: (page, first value) pairs
   int64_t inflate_bytes = 0, dict_entries = 0;
   std::vector<int64_t> inflate_at(L.pages.size(), -1);
   for (size_t p = 0; p < L.pages.size(); ++p) {
@@ -543,6 +594,11 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
     // values in the page pass)
     const bool fixed_dict = L.columns[pg.column].dtype != DType::Utf8 && pg.encoding != parquet::ENC_PLAIN;
     if (pg.type != parquet::PAGE_DICTIONARY && !fixed_dict) data_list.push_back(static_cast<int32_t>(p));
+    const bool indices = pg.type != parquet::PAGE_DICTIONARY && pg.encoding != parquet::ENC_PLAIN;
+    for (int64_t first = 0; first == 0 || (indices && first < pg.num_values); first += kPqPart) {
+      item_list.push_back(static_cast<int32_t>(p));
+      item_list.push_back(static_cast<int32_t>(first));
+    }
   }
   auto inflated = make_buffer(inflate_bytes + 16, s);
   for (size_t p = 0; p < L.pages.size(); ++p) {
@@ -585,15 +641,17 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   DevStatus* st = status->as<DevStatus>();
   const int64_t np = static_cast<int64_t>(pd.size());
   auto pages_dev = make_buffer((np > 0 ? np : 1) * static_cast<int64_t>(sizeof(PageDev)), s);
-  const int64_t nl = static_cast<int64_t>(snappy_list.size() + data_list.size());
+  const int64_t n_items = static_cast<int64_t>(item_list.size() / 2);
+  std::vector<int32_t> all_lists(item_list);
+  all_lists.insert(all_lists.end(), snappy_list.begin(), snappy_list.end());
+  all_lists.insert(all_lists.end(), data_list.begin(), data_list.end());
+  const int64_t nl = static_cast<int64_t>(all_lists.size());
   auto lists = make_buffer((nl > 0 ? nl : 1) * 4, s);
-  std::vector<int32_t> both(snappy_list);
-  both.insert(both.end(), data_list.begin(), data_list.end());
   if (np > 0) GF_CUDA(cudaMemcpyAsync(pages_dev->data(), pd.data(), np * sizeof(PageDev), cudaMemcpyHostToDevice, s));
-  if (nl > 0) GF_CUDA(cudaMemcpyAsync(lists->data(), both.data(), nl * 4, cudaMemcpyHostToDevice, s));
+  if (nl > 0) GF_CUDA(cudaMemcpyAsync(lists->data(), all_lists.data(), nl * 4, cudaMemcpyHostToDevice, s));
   PageDev* pages = pages_dev->as<PageDev>();
-  const int32_t* snappy_dev = lists->as<int32_t>();
-  const int32_t* data_dev = lists->as<int32_t>() + snappy_list.size();
+  const int32_t* snappy_dev = lists->as<int32_t>() + item_list.size();
+  const int32_t* data_dev = snappy_dev + snappy_list.size();
 
   if (!snappy_list.empty()) {
     ProfScope prof("parquet_snappy_kernel", s);
@@ -605,8 +663,8 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   if (np > 0) {
     ProfScope prof("parquet_pages_kernel", s);
     const int64_t most = static_cast<int64_t>(num_sms()) * 8;
-    parquet_pages_kernel<<<static_cast<int>(np < most ? np : most), kPqThreads, 0, s>>>(
-        pages, static_cast<int32_t>(np), dicts, st);
+    parquet_pages_kernel<<<static_cast<int>(std::min(n_items, most)), kPqThreads, 0, s>>>(
+        pages, static_cast<int32_t>(np), lists->as<PagePart>(), n_items, dicts, st);
     after_launch("parquet_pages_kernel");
     prof.stop(0.0);
   }
