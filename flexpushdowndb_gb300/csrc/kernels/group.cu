@@ -17,15 +17,15 @@
 // dedicated extra slot at index `capacity`.
 //
 // Aggregation: each CTA first folds its rows into a shared-memory table
-// (64-bit atomicCAS on keys, 64-bit atomics on accumulators) and merges the
-// table into the global open-addressing table once at the end, so
-// low-cardinality group-bys (a handful to a few thousand groups) cost one
-// global atomic per group per CTA rather than per row. Rows whose key does
-// not fit the shared table go straight to the global table. New groups are
-// counted per CTA in shared memory and added to the table's count once per
-// CTA. Integer sums are 64-bit two's-complement additions, which are
-// associative and commutative, so results are bit-exact whatever order the
-// atomics land in.
+// (64-bit atomicCAS on keys, accumulators as pairs of native 32-bit atomics)
+// and merges the table into the global open-addressing table once at the
+// end, so low-cardinality group-bys (a handful to a few thousand groups) cost
+// one global atomic per group per CTA rather than per row. Rows whose key
+// does not fit the shared table collect in a per-warp queue and go to the
+// global table 32 at a time. New groups are counted per CTA in shared memory
+// and added to the table's count once per CTA. Integer sums are 64-bit
+// two's-complement additions, which are associative and commutative, so
+// results are bit-exact whatever order the atomics land in.
 //
 // Table size: at most half full for an upper bound on the groups (groups so
 // far plus the batch's rows). A large batch whose rows are known on the host
@@ -33,8 +33,10 @@
 // sized for that estimate instead: a batch of 20M rows over 1.8M distinct
 // keys gets 4M slots (96 MB with two accumulators) rather than 64M (1.5 GB)
 // to fill and to scan at finalisation.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "eval.cuh"
@@ -44,8 +46,25 @@ namespace gfpdb {
 
 namespace {
 
+// Two block shapes. Batches of kGroupLargeRows rows and more, counted on the
+// host, run one CTA of 1,024 threads per SM whose shared-memory table takes
+// most of the SM (6,000 slots at three accumulators): a frequent key is then
+// kept once per SM and not once per 256-thread CTA, and the table holds more
+// of them. Smaller and device-counted batches run CTAs of 256 threads with
+// 1,024 slots, whose tables are quicker to clear and merge. Measured with 20M
+// rows of Zipf(1.1) int64 keys over 10M values and three aggregates: 609 us
+// and about 40% of the rows in the global table, against 1,126 us and 69% with
+// 760 small CTAs (rows that missed not queued, 64-bit shared-memory atomics);
+// with 200,000 rows of five keys the small CTAs take 17 us (66 us before).
 constexpr int kGroupThreads = 256;
-constexpr int kGroupSmemSlotsMax = 1024;  // slots of a CTA's shared-memory table
+constexpr int kGroupLargeThreads = 1024;
+constexpr int64_t kGroupLargeRows = 2 << 20;
+constexpr int kGroupSmemSlotsMax = 1024;  // slots of a small CTA's shared-memory table
+constexpr int kGroupQueue = 64;           // rows of a warp waiting for the global table (two rounds of 32)
+// A large CTA's table takes in a key on its second sight: a bit per hash
+// value remembers the first. Keys seen once would otherwise fill the table
+// before the frequent ones have all come by.
+constexpr int kGroupSeenBits = 1 << 16;
 constexpr int kGroupSmemProbes = 4;       // shared-memory slots a row tries before the global table
 constexpr uint32_t kDictSpinLimit = 1u << 20;
 
@@ -66,9 +85,10 @@ struct GroupParams {
   DevCol key_cols[2];
   AccDev acc[kMaxAggs];
   DevCol cols[kMaxCols];
-  uint64_t* keys;
+  uint64_t* keys;             // slot i's key at keys[i * key_stride], its accumulators from accs[i * acc_stride]
   unsigned long long* accs;
   uint64_t mask;
+  int32_t key_stride, acc_stride;
   int32_t use_smem;
   int32_t sm_slots;
   DevStatus* st;  // aux[0]: groups claimed, aux[1]: special slot used
@@ -95,7 +115,7 @@ __device__ __forceinline__ uint64_t pack_key(const GroupParams& p, int64_t row) 
 
 // Identity of each accumulator: 0 for sums and counts, +inf / INT64_MAX for
 // MIN, -inf / INT64_MIN for MAX (as bit patterns).
-__device__ __forceinline__ unsigned long long acc_init(int fn, int vt) {
+__host__ __device__ __forceinline__ unsigned long long acc_identity(int fn, int vt) {
   if (fn == AGG_MIN) return vt == VT_F64 ? 0x7ff0000000000000ull : static_cast<unsigned long long>(INT64_MAX);
   if (fn == AGG_MAX) return vt == VT_F64 ? 0xfff0000000000000ull : static_cast<unsigned long long>(INT64_MIN);
   return 0ull;
@@ -132,19 +152,43 @@ __device__ __forceinline__ void acc_combine(unsigned long long* addr, int fn, in
   }
 }
 
+// acc_combine on a shared-memory accumulator. 64-bit atomics there are
+// compare-and-swap loops, which rows of one key on many lanes drag through
+// round after round; 32-bit additions are native. A 64-bit sum is its low
+// half's additions, each passing its carry on (the old value tells), and its
+// high half's: together the same two's-complement sum. A minimum or maximum
+// that does not improve on the value read needs no atomic (it only ever
+// moves one way).
+__device__ __forceinline__ void smem_combine(unsigned long long* addr, int fn, int vt, unsigned long long v) {
+  if (fn == AGG_COUNT || fn == AGG_COUNT_STAR) {
+    atomicAdd(reinterpret_cast<unsigned*>(addr), 1u);  // a CTA counts fewer than 2^31 rows: no carry
+  } else if (fn == AGG_SUM && vt != VT_F64) {
+    unsigned* w = reinterpret_cast<unsigned*>(addr);
+    const unsigned lo = static_cast<unsigned>(v);
+    const unsigned old = atomicAdd(w, lo);
+    const unsigned hi = static_cast<unsigned>(v >> 32) + (old + lo < lo ? 1u : 0u);
+    if (hi != 0) atomicAdd(w + 1, hi);
+  } else if (fn != AGG_SUM && vt != VT_F64) {
+    const long long cur = *reinterpret_cast<volatile long long*>(addr), x = static_cast<long long>(v);
+    if (fn == AGG_MIN ? x < cur : x > cur) acc_combine(addr, fn, vt, v);
+  } else {
+    acc_combine(addr, fn, vt, v);
+  }
+}
+
 // Global slot of a key that is not the all-ones word, continuing from its
 // home slot `slot` whose content `s` the caller has already read; claims an
 // empty slot for a new key. Returns UINT64_MAX (and raises GFPDB_ENOMEM) if
 // the table is full.
 __device__ __forceinline__ uint64_t global_slot_from(const GroupParams& p, uint64_t key, uint64_t slot, uint64_t s,
-                                                     unsigned long long* claims) {
+                                                     unsigned* claims) {
   for (uint64_t i = 0; i <= p.mask; ++i) {
-    if (i > 0) s = *reinterpret_cast<volatile uint64_t*>(p.keys + slot);
+    if (i > 0) s = *reinterpret_cast<volatile uint64_t*>(p.keys + slot * p.key_stride);
     if (s == kEmptySlot) {
-      s = atomicCAS(reinterpret_cast<unsigned long long*>(p.keys + slot), static_cast<unsigned long long>(kEmptySlot),
+      s = atomicCAS(reinterpret_cast<unsigned long long*>(p.keys + slot * p.key_stride), static_cast<unsigned long long>(kEmptySlot),
                     static_cast<unsigned long long>(key));
       if (s == kEmptySlot) {
-        atomicAdd(claims, 1ull);
+        atomicAdd(claims, 1u);
         return slot;
       }
     }
@@ -165,10 +209,16 @@ __device__ __forceinline__ uint64_t special_slot(const GroupParams& p) {
 // `claims` counts the groups this call creates: a CTA's shared-memory
 // counter, added to the table's count once per CTA (one global address
 // taking an atomic per new group would serialise the L2 on it).
-__device__ __forceinline__ uint64_t global_slot(const GroupParams& p, uint64_t key, unsigned long long* claims) {
+__device__ __forceinline__ uint64_t global_slot(const GroupParams& p, uint64_t key, unsigned* claims) {
   if (key == kEmptySlot) return special_slot(p);
   const uint64_t slot = hash_key(static_cast<int64_t>(key)) & p.mask;
-  return global_slot_from(p, key, slot, *reinterpret_cast<volatile uint64_t*>(p.keys + slot), claims);
+  return global_slot_from(p, key, slot, *reinterpret_cast<volatile uint64_t*>(p.keys + slot * p.key_stride), claims);
+}
+
+// The value of an aggregate's input that is no plain column (out of line: the
+// update's loads of four aggregates would otherwise carry four interpreters).
+__device__ __noinline__ unsigned long long program_value(const GroupParams& p, const AccDev& a, int64_t row) {
+  return static_cast<unsigned long long>(operand_row(p.prog, p.cols, a.in, row, p.st));
 }
 
 __device__ __forceinline__ unsigned long long row_value(const GroupParams& p, const AccDev& a, int64_t row) {
@@ -179,86 +229,167 @@ __device__ __forceinline__ unsigned long long row_value(const GroupParams& p, co
       return static_cast<unsigned long long>(__ldcs(static_cast<const long long*>(c.data) + row));
     return static_cast<unsigned long long>(static_cast<int64_t>(__ldcs(static_cast<const int*>(c.data) + row)));
   }
-  return static_cast<unsigned long long>(operand_row(p.prog, p.cols, a.in, row, p.st));
+  return program_value(p, a, row);
 }
 
-__global__ void __launch_bounds__(kGroupThreads) group_update_kernel(const __grid_constant__ GroupParams p) {
+// The accumulators of four aggregates at a time: their inputs are loaded
+// together before the first is combined.
+template <class Combine>
+__device__ __forceinline__ void add_row(const GroupParams& p, int64_t row, Combine&& combine) {
+  for (int a0 = 0; a0 < p.n_acc; a0 += 4) {
+    unsigned long long v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = a0 + u < p.n_acc ? row_value(p, p.acc[a0 + u], row) : 0ull;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (a0 + u < p.n_acc) combine(a0 + u, v[u]);
+  }
+}
+
+// A warp's rows waiting for the global table: a ring of kGroupQueue.
+struct GroupQueue {
+  uint64_t* key;
+  int32_t* row;
+  unsigned head, tail;
+};
+
+// The first n (at most 32) waiting rows into the global table, one per lane.
+__device__ __forceinline__ void drain_queue(const GroupParams& p, GroupQueue& q, int n, int lane, unsigned* claims) {
+  if (lane < n) {
+    const unsigned e = (q.head + lane) & (kGroupQueue - 1);
+    const uint64_t key = q.key[e];
+    const int64_t row = q.row[e];
+    uint64_t g = UINT64_MAX;
+    for (int a0 = 0; a0 == 0 || a0 < p.n_acc; a0 += 4) {
+      unsigned long long v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = a0 + u < p.n_acc ? row_value(p, p.acc[a0 + u], row) : 0ull;
+      if (a0 == 0) {
+        g = global_slot(p, key, claims);
+        if (g == UINT64_MAX) break;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (a0 + u < p.n_acc)
+          acc_combine(p.accs + g * p.acc_stride + a0 + u, p.acc[a0 + u].fn, p.acc[a0 + u].vt, v[u]);
+    }
+  }
+  __syncwarp();
+  q.head += n;
+}
+
+// Bytes of a CTA's dynamic shared memory: the table, the large shape's seen
+// bits, the warps' queues.
+constexpr int64_t group_smem(int threads, int64_t slots, int n_acc) {
+  return slots * (8 + 8 * n_acc) + (threads == kGroupLargeThreads ? kGroupSeenBits / 8 : 0) +
+         static_cast<int64_t>(threads / 32) * kGroupQueue * 12;
+}
+
+// Bound by the L2 operations of the rows that miss the shared table: a read
+// and one reduction per accumulator each, about 44 G reductions a second
+// whatever else the kernel does.
+template <int NT>
+__global__ void __launch_bounds__(NT) group_update_kernel(const __grid_constant__ GroupParams p) {
+  constexpr bool kLarge = NT == kGroupLargeThreads;
   extern __shared__ unsigned long long s_mem[];
-  __shared__ uint16_t s_occ[kGroupSmemSlotsMax];  // the occupied slots, listed for the merge
-  __shared__ int s_scan[kGroupThreads / 32 + 1];
+  __shared__ int s_scan[NT / 32 + 1];
+  __shared__ unsigned s_claims;
+  const int S = p.use_smem ? p.sm_slots : 0;
   uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);
-  unsigned long long* s_acc = s_mem + p.sm_slots;
-  const int sm_mask = p.sm_slots - 1;
+  unsigned long long* s_acc = s_mem + S;  // [accumulator][slot]
+  uint64_t* s_qkey = reinterpret_cast<uint64_t*>(s_acc + static_cast<int64_t>(S) * p.n_acc);
+  int32_t* s_qrow = reinterpret_cast<int32_t*>(s_qkey + (NT / 32) * kGroupQueue);
+  unsigned* s_seen = reinterpret_cast<unsigned*>(s_qrow + (NT / 32) * kGroupQueue);
   const int64_t n_rows = clamp_rows(p.n_dev, p.n_rows);
   // A grid sized for a capacity can be far larger than the rows that arrive:
   // CTAs without rows leave before touching shared memory (uniform per CTA).
-  if (static_cast<int64_t>(blockIdx.x) * kGroupThreads >= n_rows) return;
-  __shared__ unsigned long long s_claims;
+  if (static_cast<int64_t>(blockIdx.x) * NT >= n_rows) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_claims = 0;
-  if (p.use_smem) {
-    for (int i = threadIdx.x; i < p.sm_slots; i += kGroupThreads) {
-      s_keys[i] = kEmptySlot;
-      for (int a = 0; a < p.n_acc; ++a) s_acc[i * p.n_acc + a] = acc_init(p.acc[a].fn, p.acc[a].vt);
-    }
+  for (int i = threadIdx.x; i < S; i += NT) s_keys[i] = kEmptySlot;
+  for (int a = 0; a < p.n_acc; ++a) {
+    const unsigned long long v = acc_identity(p.acc[a].fn, p.acc[a].vt);
+    for (int i = threadIdx.x; i < S; i += NT) s_acc[a * S + i] = v;
   }
+  if (kLarge)
+    for (int i = threadIdx.x; i < kGroupSeenBits / 32; i += NT) s_seen[i] = 0;
   __syncthreads();
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * kGroupThreads;
-  for (int64_t r = static_cast<int64_t>(blockIdx.x) * kGroupThreads + threadIdx.x; r < n_rows; r += stride) {
-    const uint64_t key = pack_key(p, r);
+  GroupQueue q{s_qkey + warp * kGroupQueue, s_qrow + warp * kGroupQueue, 0, 0};
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * NT;
+  int64_t base = static_cast<int64_t>(blockIdx.x) * NT + warp * 32;
+  uint64_t next = base + lane < n_rows ? pack_key(p, base + lane) : 0;
+  for (; base < n_rows; base += stride) {
+    const int64_t r = base + lane;
+    const uint64_t key = next;
+    if (r + stride < n_rows) next = pack_key(p, r + stride);  // a step ahead of its use
     int found = -1;
-    if (p.use_smem && key != kEmptySlot) {
+    if (r < n_rows && S > 0 && key != kEmptySlot) {
       // A short probe run: with few groups the table is sparse and a key is
       // found or placed in a step or two; with many groups (high-cardinality
       // keys) the table is soon full and a longer run only delays the row's
       // trip to the global table.
-      int slot = static_cast<int>(hash_key(static_cast<int64_t>(key)) & sm_mask);
+      const uint64_t h = hash_key(static_cast<int64_t>(key));
+      int slot = static_cast<int>(__umulhi(static_cast<unsigned>(h >> 32), static_cast<unsigned>(S)));
       for (int i = 0; i < kGroupSmemProbes; ++i) {
-        uint64_t s = *reinterpret_cast<volatile uint64_t*>(s_keys + slot);
-        if (s == kEmptySlot) {
-          s = atomicCAS(reinterpret_cast<unsigned long long*>(s_keys + slot),
+        uint64_t k = *reinterpret_cast<volatile uint64_t*>(s_keys + slot);
+        if (k == kEmptySlot) {
+          if (kLarge) {
+            const unsigned bit = static_cast<unsigned>(h) & (kGroupSeenBits - 1);
+            if ((atomicOr(s_seen + (bit >> 5), 1u << (bit & 31)) >> (bit & 31) & 1u) == 0) break;  // first sight
+          }
+          k = atomicCAS(reinterpret_cast<unsigned long long*>(s_keys + slot),
                         static_cast<unsigned long long>(kEmptySlot), static_cast<unsigned long long>(key));
-          if (s == kEmptySlot) s = key;
+          if (k == kEmptySlot) k = key;
         }
-        if (s == key) {
+        if (k == key) {
           found = slot;
           break;
         }
-        slot = (slot + 1) & sm_mask;
+        if (++slot == S) slot = 0;
       }
     }
-    if (found >= 0) {
-      for (int a = 0; a < p.n_acc; ++a)
-        acc_combine(s_acc + found * p.n_acc + a, p.acc[a].fn, p.acc[a].vt, row_value(p, p.acc[a], r));
-    } else {
-      const uint64_t g = global_slot(p, key, &s_claims);
-      if (g != UINT64_MAX)
-        for (int a = 0; a < p.n_acc; ++a)
-          acc_combine(p.accs + g * p.n_acc + a, p.acc[a].fn, p.acc[a].vt, row_value(p, p.acc[a], r));
+    if (found >= 0)
+      add_row(p, r, [&](int a, unsigned long long v) { smem_combine(s_acc + a * S + found, p.acc[a].fn, p.acc[a].vt, v); });
+    const bool miss = r < n_rows && found < 0;
+    const unsigned m = __ballot_sync(0xffffffffu, miss);
+    if (miss) {
+      const unsigned e = (q.tail + __popc(m & ((1u << lane) - 1u))) & (kGroupQueue - 1);
+      q.key[e] = key;
+      q.row[e] = static_cast<int32_t>(r);
     }
+    q.tail += __popc(m);
+    __syncwarp();
+    if (q.tail - q.head >= 32) drain_queue(p, q, 32, lane, &s_claims);
   }
-  if (p.use_smem) {
+  if (q.tail != q.head) drain_queue(p, q, static_cast<int>(q.tail - q.head), lane, &s_claims);
+  auto merge = [&](int i) {
+    const uint64_t g = global_slot(p, s_keys[i], &s_claims);
+    if (g == UINT64_MAX) return;
+    for (int a = 0; a < p.n_acc; ++a)
+      acc_combine(p.accs + g * p.acc_stride + a, p.acc[a].fn, p.acc[a].vt, s_acc[a * S + i]);
+  };
+  __syncthreads();
+  if (kLarge) {
+    for (int i = threadIdx.x; i < S; i += NT)
+      if (s_keys[i] != kEmptySlot) merge(i);
+  } else if (S > 0) {
     // Merge into the global table: the occupied slots are listed first (a
     // block scan), so each thread merges about one group, and every group's
     // global insert and atomics run in the same round instead of one after
     // another on the threads that hold several.
-    __syncthreads();
     int c = 0;
-    for (int i = threadIdx.x; i < p.sm_slots; i += kGroupThreads) c += s_keys[i] != kEmptySlot ? 1 : 0;
+    for (int i = threadIdx.x; i < S; i += NT) c += s_keys[i] != kEmptySlot ? 1 : 0;
+    uint16_t* s_occ = reinterpret_cast<uint16_t*>(s_qkey);  // the queues are empty: at most kGroupSmemSlotsMax entries
     int occupied;
-    int o = block_exclusive_sum<kGroupThreads>(c, &occupied, s_scan);
-    for (int i = threadIdx.x; i < p.sm_slots; i += kGroupThreads)
+    int o = block_exclusive_sum<NT>(c, &occupied, s_scan);
+    for (int i = threadIdx.x; i < S; i += NT)
       if (s_keys[i] != kEmptySlot) s_occ[o++] = static_cast<uint16_t>(i);
     __syncthreads();
-    for (int j = threadIdx.x; j < occupied; j += kGroupThreads) {
-      const int i = s_occ[j];
-      const uint64_t g = global_slot(p, s_keys[i], &s_claims);
-      if (g == UINT64_MAX) continue;
-      for (int a = 0; a < p.n_acc; ++a) acc_combine(p.accs + g * p.n_acc + a, p.acc[a].fn, p.acc[a].vt, s_acc[i * p.n_acc + a]);
-    }
+    for (int j = threadIdx.x; j < occupied; j += NT) merge(s_occ[j]);
   }
   __syncthreads();
   if (threadIdx.x == 0 && s_claims != 0)
-    atomicAdd(reinterpret_cast<unsigned long long*>(&p.st->aux[0]), s_claims);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&p.st->aux[0]), static_cast<unsigned long long>(s_claims));
 }
 
 // HyperLogLog sketch (Flajolet, Fusy, Gandouet, Meunier 2007) of a batch's
@@ -274,12 +405,20 @@ __global__ void __launch_bounds__(256) group_sketch_kernel(const __grid_constant
   __syncthreads();
   const int64_t n = clamp_rows(p.n_dev, p.n_rows);
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += stride) {
-    // a hash unrelated to the slot hash (another constant before the mixer)
-    const uint64_t h = mix64(pack_key(p, r) ^ 0xd6e8feb86659fd93ull);
-    const unsigned idx = static_cast<unsigned>(h >> (64 - kSketchBits));
-    const unsigned rank = static_cast<unsigned>(__clzll((h << kSketchBits) | (1ull << (kSketchBits - 1)))) + 1u;
-    if (rank > s_regs[idx]) atomicMax(&s_regs[idx], rank);
+  // four keys in flight per thread (past the end: the last key again, which
+  // changes no maximum)
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += 4 * stride) {
+    uint64_t key[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) key[u] = pack_key(p, r + u * stride < n ? r + u * stride : n - 1);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      // a hash unrelated to the slot hash (another constant before the mixer)
+      const uint64_t h = mix64(key[u] ^ 0xd6e8feb86659fd93ull);
+      const unsigned idx = static_cast<unsigned>(h >> (64 - kSketchBits));
+      const unsigned rank = static_cast<unsigned>(__clzll((h << kSketchBits) | (1ull << (kSketchBits - 1)))) + 1u;
+      if (rank > s_regs[idx]) atomicMax(&s_regs[idx], rank);
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kSketchRegs; i += blockDim.x) {
@@ -288,38 +427,55 @@ __global__ void __launch_bounds__(256) group_sketch_kernel(const __grid_constant
   }
 }
 
-struct AccKinds {
-  int8_t fn[kMaxAggs];
-  int8_t vt[kMaxAggs];
+// Fills words [0, n) with a pattern of `period` words, 16 bytes a store: a
+// 4M-slot table of 134 MB in 44 us (98 us with a thread storing one slot's
+// words one after another).
+struct InitPattern {
+  unsigned long long word[kMaxAggs + 1];
+  int32_t period;
 };
 
-__global__ void group_init_kernel(uint64_t* keys, unsigned long long* accs, uint64_t n_slots, int n_acc,
-                                  AccKinds kinds) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_slots; i += stride) {
-    keys[i] = kEmptySlot;
-    for (int a = 0; a < n_acc; ++a) accs[i * n_acc + a] = acc_init(kinds.fn[a], kinds.vt[a]);
+__global__ void __launch_bounds__(256) group_init_kernel(unsigned long long* __restrict__ out, uint64_t n,
+                                                         const __grid_constant__ InitPattern pat) {
+  __shared__ unsigned long long s_word[kMaxAggs + 1];
+  if (threadIdx.x < kMaxAggs + 1) s_word[threadIdx.x] = pat.word[threadIdx.x];
+  __syncthreads();
+  const uint64_t stride = 2 * static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  uint64_t i = 2 * (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
+  unsigned m = static_cast<unsigned>(i % pat.period);
+  const unsigned step = static_cast<unsigned>(stride % pat.period);
+  for (; i < n; i += stride) {
+    const unsigned m1 = m + 1 == static_cast<unsigned>(pat.period) ? 0 : m + 1;
+    if (i + 1 < n) *reinterpret_cast<ulonglong2*>(out + i) = make_ulonglong2(s_word[m], s_word[m1]);
+    else out[i] = s_word[m];
+    m += step;
+    if (m >= static_cast<unsigned>(pat.period)) m -= pat.period;
   }
 }
 
+// A table's slots: slot i's key at keys[i * key_stride], its accumulators
+// from accs[i * acc_stride].
+struct TableView {
+  uint64_t* keys;
+  unsigned long long* accs;
+  int32_t key_stride, acc_stride;
+};
+
 // Move every group of an old table into a larger one (accumulators copied).
-__global__ void group_rehash_kernel(const uint64_t* old_keys, const unsigned long long* old_accs, uint64_t old_cap,
-                                    uint64_t* keys, unsigned long long* accs, uint64_t mask, int n_acc, DevStatus* st) {
+__global__ void group_rehash_kernel(TableView old, uint64_t old_cap, TableView to, uint64_t mask, int n_acc,
+                                    DevStatus* st) {
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i <= old_cap; i += stride) {
-    const uint64_t key = old_keys[i];
     uint64_t dst;
     if (i == old_cap) {
-      dst = mask + 1;  // special slot stays special
-      if (key == kEmptySlot) {
-        // the special slot's key word is never written; copy its accumulators
-      }
+      dst = mask + 1;  // the special slot stays special: its key word is never written, its accumulators move
     } else {
+      const uint64_t key = old.keys[i * old.key_stride];
       if (key == kEmptySlot) continue;
       uint64_t slot = hash_key(static_cast<int64_t>(key)) & mask;
       bool ok = false;
       for (uint64_t k = 0; k <= mask; ++k) {
-        const unsigned long long prev = atomicCAS(reinterpret_cast<unsigned long long*>(keys + slot),
+        const unsigned long long prev = atomicCAS(reinterpret_cast<unsigned long long*>(to.keys + slot * to.key_stride),
                                                   static_cast<unsigned long long>(kEmptySlot),
                                                   static_cast<unsigned long long>(key));
         if (prev == kEmptySlot) {
@@ -334,7 +490,7 @@ __global__ void group_rehash_kernel(const uint64_t* old_keys, const unsigned lon
       }
       dst = slot;
     }
-    for (int a = 0; a < n_acc; ++a) accs[dst * n_acc + a] = old_accs[i * n_acc + a];
+    for (int a = 0; a < n_acc; ++a) to.accs[dst * to.acc_stride + a] = old.accs[i * old.acc_stride + a];
   }
 }
 
@@ -348,8 +504,9 @@ struct OutAggDev {
 };
 
 struct FinalParams {
-  const uint64_t* keys;
+  const uint64_t* keys;  // strides as in GroupParams
   const unsigned long long* accs;
+  int32_t key_stride, acc_stride;
   uint64_t cap;  // special slot at index cap
   const int64_t* special_dev;  // non-zero once the all-ones key has a group
   int32_t n_acc;
@@ -391,7 +548,7 @@ __global__ void __launch_bounds__(256) group_finalize_kernel(const __grid_consta
       bool live = false;
       key[k] = 0;
       if (i < p.cap) {
-        key[k] = p.keys[i];
+        key[k] = p.keys[i * p.key_stride];
         live = key[k] != kEmptySlot;
       } else if (i == p.cap) {
         key[k] = kEmptySlot;
@@ -404,34 +561,50 @@ __global__ void __launch_bounds__(256) group_finalize_kernel(const __grid_consta
     unsigned long long at = 0;
     if (lane == 0) at = atomicAdd(p.counter, static_cast<unsigned long long>(total));
     at = __shfl_sync(0xffffffffu, at, 0);
+    // a column at a time, every step's value loaded before the first is stored
+    // (4M slots, 1.8M groups, four columns: 74 us; 142 us a row at a time)
+    int64_t pos[kSteps];  // -1: no live slot
 #pragma unroll
     for (int k = 0; k < kSteps; ++k) {
-      if (m[k] >> lane & 1u) {
-        const uint64_t i = base + k * 32 + lane;
-        const int64_t pos = static_cast<int64_t>(at) + __popc(m[k] & below);
-        if (p.n_keys == 1) {
-          const int64_t v = p.key_bits[0] == 64 ? static_cast<int64_t>(key[k])
-                                                : static_cast<int32_t>(static_cast<uint32_t>(key[k]));
-          store_typed(p.key_dst[0], pos, p.key_type[0], v);
-        } else if (p.n_keys == 2) {
-          store_typed(p.key_dst[0], pos, p.key_type[0], static_cast<int32_t>(static_cast<uint32_t>(key[k] >> 32)));
-          store_typed(p.key_dst[1], pos, p.key_type[1], static_cast<int32_t>(static_cast<uint32_t>(key[k])));
-        }
-        for (int j = 0; j < p.n_out; ++j) {
-          const OutAggDev& o = p.outs[j];
-          const unsigned long long a = p.accs[i * p.n_acc + o.a0];
-          if (o.kind == 0) {
-            store_typed(o.dst, pos, o.out_type, static_cast<int64_t>(a));
-          } else {
-            const unsigned long long c = p.accs[i * p.n_acc + o.a1];
-            const double s = o.vt == VT_F64 ? __longlong_as_double(static_cast<long long>(a))
-                                            : static_cast<double>(static_cast<long long>(a));
-            const double avg = c == 0 ? 0.0 : s / static_cast<double>(c);
-            static_cast<double*>(o.dst)[pos] = avg;
-          }
+      pos[k] = (m[k] >> lane & 1u) ? static_cast<int64_t>(at) + __popc(m[k] & below) : -1;
+      at += __popc(m[k]);
+    }
+    if (p.n_keys == 1) {
+#pragma unroll
+      for (int k = 0; k < kSteps; ++k)
+        if (pos[k] >= 0)
+          store_typed(p.key_dst[0], pos[k], p.key_type[0],
+                      p.key_bits[0] == 64 ? static_cast<int64_t>(key[k])
+                                          : static_cast<int32_t>(static_cast<uint32_t>(key[k])));
+    } else if (p.n_keys == 2) {
+#pragma unroll
+      for (int k = 0; k < kSteps; ++k) {
+        if (pos[k] < 0) continue;
+        store_typed(p.key_dst[0], pos[k], p.key_type[0], static_cast<int32_t>(static_cast<uint32_t>(key[k] >> 32)));
+        store_typed(p.key_dst[1], pos[k], p.key_type[1], static_cast<int32_t>(static_cast<uint32_t>(key[k])));
+      }
+    }
+    const unsigned long long* acc = p.accs + (base + lane) * p.acc_stride;
+    const uint64_t step = static_cast<uint64_t>(32) * p.acc_stride;
+    for (int j = 0; j < p.n_out; ++j) {
+      const OutAggDev& o = p.outs[j];
+      unsigned long long a[kSteps];
+#pragma unroll
+      for (int k = 0; k < kSteps; ++k) a[k] = pos[k] >= 0 ? acc[k * step + o.a0] : 0ull;
+      if (o.kind == 0) {
+#pragma unroll
+        for (int k = 0; k < kSteps; ++k)
+          if (pos[k] >= 0) store_typed(o.dst, pos[k], o.out_type, static_cast<int64_t>(a[k]));
+      } else {
+#pragma unroll
+        for (int k = 0; k < kSteps; ++k) {
+          if (pos[k] < 0) continue;
+          const unsigned long long c = acc[k * step + o.a1];
+          const double sum = o.vt == VT_F64 ? __longlong_as_double(static_cast<long long>(a[k]))
+                                            : static_cast<double>(static_cast<long long>(a[k]));
+          static_cast<double*>(o.dst)[pos[k]] = c == 0 ? 0.0 : sum / static_cast<double>(c);
         }
       }
-      at += __popc(m[k]);
     }
   }
 }
@@ -638,7 +811,7 @@ double sketch_distinct(const GroupParams& p, int64_t n, cudaStream_t s) {
   double sum = 0;
   int zeros = 0;
   for (unsigned v : h) {
-    sum += std::ldexp(1.0, -static_cast<int>(v));
+    sum += 1.0 / static_cast<double>(uint64_t{1} << v);  // v <= 64 - kSketchBits + 1
     zeros += v == 0 ? 1 : 0;
   }
   const double m = kSketchRegs;
@@ -792,7 +965,8 @@ class GroupTable {
   RecordCols records{};
   std::unique_ptr<StringDict> record_dict;
 
-  BufferPtr keys, accbuf, status, fnvt;
+  BufferPtr keys, accbuf, status;  // accbuf is keys where a slot's key and accumulators lie together
+  TableView view{};
   uint64_t cap = 0;
   int64_t groups_upper = 0;
 
@@ -895,40 +1069,57 @@ class GroupTable {
     compiled = true;
   }
 
+  // Tables of kPackedSlots slots and more, too large for the L2 to keep whole,
+  // put a slot's key beside its accumulators when they fill 16 or 32 bytes
+  // (one or three accumulators): a row then touches one sector instead of
+  // two or three.
+  static constexpr uint64_t kPackedSlots = 1ull << 20;
+
   void init_table(uint64_t new_cap, cudaStream_t s) {
     const int na = static_cast<int>(accs.size());
     // Empty keys are all-ones and sum / count accumulators start at zero, so
-    // without MIN / MAX the table comes pre-filled (no init kernel; inside a
-    // captured plan from the graph's fill regions).
+    // without MIN / MAX a table with separate keys comes pre-filled (no init
+    // kernel; inside a captured plan from the graph's fill regions).
     bool zero_init = true;
     for (int a = 0; a < na; ++a) zero_init &= accs[a].fn != AGG_MIN && accs[a].fn != AGG_MAX;
-    const int64_t key_bytes = static_cast<int64_t>(new_cap + 1) * 8;
-    const int64_t acc_bytes = static_cast<int64_t>(new_cap + 1) * 8 * (na > 0 ? na : 1);
-    BufferPtr nk, na_buf;
-    if (zero_init) {
-      nk = make_filled(key_bytes, 0xFF, s);
-      na_buf = make_filled(acc_bytes, 0, s);
-    } else {
-      nk = make_buffer(key_bytes, s);
-      na_buf = make_buffer(acc_bytes, s);
-      AccKinds kinds{};
-      for (int a = 0; a < na; ++a) {
-        kinds.fn[a] = accs[a].fn;
-        kinds.vt[a] = accs[a].vt;
-      }
-      group_init_kernel<<<grid_for(static_cast<int64_t>(new_cap + 1)), 256, 0, s>>>(
-          nk->as<uint64_t>(), na_buf->as<unsigned long long>(), new_cap + 1, na, kinds);
+    const bool packed = new_cap >= kPackedSlots && (na == 1 || na == 3);
+    const int64_t n_slots = static_cast<int64_t>(new_cap + 1);
+    InitPattern pat{};
+    pat.period = packed ? na + 1 : na > 0 ? na : 1;
+    if (packed) pat.word[0] = kEmptySlot;
+    for (int a = 0; a < na; ++a) pat.word[packed ? a + 1 : a] = acc_identity(accs[a].fn, accs[a].vt);
+    auto init = [&](const BufferPtr& b) {
+      const uint64_t words = static_cast<uint64_t>(n_slots) * pat.period;
+      group_init_kernel<<<grid_for(static_cast<int64_t>(words / 2 + 1)), 256, 0, s>>>(b->as<unsigned long long>(), words,
+                                                                                      pat);
       after_launch("group_init_kernel");
+    };
+    BufferPtr nk, nacc;
+    TableView to{};
+    if (packed) {
+      nk = nacc = make_buffer(n_slots * 8 * (na + 1), s);
+      init(nk);
+      to = TableView{nk->as<uint64_t>(), nk->as<unsigned long long>() + 1, na + 1, na + 1};
+    } else {
+      nk = make_filled(n_slots * 8, 0xFF, s);
+      const int64_t acc_bytes = n_slots * 8 * (na > 0 ? na : 1);
+      if (zero_init) {
+        nacc = make_filled(acc_bytes, 0, s);
+      } else {
+        nacc = make_buffer(acc_bytes, s);
+        init(nacc);
+      }
+      to = TableView{nk->as<uint64_t>(), nacc->as<unsigned long long>(), 1, na};
     }
     if (!status) status = make_filled(sizeof(DevStatus), 0, s);
     if (cap > 0) {
-      group_rehash_kernel<<<grid_for(static_cast<int64_t>(cap + 1)), 256, 0, s>>>(
-          keys->as<uint64_t>(), accbuf->as<unsigned long long>(), cap, nk->as<uint64_t>(),
-          na_buf->as<unsigned long long>(), new_cap - 1, na, status->as<DevStatus>());
+      group_rehash_kernel<<<grid_for(static_cast<int64_t>(cap + 1)), 256, 0, s>>>(view, cap, to, new_cap - 1, na,
+                                                                                 status->as<DevStatus>());
       after_launch("group_rehash_kernel");
     }
     keys = nk;
-    accbuf = na_buf;
+    accbuf = nacc;
+    view = to;
     cap = new_cap;
   }
 
@@ -1025,30 +1216,48 @@ class GroupTable {
     for (int a = 0; a < p.n_acc; ++a) p.acc[a] = accs[a];
     bind_columns(slots, ts, p.cols, kMaxCols);
     p.prog = prog;
-    p.keys = keys->as<uint64_t>();
-    p.accs = accbuf->as<unsigned long long>();
+    p.keys = view.keys;
+    p.accs = view.accs;
+    p.key_stride = view.key_stride;
+    p.acc_stride = view.acc_stride;
     p.mask = cap - 1;
     p.st = status->as<DevStatus>();
     // Shared-memory pre-aggregation unless the caller expects many groups.
     const int per_slot = 8 + 8 * p.n_acc;
-    int sm_slots = kGroupSmemSlotsMax;
-    // dynamic plus static shared memory stays within the 48 KB a launch
-    // gets without opting in to more
-    while (sm_slots * per_slot > 44 * 1024) sm_slots >>= 1;
     p.use_smem = (hint == 0 || hint <= 4096) ? 1 : 0;
-    p.sm_slots = sm_slots;
-    const size_t dyn = p.use_smem ? static_cast<size_t>(sm_slots) * per_slot : 0;
-    int64_t blocks = (n + kGroupThreads * 16 - 1) / (kGroupThreads * 16);
-    // one wave: as many CTAs as fit on every SM at once
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, group_update_kernel, kGroupThreads, dyn) != cudaSuccess ||
-        per_sm < 1)
-      per_sm = 1;
-    int64_t max_blocks = static_cast<int64_t>(num_sms()) * per_sm;
-    if (blocks > max_blocks) blocks = max_blocks;
-    if (blocks < 1) blocks = 1;
     ProfScope prof("group_update_kernel", s);
-    group_update_kernel<<<static_cast<int>(blocks), kGroupThreads, dyn, s>>>(p);
+    if (p.use_smem && ts.exact() && n >= kGroupLargeRows) {
+      static std::once_flag configured;
+      std::call_once(configured, [] {
+        GF_CUDA(cudaFuncSetAttribute(group_update_kernel<kGroupLargeThreads>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 2048));
+      });
+      // the opt-in limit less the kernel's static shared memory
+      p.sm_slots = static_cast<int32_t>((max_smem_optin() - 2048 - group_smem(kGroupLargeThreads, 0, 0)) / per_slot);
+      group_update_kernel<kGroupLargeThreads>
+          <<<num_sms(), kGroupLargeThreads, group_smem(kGroupLargeThreads, p.sm_slots, p.n_acc), s>>>(p);
+    } else {
+      int sm_slots = kGroupSmemSlotsMax;
+      // dynamic plus static shared memory stays within the 48 KB a launch
+      // gets without opting in to more
+      while (group_smem(kGroupThreads, sm_slots, p.n_acc) > 47 * 1024) sm_slots >>= 1;
+      p.sm_slots = sm_slots;
+      const size_t dyn = static_cast<size_t>(group_smem(kGroupThreads, p.use_smem ? sm_slots : 0, p.n_acc));
+      // 16 rows a thread amortise a CTA's table, but while that leaves SMs
+      // without a CTA four rows do
+      int64_t blocks = (n + kGroupThreads * 16 - 1) / (kGroupThreads * 16);
+      blocks = std::max(blocks, std::min<int64_t>(num_sms(), (n + kGroupThreads * 4 - 1) / (kGroupThreads * 4)));
+      // one wave: as many CTAs as fit on every SM at once
+      int per_sm = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, group_update_kernel<kGroupThreads>, kGroupThreads,
+                                                        dyn) != cudaSuccess ||
+          per_sm < 1)
+        per_sm = 1;
+      int64_t max_blocks = static_cast<int64_t>(num_sms()) * per_sm;
+      if (blocks > max_blocks) blocks = max_blocks;
+      if (blocks < 1) blocks = 1;
+      group_update_kernel<kGroupThreads><<<static_cast<int>(blocks), kGroupThreads, dyn, s>>>(p);
+    }
     after_launch("group_update_kernel");
     double w = 0;
     for (int k = 0; k < p.n_keys; ++k) w += p.key_bits[k] / 8;
@@ -1087,8 +1296,10 @@ class GroupTable {
     }
     FinalParams fp;
     std::memset(&fp, 0, sizeof(fp));
-    fp.keys = keys->as<uint64_t>();
-    fp.accs = accbuf->as<unsigned long long>();
+    fp.keys = view.keys;
+    fp.accs = view.accs;
+    fp.key_stride = view.key_stride;
+    fp.acc_stride = view.acc_stride;
     fp.cap = cap;
     fp.special_dev = &status->as<DevStatus>()->aux[1];
     fp.n_acc = static_cast<int32_t>(accs.size());
