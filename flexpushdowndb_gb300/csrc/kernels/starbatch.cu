@@ -57,8 +57,10 @@ struct SBDimDev {
   unsigned long long* kmax_u;
   int32_t key32;
   int32_t n_group;
-  int32_t smem_off;      // byte offset of this dimension's staged masks and group values (-1: not staged)
-  int32_t smem_cap;      // keys staged when the key range fits (a multiple of 8)
+  int32_t smem_off;      // byte offset of this dimension's staged area (-1: not staged)
+  int32_t smem_cap;      // keys staged when the key range fits (a multiple of 16)
+  int32_t smem_masks;    // direct form: 1 = a query mask per key, 0 = a class byte per key and the class -> mask table
+  int32_t pad;
 };
 
 // The queries' ranges on one dimension's filter column, as segments: the
@@ -424,7 +426,7 @@ struct SBGlobalDim {
 
 // Step (2) for the entries [h1, h1 + n) of ring 1 (n <= 32), one per lane;
 // survivors go to ring 2, which is worked off 32 entries at a time.
-template <typename M, bool LOAD_FK = false>
+template <typename M>
 __device__ __forceinline__ void sb_probe_global(const SBFactParams& p, SBRings<M>& R, const SBGlobalDim* gl, int nring,
                                              uint32_t h1, int n, uint32_t& h2, uint32_t& t2, int lane) {
   const uint32_t e1 = (h1 + lane) & (kSBRing - 1);
@@ -445,18 +447,7 @@ __device__ __forceinline__ void sb_probe_global(const SBFactParams& p, SBRings<M
     dg0[u] = dg1[u] = 0;
     if (u >= nring || m == 0) continue;
     const SBGlobalDim& G = gl[u];
-    uint32_t idx;
-    if (LOAD_FK) {
-      // the entry's foreign key of this dimension, read from its column
-      // (int32 keys: the direct form)
-      const int32_t fk =
-          __ldg(static_cast<const int32_t*>(p.part_cols[static_cast<int64_t>(part) * p.n_cols + p.fd.fk_col[G.d]].data) +
-                row);
-      const uint64_t i64 = static_cast<uint64_t>(static_cast<int64_t>(fk) - G.kmin);
-      idx = i64 < G.range ? static_cast<uint32_t>(i64) : 0xFFFFFFFFu;
-    } else {
-      idx = R.idx1[u][e1];
-    }
+    const uint32_t idx = R.idx1[u][e1];
     dq[u] = 0;
     if (idx != 0xFFFFFFFFu) {
       dq[u] = sizeof(M) == 4 ? static_cast<uint64_t>(__ldg(reinterpret_cast<const unsigned*>(G.dq) + 2 * idx))
@@ -828,72 +819,196 @@ __global__ void __launch_bounds__(kSBFactThreads, 3) sb_fact_kernel(const __grid
 // and reads each 128-row slice of a tile itself, four consecutive rows per
 // lane by 16-byte loads: no producer warp, no copy stages and no waits
 // between warps, so the shared memory goes to the staged dimensions (up to
-// kSBFastStaged of them) and the rings, and each block stages them once for
-// all its warps. Steps (1)-(3) are those of sb_fact_kernel; step (1) runs
-// in 32-bit arithmetic on the lane's four rows.
+// kSBFastStaged of them), and each block stages them once for all its warps.
+//
+// The steps are those of sb_fact_kernel, arranged for the fewest
+// instructions a row, which bound this pass together with the memory its
+// foreign keys stream from:
+//  (1) a row's index into a staged dimension is its key less the smallest,
+//      in unsigned 32-bit arithmetic and at most the key range, where a
+//      sentinel holds no query; small dimensions are staged as one query mask
+//      per key (a single lookup), larger ones as a class byte per key and the
+//      class -> mask table. Rows some query still wants go to the warp's
+//      first stack as (partition, row, mask);
+//  (2) 32 stacked rows at a time, the direct dimensions in global memory;
+//      survivors go to the second stack;
+//  (3) 32 at a time, the group columns' values (looked up here, for the few
+//      rows that come this far, and not carried along), the group slot, the
+//      measures and the atomic adds.
+// Stacks, not rings: rows are taken from the top, in no particular order.
+//
+// 59,952,713 rows, 32 queries: 369 us before (class bytes for every dimension,
+// group values looked up and carried in step 1, about 124 instructions per 32
+// rows).
 constexpr int kSBDirectWarps = 16;
 constexpr int kSBDirectThreads = kSBDirectWarps * 32;
-constexpr int kSBSlice = 128;  // rows per warp step: four per lane
+constexpr int kSBDirectBlocks = 2;  // blocks an SM's registers hold
+constexpr int kSBSlice = 128;       // rows per warp step: four per lane
+constexpr int kSBStack1 = 31 + kSBSlice + 1;  // a slice on top of fewer than 32 rows
+constexpr int kSBStack2 = 64;
 
 struct SBShared {
   int64_t kmin[kSBMaxDims];
   uint64_t range[kSBMaxDims];
   int32_t off[kSBMaxDims];  // staged: byte offset in the staged area, else -1
-  SBGlobalDim gl[kSBMaxDims];
+  // direct dimensions in global memory, in probe order
+  struct Global {
+    int32_t d;
+    int32_t col;  // foreign-key column slot
+    int64_t kmin;
+    uint64_t range;
+    const uint64_t* dq;
+  } gl[kSBMaxDims];
   // staged dimensions in probe order: foreign-key column slot, smallest key,
-  // key range, class table, classes, group value offsets (-1: none)
+  // key range, masks or classes, class -> mask table (-1: masks per key)
   int32_t st_col[kSBFastStaged];
-  int32_t st_kmin[kSBFastStaged];
+  uint32_t st_kmin[kSBFastStaged];
   uint32_t st_range[kSBFastStaged];
-  int32_t st_tab[kSBFastStaged], st_cls[kSBFastStaged], st_g0[kSBFastStaged], st_g1[kSBFastStaged];
+  int32_t st_keys[kSBFastStaged], st_tab[kSBFastStaged];
   int32_t nst, ngl, nhash;
 };
 
-// Step (1)'s lookups of a row in the dimensions the direct form cannot
-// stage or ring: direct dimensions past the ring's kSBRingDims, and
-// dimensions looked up by hash (sparse keys).
+// A warp's stacks of rows: after the staged dimensions, and after all.
 template <typename M>
-__device__ __forceinline__ void sb_extra_lookups(const SBFactParams& p, const SBShared& sh, const DevCol* cols, int64_t row,
-                                              int nring, M& m, uint32_t& g0, uint32_t& g1) {
-  const int gd0 = p.fd.n_group > 0 ? p.fd.group_dim[0] : -1;
-  const int gd1 = p.fd.n_group > 1 ? p.fd.group_dim[1] : -1;
-  for (int j = nring; m != 0 && j < sh.ngl + (sh.nhash > 0 ? p.n_dims : 0); ++j) {
+struct SBStacks {
+  M m1[kSBStack1];
+  M m2[kSBStack2];
+  uint32_t row1[kSBStack1];
+  uint32_t row2[kSBStack2];
+  uint8_t part1[kSBStack1];
+  uint8_t part2[kSBStack2];
+};
+static_assert(kSBMaxParts <= 256, "a stacked row keeps its partition in a byte");
+
+// Step (1)'s lookups of a row in the dimensions the direct form neither
+// stages nor takes to step (2): direct dimensions past the first kSBRingDims,
+// and dimensions looked up by hash (sparse keys).
+template <typename M>
+__device__ __noinline__ M sb_extra_lookups(const SBFactParams& p, const SBShared& sh, const DevCol* cols, int64_t row,
+                                              int ndirect, M m) {
+  for (int j = ndirect; m != 0 && j < sh.ngl + (sh.nhash > 0 ? p.n_dims : 0); ++j) {
     const bool hashed = j >= sh.ngl;
     const int d = hashed ? j - sh.ngl : sh.gl[j].d;
     if (hashed && sh.range[d] != 0) continue;
     const SBDimDev& D = p.dims[d];
     const int64_t key = load_int(cols[p.fd.fk_col[d]], row);
-    int64_t dr = -1;
     M q = 0;
     if (hashed) {
-      dr = sb_lookup(D, key);
+      const int64_t dr = sb_lookup(D, key);
       if (dr >= 0) q = sb_mask_cast<M>(__ldg(reinterpret_cast<const unsigned long long*>(D.qmask + dr)));
     } else {
       const uint64_t idx = static_cast<uint64_t>(key) - static_cast<uint64_t>(sh.kmin[d]);
-      if (idx < sh.range[d]) {
-        q = sb_mask_cast<M>(__ldg(reinterpret_cast<const unsigned long long*>(D.dq + idx)));
-        dr = static_cast<int64_t>(idx);
-      }
+      if (idx < sh.range[d]) q = sb_mask_cast<M>(__ldg(reinterpret_cast<const unsigned long long*>(D.dq + idx)));
     }
     m &= q;
-    if (m != 0 && d == gd0)
-      g0 = static_cast<uint32_t>(hashed ? load_int(D.group[p.fd.group_idx[0]], dr) : __ldg(D.dg[p.fd.group_idx[0]] + dr));
-    if (m != 0 && d == gd1)
-      g1 = static_cast<uint32_t>(hashed ? load_int(D.group[p.fd.group_idx[1]], dr) : __ldg(D.dg[p.fd.group_idx[1]] + dr));
+  }
+  return m;
+}
+
+// The value of group column g for a row that every dimension selects.
+__device__ __forceinline__ uint32_t sb_group_value(const SBFactParams& p, const SBShared& sh, const DevCol* cols,
+                                                   int64_t row, int g) {
+  const int d = p.fd.group_dim[g], c = p.fd.group_idx[g];
+  const SBDimDev& D = p.dims[d];
+  const int64_t key = load_int(cols[p.fd.fk_col[d]], row);
+  if (sh.range[d] != 0)
+    return static_cast<uint32_t>(__ldg(D.dg[c] + (static_cast<uint64_t>(key) - static_cast<uint64_t>(sh.kmin[d]))));
+  return static_cast<uint32_t>(load_int(D.group[c], sb_lookup(D, key)));
+}
+
+// Step (3) for the n (at most 32) rows of the second stack from `base`.
+template <typename M>
+__device__ __forceinline__ void sb_direct_groups(const SBFactParams& p, const SBShared& sh, const SBStacks<M>& R, int base,
+                                                 int n, int lane) {
+  if (lane >= n) return;
+  M mi = R.m2[base + lane];
+  const int64_t row = R.row2[base + lane];
+  const DevCol* cols = p.part_cols + static_cast<int64_t>(R.part2[base + lane]) * p.n_cols;
+  unsigned long long vals[kSBMaxAggsFact];
+#pragma unroll
+  for (int a = 0; a < kSBMaxAggsFact; ++a) {
+    vals[a] = 0;
+    if (a >= p.n_aggs) continue;
+    const SBAgg& g = p.aggs[a];
+    if (g.fn == AGG_COUNT_STAR) {
+      vals[a] = 1ull;
+    } else {
+      uint64_t x = static_cast<uint64_t>(load_int(cols[g.a], row));
+      if (g.b >= 0) x *= static_cast<uint64_t>(load_int(cols[g.b], row));  // int64 wrap
+      vals[a] = x;
+    }
+  }
+  const uint32_t g0 = p.fd.n_group > 0 ? sb_group_value(p, sh, cols, row, 0) : 0;
+  const uint32_t g1 = p.fd.n_group > 1 ? sb_group_value(p, sh, cols, row, 1) : 0;
+  const uint64_t slot = sb_group_slot(p, sb_group_key(p.fd.n_group, g0, g1));
+  if (slot == UINT64_MAX) return;
+  // a query's bit is set once and stays: an old value that shows it is enough
+  if ((p.touched[slot] & static_cast<unsigned long long>(mi)) != static_cast<unsigned long long>(mi))
+    atomicOr(p.touched + slot, static_cast<unsigned long long>(mi));
+  while (mi != 0) {
+    const int q = sb_ffs(mi) - 1;
+    mi &= mi - 1;
+    unsigned long long* acc =
+        p.gaccs + (static_cast<uint64_t>(q) * (p.gmask + 2) + slot) * static_cast<uint64_t>(p.n_aggs);
+#pragma unroll
+    for (int a = 0; a < kSBMaxAggsFact; ++a)
+      if (a < p.n_aggs) atomicAdd(acc + a, vals[a]);
+  }
+}
+
+// Step (2) for the n (at most 32) rows of the first stack from `base`;
+// survivors go on the second stack, which is worked off 32 at a time.
+template <typename M>
+__device__ __forceinline__ void sb_direct_probe(const SBFactParams& p, const SBShared& sh, SBStacks<M>& R, int ndirect,
+                                                int base, int n, int& t2, unsigned& seen2, int lane) {
+  M m = 0;
+  uint32_t part = 0, row = 0;
+  if (lane < n) {
+    m = R.m1[base + lane];
+    row = R.row1[base + lane];
+    part = R.part1[base + lane];
+  }
+  const DevCol* cols = p.part_cols + static_cast<int64_t>(part) * p.n_cols;
+  M q[kSBRingDims];
+#pragma unroll
+  for (int u = 0; u < kSBRingDims; ++u) {
+    q[u] = u < ndirect ? M(0) : ~M(0);
+    if (u >= ndirect || m == 0) continue;
+    const SBShared::Global& G = sh.gl[u];
+    const int32_t fk = __ldg(static_cast<const int32_t*>(cols[G.col].data) + row);
+    const uint64_t idx = static_cast<uint64_t>(static_cast<int64_t>(fk) - G.kmin);
+    if (idx < G.range)
+      q[u] = sizeof(M) == 4 ? static_cast<M>(__ldg(reinterpret_cast<const unsigned*>(G.dq) + 2 * idx))
+                            : static_cast<M>(__ldg(reinterpret_cast<const unsigned long long*>(G.dq) + idx));
+  }
+#pragma unroll
+  for (int u = 0; u < kSBRingDims; ++u) m &= q[u];
+  const unsigned b = __ballot_sync(0xffffffffu, m != 0);
+  if (m != 0) {
+    const int e = t2 + __popc(b & ((1u << lane) - 1u));
+    R.m2[e] = m;
+    R.row2[e] = row;
+    R.part2[e] = static_cast<uint8_t>(part);
+  }
+  t2 += __popc(b);
+  __syncwarp();  // also: the first stack's rows are read
+  if (t2 >= 32) {
+    t2 -= 32;
+    seen2 += 32;
+    sb_direct_groups<M>(p, sh, R, t2, 32, lane);
+    __syncwarp();
   }
 }
 
 template <int ITEMS, typename M>
-__global__ void __launch_bounds__(kSBDirectThreads, 2) sb_fact_direct_kernel(const __grid_constant__ SBFactParams p) {
+__global__ void __launch_bounds__(kSBDirectThreads, kSBDirectBlocks)
+    sb_fact_direct_kernel(const __grid_constant__ SBFactParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t staging;
   __shared__ SBShared sh;
   unsigned char* staged_dims = smem + p.masks_off;
-  SBRings<M>* rings = reinterpret_cast<SBRings<M>*>(smem + p.rings_off);
+  SBStacks<M>* stacks = reinterpret_cast<SBStacks<M>*>(smem + p.rings_off);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int gd0 = p.fd.n_group > 0 ? p.fd.group_dim[0] : -1;
-  const int gd1 = p.fd.n_group > 1 ? p.fd.group_dim[1] : -1;
   if (threadIdx.x < p.n_dims) {
     const SBDimDev& D = p.dims[threadIdx.x];
     const SBDirect dr = sb_direct(D);
@@ -902,45 +1017,28 @@ __global__ void __launch_bounds__(kSBDirectThreads, 2) sb_fact_direct_kernel(con
     sh.off[threadIdx.x] =
         (dr.range != 0 && D.smem_off >= 0 && dr.range <= static_cast<uint64_t>(D.smem_cap)) ? D.smem_off : -1;
   }
-  if (threadIdx.x == 0) {
-    mbar_init(&staging, 1);
-    mbar_fence_init();
-  }
   __syncthreads();
   if (threadIdx.x == 0) {
     int nst = 0, ngl = 0, nh = 0;
-    uint32_t bytes = 0;
     for (int j = 0; j < p.n_dims; ++j) {
       const int d = p.fd.order[j];
       const SBDimDev& D = p.dims[d];
       if (sh.off[d] >= 0 && nst < kSBFastStaged) {
-        // staged layout: the class -> mask table (256 masks), each group
-        // column's values, then the classes (one byte per key)
-        const int cap = D.smem_cap;
-        const int tab = 256 * static_cast<int>(sizeof(M));
         const int o = sh.off[d];
         sh.st_col[nst] = p.fd.fk_col[d];
-        sh.st_kmin[nst] = static_cast<int32_t>(sh.kmin[d]);
+        sh.st_kmin[nst] = static_cast<uint32_t>(static_cast<int32_t>(sh.kmin[d]));
         sh.st_range[nst] = static_cast<uint32_t>(sh.range[d]);
-        sh.st_tab[nst] = o;
-        sh.st_g0[nst] = d == gd0 ? o + tab + p.fd.group_idx[0] * cap * 4 : -1;
-        sh.st_g1[nst] = d == gd1 ? o + tab + p.fd.group_idx[1] * cap * 4 : -1;
-        sh.st_cls[nst] = o + tab + D.n_group * cap * 4;
-        const uint32_t keys = static_cast<uint32_t>((sh.range[d] + 15) / 16 * 16);
-        bytes += keys * (1 + 4 * D.n_group);
+        sh.st_tab[nst] = D.smem_masks ? -1 : o;
+        sh.st_keys[nst] = D.smem_masks ? o : o + 256 * static_cast<int>(sizeof(M));
         ++nst;
       } else if (sh.range[d] != 0) {
         sh.off[d] = -1;  // looked up in global memory
-        SBGlobalDim& G = sh.gl[ngl];
+        SBShared::Global& G = sh.gl[ngl++];
         G.d = d;
-        G.seg = 0;
-        G.w8 = 0;
+        G.col = p.fd.fk_col[d];
         G.kmin = sh.kmin[d];
         G.range = sh.range[d];
         G.dq = D.dq;
-        G.g0 = d == gd0 ? D.dg[p.fd.group_idx[0]] : nullptr;
-        G.g1 = d == gd1 ? D.dg[p.fd.group_idx[1]] : nullptr;
-        ++ngl;
       } else {
         ++nh;
       }
@@ -948,37 +1046,49 @@ __global__ void __launch_bounds__(kSBDirectThreads, 2) sb_fact_direct_kernel(con
     sh.nst = nst;
     sh.ngl = ngl;
     sh.nhash = nh;
-    // classes and group values of the staged dimensions by bulk copies
-    // (16-byte multiples: the device arrays and the staged area hold whole
-    // multiples of 16 keys)
-    mbar_arrive_expect_tx(&staging, bytes);
-    for (int j = 0; j < p.n_dims; ++j) {
-      const int d = p.fd.order[j];
-      if (sh.off[d] < 0) continue;
-      const SBDimDev& D = p.dims[d];
-      const int cap = D.smem_cap;
-      const uint32_t keys = static_cast<uint32_t>((sh.range[d] + 15) / 16 * 16);
-      for (int c = 0; c < D.n_group; ++c)
-        bulk_g2s(staged_dims + sh.off[d] + 256 * sizeof(M) + c * cap * 4, D.dg[c], keys * 4, &staging);
-      bulk_g2s(staged_dims + sh.off[d] + 256 * sizeof(M) + D.n_group * cap * 4, D.dclass, keys, &staging);
+  }
+  __syncthreads();
+  // Staging: the class bytes of [0, range) come 16 at a time (a dimension's
+  // device array holds whole multiples of 64 keys); a masks-per-key
+  // dimension's classes are turned into masks on the way. Entry `range` is
+  // the sentinel of keys outside the range.
+  for (int d = 0; d < p.n_dims; ++d) {
+    if (sh.off[d] < 0) continue;
+    const SBDimDev& D = p.dims[d];
+    const uint32_t range = static_cast<uint32_t>(sh.range[d]);
+    const uint4* src = reinterpret_cast<const uint4*>(D.dclass);
+    M* tab = reinterpret_cast<M*>(staged_dims + sh.off[d]);
+    if (D.smem_masks) {
+      for (uint32_t i = threadIdx.x; i < (range + 15) / 16; i += kSBDirectThreads) {
+        const uint4 v = src[i];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+          tab[16 * i + k] = sb_mask_cast<M>(__ldg(&p.segs[d].cmask[(w[k >> 2] >> (8 * (k & 3))) & 0xFFu]));
+      }
+    } else {
+      uint4* cls = reinterpret_cast<uint4*>(tab + 256);
+      for (uint32_t i = threadIdx.x; i < (range + 15) / 16; i += kSBDirectThreads) cls[i] = src[i];
+      for (int i = threadIdx.x; i < 256; i += kSBDirectThreads) tab[i] = sb_mask_cast<M>(p.segs[d].cmask[i]);
     }
   }
   __syncthreads();
-  for (int d = 0; d < p.n_dims; ++d) {
-    if (sh.off[d] < 0) continue;
+  if (threadIdx.x < p.n_dims && sh.off[threadIdx.x] >= 0) {
+    const int d = threadIdx.x;
     M* tab = reinterpret_cast<M*>(staged_dims + sh.off[d]);
-    for (int i = threadIdx.x; i < 256; i += kSBDirectThreads) tab[i] = sb_mask_cast<M>(p.segs[d].cmask[i]);
+    if (p.dims[d].smem_masks) tab[sh.range[d]] = 0;
+    else reinterpret_cast<uint8_t*>(tab + 256)[sh.range[d]] = kSBNoRow;
   }
-  if (!mbar_wait(&staging, 0)) raise_status(p.st, GFPDB_ETIMEDOUT, 134);
   __syncthreads();
 
-  SBRings<M>& R = rings[warp];
+  SBStacks<M>& R = stacks[warp];
   const M qvalid = sb_mask_cast<M>(p.qvalid);
   const unsigned lt_mask = (1u << lane) - 1u;
-  const int nst = sh.nst, ngl = sh.ngl, nhash = sh.nhash;
-  const int nring = ngl < kSBRingDims ? ngl : kSBRingDims;
-  const bool extra = ngl > nring || nhash > 0;  // lookups step (1) makes per row
-  uint32_t h1 = 0, t1 = 0, h2 = 0, t2 = 0;
+  const int nst = sh.nst, ngl = sh.ngl;
+  const int ndirect = ngl < kSBRingDims ? ngl : kSBRingDims;
+  const bool extra = ngl > ndirect || sh.nhash > 0;  // lookups step (1) makes per row
+  int t1 = 0, t2 = 0;                       // rows on the stacks
+  unsigned seen1 = 0, seen2 = 0;            // rows taken off them (a warp's: under 2^32)
   constexpr int64_t kTileRows = static_cast<int64_t>(kSBConsumerWarps) * 32 * ITEMS;
   int part = 0;
   const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kSBDirectWarps;
@@ -986,92 +1096,83 @@ __global__ void __launch_bounds__(kSBDirectThreads, 2) sb_fact_direct_kernel(con
        tile += nwarps) {
     const SBTile t = sb_tile(p, tile, kTileRows, &part);
     const DevCol* cols = p.part_cols + static_cast<int64_t>(t.part) * p.n_cols;
-    for (int64_t sub = 0; sub < t.rows; sub += kSBSlice) {
-      const int64_t row0 = t.start + sub;  // the slice's first row in the partition
-      const int nrows = t.rows - sub < kSBSlice ? static_cast<int>(t.rows - sub) : kSBSlice;
+    const int32_t* fk[kSBFastStaged];  // the lane's keys of the tile's first slice
+#pragma unroll
+    for (int j = 0; j < kSBFastStaged; ++j)
+      fk[j] = j < nst ? static_cast<const int32_t*>(cols[sh.st_col[j]].data) + t.start + lane * 4 : nullptr;
+    for (int sub = 0; sub < static_cast<int>(t.rows); sub += kSBSlice) {
+      const int nrows = static_cast<int>(t.rows) - sub;  // of this slice and the ones after it
+      const bool whole = nrows >= kSBSlice;
       const int r4 = lane * 4;  // the lane's first row in the slice
-      // foreign keys of the lane's four rows: staged and ring dimensions
       int4 fs[kSBFastStaged];
-      auto load4 = [&](int col) -> int4 {
-        const int32_t* c = static_cast<const int32_t*>(cols[col].data) + row0 + r4;
-        if (nrows == kSBSlice) return __ldg(reinterpret_cast<const int4*>(c));
-        int4 v = make_int4(0, 0, 0, 0);
-        if (r4 + 0 < nrows) v.x = __ldg(c + 0);
-        if (r4 + 1 < nrows) v.y = __ldg(c + 1);
-        if (r4 + 2 < nrows) v.z = __ldg(c + 2);
-        if (r4 + 3 < nrows) v.w = __ldg(c + 3);
-        return v;
-      };
 #pragma unroll
-      for (int j = 0; j < kSBFastStaged; ++j) fs[j] = j < nst ? load4(sh.st_col[j]) : make_int4(0, 0, 0, 0);
-      // Step (1): the staged dimensions in probe order, each one's facts
-      // read once for the lane's four rows
-      M mk[4];
-      uint32_t g0k[4], g1k[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        mk[k] = r4 + k < nrows ? qvalid : M(0);
-        g0k[k] = g1k[k] = 0;
+      for (int j = 0; j < kSBFastStaged; ++j) {
+        fs[j] = make_int4(0, 0, 0, 0);
+        if (j >= nst) continue;
+        const int32_t* c = fk[j] + sub;
+        if (whole) {
+          fs[j] = __ldg(reinterpret_cast<const int4*>(c));
+        } else {
+          if (r4 + 0 < nrows) fs[j].x = __ldg(c + 0);
+          if (r4 + 1 < nrows) fs[j].y = __ldg(c + 1);
+          if (r4 + 2 < nrows) fs[j].z = __ldg(c + 2);
+          if (r4 + 3 < nrows) fs[j].w = __ldg(c + 3);
+        }
       }
+      M mk[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) mk[k] = whole || r4 + k < nrows ? qvalid : M(0);
 #pragma unroll
       for (int j = 0; j < kSBFastStaged; ++j) {
         if (j >= nst) break;
-        const int32_t kmin = sh.st_kmin[j];
-        const uint32_t range = sh.st_range[j];
-        const M* tab = reinterpret_cast<const M*>(staged_dims + sh.st_tab[j]);
-        const uint8_t* cls = staged_dims + sh.st_cls[j];
-        const int go0 = sh.st_g0[j], go1 = sh.st_g1[j];
+        const uint32_t kmin = sh.st_kmin[j], range = sh.st_range[j];
+        const uint32_t idx[4] = {min(static_cast<uint32_t>(fs[j].x) - kmin, range),
+                                 min(static_cast<uint32_t>(fs[j].y) - kmin, range),
+                                 min(static_cast<uint32_t>(fs[j].z) - kmin, range),
+                                 min(static_cast<uint32_t>(fs[j].w) - kmin, range)};
+        const int tab = sh.st_tab[j];
+        if (tab < 0) {
+          const M* masks = reinterpret_cast<const M*>(staged_dims + sh.st_keys[j]);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int32_t fk = k == 0 ? fs[j].x : k == 1 ? fs[j].y : k == 2 ? fs[j].z : fs[j].w;
-          const uint32_t idx = static_cast<uint32_t>(fk) - static_cast<uint32_t>(kmin);
-          const bool in = mk[k] != 0 && fk >= kmin && idx < range;
-          mk[k] = in ? mk[k] & tab[cls[idx]] : M(0);
-          if (mk[k] != 0 && go0 >= 0) g0k[k] = reinterpret_cast<const uint32_t*>(staged_dims + go0)[idx];
-          if (mk[k] != 0 && go1 >= 0) g1k[k] = reinterpret_cast<const uint32_t*>(staged_dims + go1)[idx];
+          for (int k = 0; k < 4; ++k) mk[k] &= masks[idx[k]];
+        } else {
+          const uint8_t* cls = staged_dims + sh.st_keys[j];
+          const M* masks = reinterpret_cast<const M*>(staged_dims + tab);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mk[k] &= masks[cls[idx[k]]];
         }
       }
+      if (extra) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (mk[k] != 0) mk[k] = sb_extra_lookups<M>(p, sh, cols, t.start + sub + r4 + k, ndirect, mk[k]);
+      }
+      const uint32_t row0 = static_cast<uint32_t>(t.start) + static_cast<uint32_t>(sub + r4);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int rin = r4 + k;
-        M m = mk[k];
-        uint32_t g0 = g0k[k], g1 = g1k[k];
-        // direct dimensions past the ring's, and dimensions looked up by
-        // hash (sparse keys): per row, out of line
-        if (extra && m != 0) sb_extra_lookups<M>(p, sh, cols, row0 + rin, nring, m, g0, g1);
-        const unsigned b = __ballot_sync(0xffffffffu, m != 0);
-        if (m != 0) {
-          const uint32_t e = (t1 + __popc(b & lt_mask)) & (kSBRing - 1);
-          R.part1[e] = static_cast<uint32_t>(t.part);
-          R.row1[e] = static_cast<uint32_t>(row0 + rin);
-          R.m1[e] = m;
-          R.g1a[e] = g0;
-          R.g1b[e] = g1;
+        const unsigned b = __ballot_sync(0xffffffffu, mk[k] != 0);
+        if (mk[k] != 0) {
+          const int e = t1 + __popc(b & lt_mask);
+          R.m1[e] = mk[k];
+          R.row1[e] = row0 + k;
+          R.part1[e] = static_cast<uint8_t>(t.part);
         }
         t1 += __popc(b);
-        __syncwarp();
-        if (t1 - h1 >= 32) {
-          sb_probe_global<M, true>(p, R, sh.gl, nring, h1, 32, h2, t2, lane);
-          h1 += 32;
-        }
+      }
+      __syncwarp();
+      while (t1 >= 32) {
+        t1 -= 32;
+        seen1 += 32;
+        sb_direct_probe<M>(p, sh, R, ndirect, t1, 32, t2, seen2, lane);
       }
     }
   }
-  // the warp's last rows: ring 1, then ring 2
-  while (t1 != h1) {
-    const int n = t1 - h1 < 32 ? static_cast<int>(t1 - h1) : 32;
-    sb_probe_global<M, true>(p, R, sh.gl, nring, h1, n, h2, t2, lane);
-    h1 += n;
-  }
-  while (t2 != h2) {
-    const int n = t2 - h2 < 32 ? static_cast<int>(t2 - h2) : 32;
-    sb_update_groups<M>(p, R, h2, n, lane);
-    h2 += n;
-    __syncwarp();
-  }
+  // the warp's last rows
+  if (t1 > 0) sb_direct_probe<M>(p, sh, R, ndirect, 0, t1, t2, seen2, lane);
+  if (t2 > 0) sb_direct_groups<M>(p, sh, R, 0, t2, lane);
   if (lane == 0) {
-    atomicAdd(p.gathered, static_cast<unsigned long long>(t1));
-    atomicAdd(p.gathered + 1, static_cast<unsigned long long>(t2));
+    atomicAdd(p.gathered, static_cast<unsigned long long>(seen1 + t1));
+    atomicAdd(p.gathered + 1, static_cast<unsigned long long>(seen2 + t2));
   }
 }
 
@@ -1227,7 +1328,7 @@ struct StarBatchState {
   std::vector<TileGroup> group_tiles;
   int64_t host_bytes = 0;
   std::vector<char> in_place;       // per fact column: read in place from page-locked host memory
-  int n_in_place_fk = 0, n_in_place_measures = 0;
+  int n_in_place_fk = 0, n_in_place_measures = 0, n_in_place_group_fk = 0;
   unsigned long long* gathered = nullptr;
   cudaStream_t copy_stream = nullptr;
   std::vector<cudaEvent_t> events;  // start, dimensions, then one per group
@@ -1263,7 +1364,8 @@ const unsigned long long* StarBatch::gathered() const { return st_->gathered; }
 int64_t StarBatch::in_place_bytes(uint64_t ring_rows, uint64_t survivor_rows) const {
   // one 32-byte sector per row and column read in place (an upper bound:
   // rows that share a sector are counted once each)
-  return static_cast<int64_t>(32 * (ring_rows * st_->n_in_place_fk + survivor_rows * st_->n_in_place_measures));
+  return static_cast<int64_t>(32 * (ring_rows * st_->n_in_place_fk +
+                                    survivor_rows * (st_->n_in_place_measures + st_->n_in_place_group_fk)));
 }
 
 StarBatchState::~StarBatchState() {
@@ -1459,9 +1561,8 @@ void StarBatchState::prepare(cudaStream_t s) {
     group_types[g] = c->type;
     ++D.n_group;
   }
-  // Shared-memory staging: the smallest dimensions first, one 64-bit mask
-  // per key, within a per-block budget that leaves room for blocks_per_sm
-  // blocks on an SM.
+  // Shared-memory staging: the smallest dimensions first, within a per-block
+  // budget that leaves room for blocks_per_sm blocks on an SM.
   std::vector<int> by_rows(nd);
   for (int d = 0; d < nd; ++d) by_rows[d] = d;
   std::stable_sort(by_rows.begin(), by_rows.end(),
@@ -1475,24 +1576,53 @@ void StarBatchState::prepare(cudaStream_t s) {
   fact_params.masks_off = static_cast<int32_t>(masks_off);
   // Query masks are 32 bits wide for batches of at most 32 queries.
   mask_bytes = nq <= 32 ? 4 : 8;
-  const int64_t rings_bytes = static_cast<int64_t>(direct ? kSBDirectWarps : kSBConsumerWarps) *
-                              (mask_bytes == 4 ? sizeof(SBRings<uint32_t>) : sizeof(SBRings<uint64_t>));
-  const int64_t block_target = std::min<int64_t>(kSBSmemBudget / std::max(1, spec.blocks_per_sm), kSBSmemPerBlockMax);
+  const int64_t rings_bytes =
+      direct ? kSBDirectWarps * static_cast<int64_t>(mask_bytes == 4 ? sizeof(SBStacks<uint32_t>) : sizeof(SBStacks<uint64_t>))
+             : kSBConsumerWarps * static_cast<int64_t>(mask_bytes == 4 ? sizeof(SBRings<uint32_t>) : sizeof(SBRings<uint64_t>));
+  // Blocks that share an SM's staging room: as asked for, but in the direct
+  // form no more than its registers hold. (Room for four blocks of which two
+  // run left the 30,000-key dimension of a 15M-row, 8-query batch unstaged:
+  // 253 us for the fact pass.)
+  const int sharing = std::max(1, direct ? std::min(spec.blocks_per_sm, kSBDirectBlocks) : spec.blocks_per_sm);
+  const int64_t block_target = std::min<int64_t>(kSBSmemBudget / sharing, kSBSmemPerBlockMax);
   const int64_t budget = std::max<int64_t>(0, block_target - masks_off - rings_bytes);
   int64_t staged = 0;  // bytes
   int n_staged = 0;
-  for (int d = 0; d < nd; ++d) dims_params.dims[d].smem_off = -1;
+  for (int d = 0; d < nd; ++d) {
+    dims_params.dims[d].smem_off = -1;
+    dims_params.dims[d].smem_masks = 0;
+  }
+  // bytes of a staged dimension: the class -> mask table, each group column's
+  // values (not in the direct form, which looks them up later), one class
+  // byte per key and, in the direct form, a sentinel; or there a mask per key
+  auto staged_bytes = [&](const SBDimDev& D, bool masks) {
+    const int64_t keys = (D.rows + 15) / 16 * 16;  // a dense key range needs one entry per row
+    if (!direct) return 256 * mask_bytes + keys * (1 + 4 * D.n_group);
+    return masks ? (keys + 4) * mask_bytes : 256 * mask_bytes + keys + 16;
+  };
+  std::vector<int> chosen;
   for (int d : by_rows) {
     SBDimDev& D = dims_params.dims[d];
     if (direct && n_staged == kSBFastStaged) break;
-    const int64_t keys = (D.rows + 15) / 16 * 16;  // a dense key range needs one entry per row
-    // the class -> mask table, each group column's values, one class byte per key
-    const int64_t bytes = 256 * mask_bytes + keys * (1 + 4 * D.n_group);
-    if (D.rows == 0 || staged + bytes > budget) continue;
-    D.smem_off = static_cast<int32_t>(staged);
-    D.smem_cap = static_cast<int32_t>(keys);
-    staged += bytes;
+    if (D.rows == 0 || staged + staged_bytes(D, false) > budget) continue;
+    staged += staged_bytes(D, false);
+    chosen.push_back(d);
     ++n_staged;
+  }
+  // with room left, the smallest dimensions' classes become masks
+  for (int d : chosen) {
+    SBDimDev& D = dims_params.dims[d];
+    const int64_t more = staged_bytes(D, true) - staged_bytes(D, false);
+    if (!direct || staged + more > budget) break;
+    D.smem_masks = 1;
+    staged += more;
+  }
+  staged = 0;
+  for (int d : chosen) {
+    SBDimDev& D = dims_params.dims[d];
+    D.smem_off = static_cast<int32_t>(staged);
+    D.smem_cap = static_cast<int32_t>((D.rows + 15) / 16 * 16);
+    staged += (staged_bytes(D, D.smem_masks != 0) + 15) / 16 * 16;
   }
   const int64_t rings_off = (masks_off + staged + 15) / 16 * 16;
   fact_params.rings_off = static_cast<int32_t>(rings_off);
@@ -1586,7 +1716,7 @@ void StarBatchState::prepare(cudaStream_t s) {
   // measures) are read in place from page-locked host memory; the columns
   // it reads in full are copied by every run (plan_host_copies).
   in_place.assign(nc, 0);
-  n_in_place_fk = n_in_place_measures = 0;
+  n_in_place_fk = n_in_place_measures = n_in_place_group_fk = 0;
   if (direct && !host_cols.empty()) {
     for (int c = 0; c < nc; ++c) {
       bool fk = false, staged_fk = false;
@@ -1609,10 +1739,12 @@ void StarBatchState::prepare(cudaStream_t s) {
       if (!ok) continue;
       for (size_t pi = 0; pi < parts.size(); ++pi) hcols[pi * nc + c].data = views[pi];
       in_place[c] = 1;
-      if (fk)
+      if (fk) {
         ++n_in_place_fk;
-      else
+        for (const auto& g : spec.group) n_in_place_group_fk += fk_slot[g.dim] == c ? 1 : 0;  // read again for its group
+      } else {
         ++n_in_place_measures;
+      }
     }
   }
   // Metadata goes up once, from host memory that this object keeps (so a
