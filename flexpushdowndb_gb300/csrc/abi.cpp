@@ -73,9 +73,9 @@ struct CapturedPlan {
 void capture_epilogue(CapturedPlan& cp, cudaStream_t cs) {
   std::vector<CopySpan> spans;
   int64_t off = 0;
-  auto add = [&](const void* src, int64_t bytes) {
+  auto add = [&](const void* src, int64_t bytes, const int64_t* rows = nullptr, int64_t row_bytes = 0) {
     const int64_t o = off;
-    spans.push_back(CopySpan{src, bytes, o});
+    spans.push_back(CopySpan{src, bytes, o, rows, row_bytes});
     off += (bytes + 255) / 256 * 256;
     return o;
   };
@@ -92,7 +92,8 @@ void capture_epilogue(CapturedPlan& cp, cudaStream_t cs) {
       const int64_t o2 = add(c->data, c->data_buf->size());
       cp.col_off.push_back({o1, o2});
     } else {
-      cp.col_off.push_back({add(c->data, cap * dtype_width(c->type))});
+      const int w = dtype_width(c->type);
+      cp.col_off.push_back({add(c->data, cap * w, r.exact() ? nullptr : r.rows_dev(), w)});
     }
   }
   cp.pinned_bytes = off > 0 ? off : 256;
@@ -1287,9 +1288,9 @@ int32_t gfpdb_batch_prepare(const char* spec_json, int32_t n_tables, const char*
     const TupleSet& r = *b->result;
     std::vector<CopySpan> spans;
     int64_t off = 0;
-    auto add = [&](const void* src, int64_t bytes) {
+    auto add = [&](const void* src, int64_t bytes, const int64_t* rows = nullptr, int64_t row_bytes = 0) {
       const int64_t o = off;
-      spans.push_back(CopySpan{src, bytes, o});
+      spans.push_back(CopySpan{src, bytes, o, rows, row_bytes});
       off += (bytes + 255) / 256 * 256;
       return o;
     };
@@ -1298,7 +1299,8 @@ int32_t gfpdb_batch_prepare(const char* spec_json, int32_t n_tables, const char*
     b->count_off = add(r.rows_dev(), sizeof(int64_t));
     for (int i = 0; i < r.num_columns(); ++i) {
       const auto& c = r.column(i);
-      b->col_off.push_back(add(c->data, r.num_rows() * dtype_width(c->type)));
+      const int w = dtype_width(c->type);
+      b->col_off.push_back(add(c->data, r.num_rows() * w, r.rows_dev(), w));
     }
     b->pinned_bytes = off;
     GF_CUDA(cudaMallocHost(reinterpret_cast<void**>(&b->pinned), static_cast<size_t>(off)));

@@ -154,7 +154,12 @@ __global__ void __launch_bounds__(256) pack_spans_kernel(const __grid_constant__
   // on both sides in practice), four loads in flight per thread, then the
   // tail under 16 bytes
   const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
-  const int64_t n16 = vec ? sp.bytes / 16 : 0;
+  int64_t bytes = sp.bytes;
+  if (sp.rows != nullptr) {
+    const int64_t rows = *sp.rows;
+    if (rows < bytes / sp.row_bytes) bytes = rows > 0 ? rows * sp.row_bytes : 0;
+  }
+  const int64_t n16 = vec ? bytes / 16 : 0;
   const uint4* s4 = reinterpret_cast<const uint4*>(src);
   uint4* d4 = reinterpret_cast<uint4*>(dst);
   int64_t i = threadIdx.x;
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(256) pack_spans_kernel(const __grid_constant__
     d4[i + 768] = d;
   }
   for (; i < n16; i += 256) d4[i] = s4[i];
-  for (int64_t j = n16 * 16 + threadIdx.x; j < sp.bytes; j += 256) dst[j] = src[j];
+  for (int64_t j = n16 * 16 + threadIdx.x; j < bytes; j += 256) dst[j] = src[j];
 }
 
 // Host-to-device copy done by the SMs: each thread streams 16-byte words from

@@ -43,6 +43,8 @@ struct CopySpan {
   const void* src;
   int64_t bytes;
   int64_t dst_off;
+  const int64_t* rows = nullptr;  // device row count: no more than *rows * row_bytes of the bytes are wanted
+  int64_t row_bytes = 0;
 };
 void pack_spans(const std::vector<CopySpan>& spans, void* dst, cudaStream_t s);
 

@@ -115,15 +115,28 @@ __device__ __forceinline__ SBDirect sb_direct(const SBDimDev& D) {
   return SBDirect{static_cast<int64_t>(lo ^ kSignBit), range};
 }
 
-// Key range of every dimension: blockIdx.y is the dimension.
+// Key range of every dimension: blockIdx.y is the dimension. A handful of
+// microseconds of latency: four keys in flight per thread, one pair of atomics
+// per block.
+constexpr int kSBRangeRows = 4 * kSBThreads;  // rows of a block's step
+
 __global__ void __launch_bounds__(kSBThreads) sb_range_kernel(const __grid_constant__ SBDimsParams p) {
+  __shared__ unsigned long long s_lo[kSBThreads / 32], s_hi[kSBThreads / 32];
   const SBDimDev& D = p.dims[blockIdx.y];
   unsigned long long lo = ~0ull, hi = 0ull;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < D.rows; r += stride) {
-    const unsigned long long u = static_cast<unsigned long long>(load_int(D.key, r)) ^ kSignBit;
-    lo = u < lo ? u : lo;
-    hi = u > hi ? u : hi;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kSBRangeRows;
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * kSBRangeRows; base < D.rows; base += stride) {
+    unsigned long long u[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {  // past the end: the last row again
+      const int64_t r = base + k * kSBThreads + threadIdx.x;
+      u[k] = static_cast<unsigned long long>(load_int(D.key, r < D.rows ? r : D.rows - 1)) ^ kSignBit;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      lo = u[k] < lo ? u[k] : lo;
+      hi = u[k] > hi ? u[k] : hi;
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -132,9 +145,20 @@ __global__ void __launch_bounds__(kSBThreads) sb_range_kernel(const __grid_const
     lo = a < lo ? a : lo;
     hi = b > hi ? b : hi;
   }
-  if ((threadIdx.x & 31) == 0 && lo <= hi) {
-    atomicMin(D.kmin_u, lo);
-    atomicMax(D.kmax_u, hi);
+  if ((threadIdx.x & 31) == 0) {
+    s_lo[threadIdx.x >> 5] = lo;
+    s_hi[threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kSBThreads / 32; ++w) {
+      lo = s_lo[w] < lo ? s_lo[w] : lo;
+      hi = s_hi[w] > hi ? s_hi[w] : hi;
+    }
+    if (lo <= hi) {
+      atomicMin(D.kmin_u, lo);
+      atomicMax(D.kmax_u, hi);
+    }
   }
 }
 
@@ -145,22 +169,28 @@ __global__ void __launch_bounds__(kSBThreads) sb_dims_kernel(const __grid_consta
     while (d + 1 < p.n_dims && i >= p.dims[d + 1].row_base) ++d;
     const SBDimDev& D = p.dims[d];
     const int64_t r = i - D.row_base;
+    // everything the row may need is asked for at once
     const int64_t v = load_int(D.filter, r);
+    const int64_t k = load_int(D.key, r);
+    const SBDirect dr = sb_direct(D);
+    int64_t gv[2] = {0, 0};
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (c < D.n_group) gv[c] = load_int(D.group[c], r);
     const int seg = sb_segment(p.segs[d], v);
     const uint64_t m = p.segs[d].cmask[seg];
     D.qmask[r] = m;
     if (m == 0) continue;
-    const int64_t k = load_int(D.key, r);
-    const SBDirect dr = sb_direct(D);
     if (dr.range != 0) {
       const uint64_t idx = static_cast<uint64_t>(k) - static_cast<uint64_t>(dr.kmin);  // < range by construction
-      if (atomicCAS(D.drow + idx, 0xFFFFFFFFu, static_cast<uint32_t>(r)) != 0xFFFFFFFFu) {
-        raise_status(p.st, GFPDB_EINVAL, 100 + d);  // repeated dimension key
-      } else {
-        D.dq[idx] = m;
-        D.dclass[idx] = static_cast<uint8_t>(seg);
-        for (int c = 0; c < D.n_group; ++c) D.dg[c][idx] = static_cast<int32_t>(load_int(D.group[c], r));
-      }
+      D.dq[idx] = m;
+      D.dclass[idx] = static_cast<uint8_t>(seg);
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (c < D.n_group) D.dg[c][idx] = static_cast<int32_t>(gv[c]);
+      // a key met before makes the batch an error, whatever was stored
+      if (atomicCAS(D.drow + idx, 0xFFFFFFFFu, static_cast<uint32_t>(r)) != 0xFFFFFFFFu)
+        raise_status(p.st, GFPDB_EINVAL, 100 + d);
       continue;
     }
     const uint64_t h = hash_key(k);
@@ -837,9 +867,12 @@ __global__ void __launch_bounds__(kSBFactThreads, 3) sb_fact_kernel(const __grid
 //      measures and the atomic adds.
 // Stacks, not rings: rows are taken from the top, in no particular order.
 //
-// 59,952,713 rows, 32 queries: 369 us before (class bytes for every dimension,
-// group values looked up and carried in step 1, about 124 instructions per 32
-// rows).
+// 59,952,713 rows, 32 queries: 266 us and 76 instructions per 32 rows (369 us
+// and 124 with class bytes for every dimension and the group values looked up
+// and carried in step 1), 69% of the measured copy bandwidth over the 1.24 GB
+// it moves; the wait left is for loads, with 32 warps an SM. Measured slower:
+// the next slice's keys read ahead (275 us, spills), and step (2) done in
+// place without a stack (321 us).
 constexpr int kSBDirectWarps = 16;
 constexpr int kSBDirectThreads = kSBDirectWarps * 32;
 constexpr int kSBDirectBlocks = 2;  // blocks an SM's registers hold
@@ -1249,6 +1282,64 @@ __global__ void __launch_bounds__(256) sb_final_kernel(const __grid_constant__ S
   }
 }
 
+// Both stages in one launch, a block per query, for group tables of up to
+// kSBOneLaunchSlots slots: a block counts the rows of the queries before its
+// own (the lower bits of every slot's touched word) along with its own, and
+// places its rows by a block scan in slot order, with no atomics. Larger
+// tables would be scanned by too few blocks. 512 slots and 32 queries: about
+// 4 us against 12 us for the two launches.
+constexpr uint64_t kSBOneLaunchSlots = 16384;
+constexpr int kSBFinalThreads = 512;
+
+__global__ void __launch_bounds__(kSBFinalThreads) sb_final_one_kernel(const __grid_constant__ SBFinalParams p) {
+  __shared__ int s_warp[kSBFinalThreads / 32 + 1];
+  const int q = blockIdx.x;
+  int before = 0, mine = 0;  // at most 64 * (kSBOneLaunchSlots + 1) rows in all
+  for (uint64_t s = threadIdx.x; s < p.slots; s += kSBFinalThreads) {
+    const unsigned long long t = p.touched[s];
+    before += __popcll(t & ((1ull << q) - 1));
+    mine += static_cast<int>(t >> q & 1ull);
+  }
+  int off, total;
+  (void)block_exclusive_sum<kSBFinalThreads>(before, &off, s_warp);
+  __syncthreads();
+  (void)block_exclusive_sum<kSBFinalThreads>(mine, &total, s_warp);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    p.qoff[q] = static_cast<unsigned long long>(off);
+    if (q == p.n_queries - 1) {
+      const unsigned long long all = static_cast<unsigned long long>(off + total);
+      for (int k = p.n_queries; k <= kSBMaxQueries; ++k) p.qoff[k] = all;
+      *p.counter = all;
+    }
+  }
+  int at = off;
+  for (uint64_t s0 = 0; s0 < p.slots; s0 += kSBFinalThreads) {
+    const uint64_t s = s0 + threadIdx.x;
+    const bool live = s < p.slots && (p.touched[s] >> q & 1ull) != 0;
+    int n;
+    const int64_t pos = at + block_exclusive_sum<kSBFinalThreads>(live ? 1 : 0, &n, s_warp);
+    __syncthreads();
+    at += n;
+    if (!live) continue;
+    const uint64_t key = s + 1 < p.slots ? p.gkeys[s] : kEmptySlot;
+    const unsigned long long* acc = p.gaccs + (static_cast<uint64_t>(q) * p.slots + s) * p.n_aggs;
+    unsigned long long a[kSBMaxAggsFact];
+#pragma unroll
+    for (int k = 0; k < kSBMaxAggsFact; ++k) a[k] = k < p.n_aggs ? acc[k] : 0ull;
+    p.out_q[pos] = q;
+    if (p.n_group == 1) {
+      static_cast<int32_t*>(p.out_g[0])[pos] = static_cast<int32_t>(static_cast<uint32_t>(key));
+    } else if (p.n_group == 2) {
+      static_cast<int32_t*>(p.out_g[0])[pos] = static_cast<int32_t>(static_cast<uint32_t>(key >> 32));
+      static_cast<int32_t*>(p.out_g[1])[pos] = static_cast<int32_t>(static_cast<uint32_t>(key));
+    }
+#pragma unroll
+    for (int k = 0; k < kSBMaxAggsFact; ++k)
+      if (k < p.n_aggs) p.out_a[k][pos] = static_cast<long long>(a[k]);
+  }
+}
+
 uint64_t pow2_at_least(uint64_t x) {
   uint64_t c = 64;
   while (c < x) c <<= 1;
@@ -1298,8 +1389,8 @@ struct StarBatchState {
   std::vector<std::string> fact_cols;
   SBDimsParams dims_params;
   SBFactParams fact_params;
-  BufferPtr tables_buf, masks_buf, dq_buf, drow_buf, dg_buf, dclass_buf, krange_buf, gkeys_buf, touched_buf, gaccs_buf, misc_buf, meta_buf,
-      out_q;
+  BufferPtr ones_buf, zeros_buf, masks_buf, dg_buf, meta_buf, out_q;
+  char* misc = nullptr;  // the status block and counts, in zeros_buf
   BufferPtr out_g[2], out_a[kMaxAggs];
   size_t fact_smem = 0;  // dynamic shared memory of a fact-stage block
   int mask_bytes = 8;    // query mask width in the fact stage (4: at most 32 queries)
@@ -1663,20 +1754,31 @@ void StarBatchState::prepare(cudaStream_t s) {
   gcap = pow2_at_least(static_cast<uint64_t>(2 * std::max<int64_t>(spec.groups_hint, 16)));
   const int na = static_cast<int>(spec.aggs.size());
   const int64_t gslots = static_cast<int64_t>(nq) * static_cast<int64_t>(gcap + 1);
-  tables_buf = make_buffer(table_words * 8, s);
-  dq_buf = make_buffer(table_words * 8, s);
-  drow_buf = make_buffer(table_words * 4, s);
+  // what a run clears lies in two regions, one of zeros and one of ones, each
+  // part at a multiple of 256 bytes
+  int64_t clear_bytes[2] = {0, 0};
+  auto part = [&](int ones, int64_t bytes) {
+    const int64_t at = clear_bytes[ones];
+    clear_bytes[ones] += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  // join tables, direct rows and classes, smallest keys and group keys empty
+  const int64_t tables_at = part(1, table_words * 8), drow_at = part(1, table_words * 4), dclass_at = part(1, table_words),
+                kmin_at = part(1, kSBMaxDims * 8), gkeys_at = part(1, static_cast<int64_t>(gcap) * 8);
+  static_assert(kSBNoRow == 0xFF, "classes are cleared with the bytes of the empty slots");
+  // direct masks, largest keys, touched words, accumulators; the status
+  // block, output count, then per-query counts, cursors and offsets
+  const int64_t dq_at = part(0, table_words * 8), kmax_at = part(0, kSBMaxDims * 8),
+                touched_at = part(0, static_cast<int64_t>(gcap + 1) * 8), gaccs_at = part(0, gslots * 8 * na),
+                misc_at = part(0, sizeof(DevStatus) + 64 + 8 * (3 * kSBMaxQueries + 1) + 16);
+  ones_buf = make_buffer(clear_bytes[1], s);
+  zeros_buf = make_buffer(clear_bytes[0], s);
+  char* const ones = ones_buf->as<char>();
+  char* const zeros = zeros_buf->as<char>();
   int64_t group_words = 0;
   for (int d = 0; d < nd; ++d) group_words += static_cast<int64_t>(dims_params.dims[d].mask + 1) * dims_params.dims[d].n_group;
   dg_buf = make_buffer(std::max<int64_t>(group_words, 1) * 4, s);
-  dclass_buf = make_buffer(table_words, s);
-  krange_buf = make_buffer(2 * kSBMaxDims * 8, s);
   masks_buf = make_buffer(std::max<int64_t>(mask_words, 1) * 8, s);
-  gkeys_buf = make_buffer(static_cast<int64_t>(gcap) * 8, s);
-  touched_buf = make_buffer(static_cast<int64_t>(gcap + 1) * 8, s);
-  gaccs_buf = make_buffer(gslots * 8 * na, s);
-  // status block, output count, then per-query counts, cursors and offsets
-  misc_buf = make_buffer(sizeof(DevStatus) + 64 + 8 * (3 * kSBMaxQueries + 1) + 16, s);
   meta_buf = make_buffer(static_cast<int64_t>(hcols.size() * sizeof(DevCol) + hbase.size() * 8 + hrows.size() * 8 +
                                               kSBMaxDims * sizeof(SBSegments)),
                          s);
@@ -1688,21 +1790,21 @@ void StarBatchState::prepare(cudaStream_t s) {
   int64_t toff = 0, moff = 0, goff = 0;
   for (int d = 0; d < nd; ++d) {
     SBDimDev& D = dims_params.dims[d];
-    D.slots = tables_buf->as<uint64_t>() + toff;
+    D.slots = reinterpret_cast<uint64_t*>(ones + tables_at) + toff;
     D.qmask = masks_buf->as<uint64_t>() + moff;
-    D.dq = dq_buf->as<uint64_t>() + toff;
-    D.drow = drow_buf->as<uint32_t>() + toff;
-    D.dclass = dclass_buf->as<uint8_t>() + toff;
+    D.dq = reinterpret_cast<uint64_t*>(zeros + dq_at) + toff;
+    D.drow = reinterpret_cast<uint32_t*>(ones + drow_at) + toff;
+    D.dclass = reinterpret_cast<uint8_t*>(ones + dclass_at) + toff;
     for (int c = 0; c < D.n_group; ++c) {
       D.dg[c] = dg_buf->as<int32_t>() + goff;
       goff += static_cast<int64_t>(D.mask + 1);
     }
-    D.kmin_u = krange_buf->as<unsigned long long>() + d;
-    D.kmax_u = krange_buf->as<unsigned long long>() + kSBMaxDims + d;
+    D.kmin_u = reinterpret_cast<unsigned long long*>(ones + kmin_at) + d;
+    D.kmax_u = reinterpret_cast<unsigned long long*>(zeros + kmax_at) + d;
     toff += static_cast<int64_t>(D.mask + 1);
     moff += D.rows;
   }
-  char* misc = misc_buf->as<char>();
+  misc = zeros + misc_at;
   DevStatus* st = reinterpret_cast<DevStatus*>(misc);
   dims_params.st = st;
   char* meta = meta_buf->as<char>();
@@ -1768,10 +1870,10 @@ void StarBatchState::prepare(cudaStream_t s) {
   fact_params.tile_base = dbase;
   fact_params.part_rows = drows;
   fact_params.n_tiles = n_tiles;
-  fact_params.gkeys = gkeys_buf->as<uint64_t>();
-  fact_params.gaccs = gaccs_buf->as<unsigned long long>();
+  fact_params.gkeys = reinterpret_cast<uint64_t*>(ones + gkeys_at);
+  fact_params.gaccs = reinterpret_cast<unsigned long long*>(zeros + gaccs_at);
   fact_params.gmask = gcap - 1;
-  fact_params.touched = touched_buf->as<unsigned long long>();
+  fact_params.touched = reinterpret_cast<unsigned long long*>(zeros + touched_at);
   fact_params.st = st;
   fact_params.segs = dsegs;
   for (int d = 0; d < nd; ++d) fact_params.dims[d] = dims_params.dims[d];
@@ -1891,24 +1993,15 @@ void StarBatchState::run(cudaStream_t s) {
       GF_CUDA(cudaEventRecord(events[2 + g], copy_stream));
     }
   }
-  // clear: join tables to empty, group keys to empty, accumulators / status / counters to zero
-  GF_CUDA(cudaMemsetAsync(tables_buf->data(), 0xFF, tables_buf->size(), s));
-  GF_CUDA(cudaMemsetAsync(dq_buf->data(), 0, dq_buf->size(), s));
-  GF_CUDA(cudaMemsetAsync(drow_buf->data(), 0xFF, drow_buf->size(), s));
-  GF_CUDA(cudaMemsetAsync(dclass_buf->data(), kSBNoRow, dclass_buf->size(), s));
-  GF_CUDA(cudaMemsetAsync(krange_buf->data(), 0xFF, kSBMaxDims * 8, s));  // minima
-  GF_CUDA(cudaMemsetAsync(krange_buf->as<char>() + kSBMaxDims * 8, 0, kSBMaxDims * 8, s));  // maxima
-  GF_CUDA(cudaMemsetAsync(gkeys_buf->data(), 0xFF, gkeys_buf->size(), s));
-  GF_CUDA(cudaMemsetAsync(touched_buf->data(), 0, touched_buf->size(), s));
-  GF_CUDA(cudaMemsetAsync(gaccs_buf->data(), 0, gaccs_buf->size(), s));
-  GF_CUDA(cudaMemsetAsync(misc_buf->data(), 0, misc_buf->size(), s));
+  const FillSpan clear[2] = {{ones_buf->data(), ones_buf->size(), 0xFF, 0}, {zeros_buf->data(), zeros_buf->size(), 0, 0}};
+  fill_regions(clear, 2, s);
   const int sms = num_sms();
   if (host) GF_CUDA(cudaStreamWaitEvent(s, events[1], 0));  // the dimensions have landed
   {
     int64_t max_rows = 1;
     for (int d = 0; d < dims_params.n_dims; ++d) max_rows = std::max<int64_t>(max_rows, dims_params.dims[d].rows);
-    int64_t bx = (max_rows + kSBThreads - 1) / kSBThreads;
-    if (bx > 64) bx = 64;
+    int64_t bx = (max_rows + kSBRangeRows - 1) / kSBRangeRows;
+    if (bx > sms * 2) bx = sms * 2;
     ProfScope prof("sb_range_kernel", s);
     sb_range_kernel<<<dim3(static_cast<unsigned>(bx), static_cast<unsigned>(dims_params.n_dims)), kSBThreads, 0, s>>>(
         dims_params);
@@ -1935,9 +2028,9 @@ void StarBatchState::run(cudaStream_t s) {
   {
     SBFinalParams fp;
     std::memset(&fp, 0, sizeof(fp));
-    fp.gkeys = gkeys_buf->as<uint64_t>();
-    fp.touched = touched_buf->as<unsigned long long>();
-    fp.gaccs = gaccs_buf->as<unsigned long long>();
+    fp.gkeys = fact_params.gkeys;
+    fp.touched = fact_params.touched;
+    fp.gaccs = fact_params.gaccs;
     fp.slots = gcap + 1;
     fp.n_queries = static_cast<int32_t>(spec.queries.size());
     fp.n_aggs = static_cast<int32_t>(spec.aggs.size());
@@ -1950,6 +2043,13 @@ void StarBatchState::run(cudaStream_t s) {
     fp.qcursor = qcursor;
     fp.qoff = qoff;
     const uint64_t total = fp.slots * static_cast<uint64_t>(fp.n_queries);
+    if (fp.slots <= kSBOneLaunchSlots + 1) {
+      ProfScope prof("sb_final_kernel", s);
+      sb_final_one_kernel<<<fp.n_queries, kSBFinalThreads, 0, s>>>(fp);
+      after_launch("sb_final_kernel");
+      prof.stop(static_cast<double>(total) * 8.0 * (1 + fp.n_aggs));
+      return;
+    }
     int64_t cblocks = static_cast<int64_t>((fp.slots + 255) / 256);
     if (cblocks > sms * 2) cblocks = sms * 2;
     sb_count_kernel<<<static_cast<int>(cblocks), 256, 0, s>>>(fp);
@@ -1991,10 +2091,10 @@ TupleSetPtr StarBatchState::result_view() const {
     fields.push_back(Field{spec.aggs[a].name, DType::Int64});
     cols.push_back(make_fixed_column(DType::Int64, out_cap, out_a[a]));
   }
-  return TupleSet::make_deferred(std::move(fields), std::move(cols), out_cap, misc_buf,
+  return TupleSet::make_deferred(std::move(fields), std::move(cols), out_cap, zeros_buf,
                                  reinterpret_cast<const int64_t*>(counter));
 }
 
-const DevStatus* StarBatchState::status() const { return misc_buf->as<DevStatus>(); }
+const DevStatus* StarBatchState::status() const { return reinterpret_cast<const DevStatus*>(misc); }
 
 }  // namespace gfpdb
