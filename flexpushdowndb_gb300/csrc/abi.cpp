@@ -267,7 +267,7 @@ BatchInputs import_batch_inputs(int32_t n_tables, const char* const* table_names
     const int32_t dt = arrays[i]->device_type;
     if (dt != ARROW_DEVICE_CUDA && dt != ARROW_DEVICE_CPU && dt != ARROW_DEVICE_CUDA_HOST)
       fail(GFPDB_EUNSUPPORTED, "unsupported ArrowDeviceArray device_type " + std::to_string(dt));
-    TupleSetPtr t = import_tupleset(schemas[i], arrays[i], s, false);
+    TupleSetPtr t = import_tupleset(schemas[i], arrays[i], s);
     if (dt != ARROW_DEVICE_CUDA) {
       in.pageable |= dt == ARROW_DEVICE_CPU;
       const ArrowArray& a = arrays[i]->array;
@@ -733,8 +733,25 @@ int32_t gfpdb_hashjoin_put_build(gfpdb_hashjoin* join, const ArrowSchema* schema
     require(join != nullptr, "null join");
     if (join->built) fail(GFPDB_EINVAL, "build input after finalize_build");
     ensure_device();
-    // The batch outlives this call, so device inputs are copied.
-    join->build.push_back(import_tupleset(schema, batch, as_stream(stream), true));
+    cudaStream_t s = as_stream(stream);
+    TupleSetPtr t = import_tupleset(schema, batch, s);
+    std::vector<Field> fields = t->fields();
+    // The join outlives the batch, so the columns it needs of a device batch
+    // are copied (a host batch came as a copy).
+    if (batch->device_type == ARROW_DEVICE_CUDA) {
+      std::vector<std::string> keep(join->build_keys);
+      keep.insert(keep.end(), join->needed.begin(), join->needed.end());
+      t = TupleSet::copy(*t, join->all_columns ? nullptr : &keep, s);
+    } else if (!join->all_columns) {
+      std::vector<std::string> keep;
+      for (auto& f : fields)
+        if (std::find(join->build_keys.begin(), join->build_keys.end(), f.name) != join->build_keys.end() ||
+            std::find(join->needed.begin(), join->needed.end(), f.name) != join->needed.end())
+          keep.push_back(f.name);
+      t = t->project(keep);  // the same columns whatever memory a batch came in
+    }
+    join->build.push_back(t);
+    join->build_fields.push_back(std::move(fields));
   });
 }
 
@@ -744,9 +761,18 @@ int32_t gfpdb_hashjoin_finalize_build(gfpdb_hashjoin* join, void* stream) {
     if (join->built) return;
     if (join->build.empty()) fail(GFPDB_EINVAL, "no build-side input");
     cudaStream_t s = as_stream(stream);
+    // batches agree on every column, the ones that are not kept included
+    const auto& first = join->build_fields[0];
+    for (auto& fields : join->build_fields) {
+      if (fields.size() != first.size()) fail(GFPDB_EINVAL, "concatenate: schema mismatch");
+      for (size_t i = 0; i < first.size(); ++i)
+        if (fields[i].type != first[i].type || fields[i].name != first[i].name)
+          fail(GFPDB_EINVAL, "concatenate: schema mismatch on column '" + first[i].name + "'");
+    }
     join->table = pop::build_join_table(TupleSet::concatenate(join->build, s), join->build_keys, join->load_factor, s,
                                         pop::join_kind_marks(static_cast<pop::JoinKind>(join->join_type)));
     join->build.clear();
+    join->build_fields.clear();
     join->built = true;
   });
 }
@@ -822,6 +848,7 @@ int32_t gfpdb_hashjoin_clear(gfpdb_hashjoin* join) {
   return guarded([&] {
     require(join != nullptr, "null argument");
     join->build.clear();
+    join->build_fields.clear();
     join->table = JoinTable{};
     join->probe_fields.clear();
     join->built = false;

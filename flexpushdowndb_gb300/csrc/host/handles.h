@@ -21,7 +21,8 @@ struct gfpdb_hashjoin {
   std::vector<std::string> needed;
   bool all_columns = true;
   double load_factor = 0.5;
-  std::vector<gfpdb::TupleSetPtr> build;
+  std::vector<gfpdb::TupleSetPtr> build;              // the columns the join needs of each batch
+  std::vector<std::vector<gfpdb::Field>> build_fields;  // every column of each
   gfpdb::JoinTable table;
   std::vector<gfpdb::Field> probe_fields;  // from the first probed batch
   bool built = false;

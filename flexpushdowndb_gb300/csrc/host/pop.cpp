@@ -105,7 +105,7 @@ class TableScanPOp : public PhysicalOp {
     // host tables: only the scanned columns come over, those named in
     // inPlaceColumns read in place when the table is page-locked
     TupleSetPtr ts = in.device ? in.device
-                               : import_tupleset(in.schema, in.array, ctx()->stream(), false,
+                               : import_tupleset(in.schema, in.array, ctx()->stream(),
                                                  columns_.empty() ? nullptr : &columns_, &in_place_);
     if (!columns_.empty()) ts = ts->project(columns_);
     const int64_t n = ts->num_rows();

@@ -213,6 +213,7 @@ TupleSetPtr TupleSet::concatenate(const std::vector<TupleSetPtr>& sets, cudaStre
     total += t->num_rows();
   }
   std::vector<ColumnPtr> cols;
+  std::vector<DeviceCopy> copies;
   for (size_t ci = 0; ci < fields.size(); ++ci) {
     DType t = fields[ci].type;
     if (t != DType::Utf8) {
@@ -221,8 +222,7 @@ TupleSetPtr TupleSet::concatenate(const std::vector<TupleSetPtr>& sets, cudaStre
       int64_t at = 0;
       for (auto& ts : sets) {
         const auto& c = ts->column(static_cast<int>(ci));
-        if (c->length > 0)
-          GF_CUDA(cudaMemcpyAsync(buf->as<char>() + at * w, c->data, c->length * w, cudaMemcpyDeviceToDevice, s));
+        if (c->length > 0) copies.push_back(DeviceCopy{buf->as<char>() + at * w, c->data, c->length * w});
         at += c->length;
       }
       cols.push_back(make_fixed_column(t, total, buf));
@@ -239,7 +239,30 @@ TupleSetPtr TupleSet::concatenate(const std::vector<TupleSetPtr>& sets, cudaStre
       cols.back() = with_validity(cols.back(), validity_concat(parts, total, s));
     }
   }
+  copy_device(copies, s);
   return make(fields, std::move(cols), total);
+}
+
+TupleSetPtr TupleSet::copy(const TupleSet& t, const std::vector<std::string>* wanted, cudaStream_t s) {
+  std::vector<Field> fields;
+  std::vector<ColumnPtr> cols;
+  std::vector<DeviceCopy> copies;
+  for (int i = 0; i < t.num_columns(); ++i) {
+    const Field& f = t.field(i);
+    if (wanted != nullptr && std::find(wanted->begin(), wanted->end(), f.name) == wanted->end()) continue;
+    const auto& c = t.column(i);
+    fields.push_back(f);
+    if (f.type == DType::Utf8) {
+      cols.push_back(concat_utf8({c.get()}, s));
+      continue;
+    }
+    const int64_t bytes = t.num_rows() * dtype_width(f.type);
+    auto buf = make_buffer(bytes, s);
+    if (bytes > 0) copies.push_back(DeviceCopy{buf->data(), c->data, bytes});
+    cols.push_back(make_fixed_column(f.type, t.num_rows(), buf));
+  }
+  copy_device(copies, s);
+  return make(std::move(fields), std::move(cols), t.num_rows());
 }
 
 // ---------------------------------------------------------------- import
@@ -272,7 +295,7 @@ const void* device_view_of_host(const void* p) {
 }
 
 TupleSetPtr import_tupleset(const ArrowSchema* schema, const ArrowDeviceArray* darr, cudaStream_t s,
-                            bool copy_device, const std::vector<std::string>* wanted,
+                            const std::vector<std::string>* wanted,
                             const std::vector<std::string>* in_place) {
   auto all_fields = import_schema(schema);
   auto listed = [](const std::vector<std::string>* v, const std::string& n) {
@@ -309,7 +332,7 @@ TupleSetPtr import_tupleset(const ArrowSchema* schema, const ArrowDeviceArray* d
       if (n > 0 && c->buffers[1] == nullptr) fail(GFPDB_EINVAL, "column '" + all_fields[i].name + "' has no values");
       int w = dtype_width(t);
       const char* src = static_cast<const char*>(c->buffers[1]) + off * w;
-      const bool zero_copy = host && !copy_device && (host_copy_mode() == 2 || listed(in_place, all_fields[i].name));
+      const bool zero_copy = host && (host_copy_mode() == 2 || listed(in_place, all_fields[i].name));
       const void* zc = zero_copy ? device_view_of_host(src) : nullptr;
       if (zc != nullptr) {
         // Zero-copy: kernels read the page-locked host column over the
@@ -317,13 +340,9 @@ TupleSetPtr import_tupleset(const ArrowSchema* schema, const ArrowDeviceArray* d
         auto buf = std::make_shared<DeviceBuffer>(const_cast<void*>(zc), n * w);
         cols.push_back(make_fixed_column(t, n, buf));
         copy_counters().in_place += n * w;
-      } else if (host || copy_device) {
+      } else if (host) {
         auto buf = make_buffer(n * w, s);
-        if (host) {
-          copy_h2d(buf->data(), src, n * w, s);
-        } else if (n > 0) {
-          GF_CUDA(cudaMemcpyAsync(buf->data(), src, n * w, cudaMemcpyDeviceToDevice, s));
-        }
+        copy_h2d(buf->data(), src, n * w, s);
         cols.push_back(make_fixed_column(t, n, buf));
       } else {
         auto buf = std::make_shared<DeviceBuffer>(const_cast<char*>(src), n * w);
@@ -349,14 +368,6 @@ TupleSetPtr import_tupleset(const ArrowSchema* schema, const ArrowDeviceArray* d
         // The rebased vector must outlive the async copy.
         sync(s);
         cols.push_back(make_utf8_column(n, ob, bb));
-      } else if (copy_device) {
-        Column tmp;
-        tmp.type = DType::Utf8;
-        tmp.length = n;
-        tmp.offsets = offs;
-        tmp.data = bytes;
-        std::vector<const Column*> parts{&tmp};
-        cols.push_back(concat_utf8(parts, s));
       } else {
         auto c2 = std::make_shared<Column>();
         c2->type = DType::Utf8;

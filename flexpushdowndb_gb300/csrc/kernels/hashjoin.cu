@@ -6,20 +6,23 @@
 // (fpdb-tuple/src/TupleSetIndex.cpp:44-88,238-245).
 //
 // Table: a power-of-two array of 64-bit slots, each (tag << 32 | build row),
-// all-ones when empty, filled with one 64-bit atomicCAS per build row and
-// linear probing. For 32-bit keys the tag is the key itself, so a probe
-// decides a match from the slot alone; for 64-bit keys the tag is the high
-// half of the hash and a tag hit is confirmed against the build key column.
-// Duplicate build keys occupy separate slots (multimap semantics). A build
-// may test up to four bloom filters on its key (a bloom selection folded
-// into the join) and leave out the rows that fail one. Probing:
-// a lane walks one probe row's run at a time, reading per step the aligned
-// four-slot group (one sector) that holds the run's next slot, and takes the
-// warp's next row as soon as its run ends. Matches collect per warp in
+// all-ones when empty, in groups of four (one 32-byte sector). A key goes into
+// an empty slot of the group that it hashes to, or of the first group after it
+// that has one, by 64-bit atomicCAS: a lookup reads whole groups until one has
+// an empty slot, and at load factor 0.5 about one key in seven goes past its
+// first (probing slot by slot from the one a key hashes to, one in four did).
+// For 32-bit keys the tag is the key itself, so a probe decides a match from
+// the slot alone; for 64-bit keys the tag is the high half of the hash and a
+// tag hit is confirmed against the build key column. Duplicate build keys
+// occupy separate slots (multimap semantics). A build may test up to four
+// bloom filters on its key (a bloom selection folded into the join) and leave
+// out the rows that fail one. Probing: a warp
+// makes 64 lookups a step, two in flight per lane; rows whose group was full
+// wait on the warp's stack and go on 64 at a time. Matches collect per warp in
 // shared memory and leave in runs of up to kStage pairs, each run taking its
 // output positions with one atomic on the shared cursor: the cursor is a
-// single address whose atomics the L2 serialises, so one atomic per warp
-// step held a 20M-row probe to the rate of that one address.
+// single address whose atomics the L2 serialises, so one atomic per warp step
+// held a 20M-row probe to the rate of that one address.
 #include "bloom.cuh"
 #include "common.cuh"
 #include "launch.h"
@@ -41,6 +44,45 @@ struct BuildFilters {
   int32_t n;
 };
 
+// The first slot a key with hash h may take: the start of its group.
+__device__ __forceinline__ uint64_t group_start(uint64_t h, uint64_t mask) { return h & mask & ~3ull; }
+
+// The slot value at index q (0..3) of a four-slot group held as two 16-byte
+// halves.
+__device__ __forceinline__ uint64_t group_slot(const ulonglong2& lo, const ulonglong2& hi, int q) {
+  const unsigned long long a = (q & 1) ? lo.y : lo.x;
+  const unsigned long long b = (q & 1) ? hi.y : hi.x;
+  return (q & 2) ? b : a;
+}
+
+// One group, in one 32-byte load: lanes read groups at random, so a load
+// costs the L1 about a cycle a lane, and two 16-byte halves cost it twice.
+__device__ __forceinline__ void load_group(const uint64_t* slots, uint64_t grp, ulonglong2& lo, ulonglong2& hi) {
+  asm("ld.global.nc.L1::no_allocate.v4.u64 {%0, %1, %2, %3}, [%4];"
+      : "=l"(lo.x), "=l"(lo.y), "=l"(hi.x), "=l"(hi.y)
+      : "l"(slots + grp));
+}
+
+// Bits of the group's slots that hold `tag`, and whether it has an empty slot
+// (the run ends here).
+__device__ __forceinline__ uint32_t group_matches(const ulonglong2& lo, const ulonglong2& hi, uint32_t tag, bool* ends) {
+  uint32_t eb = 0, tb = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint64_t v = group_slot(lo, hi, q);
+    if (static_cast<uint32_t>(v) == 0xFFFFFFFFu)  // no row has this index: an empty slot
+      eb |= 1u << q;
+    else if (static_cast<uint32_t>(v >> 32) == tag)
+      tb |= 1u << q;
+  }
+  *ends = eb != 0;
+  return tb;
+}
+
+// A row tries its group's slots from the one that other bits of its hash say,
+// in turn: rows of one group mostly begin at different slots, so most rows
+// need one compare-and-swap (a read of the group first, to pick an empty slot,
+// made the build of 2M rows 72 us instead of 60).
 __global__ void __launch_bounds__(256)
     join_build_kernel(DevCol key, int64_t cap, const int64_t* n_dev, uint64_t* __restrict__ slots, uint64_t mask,
                       int key32, DevStatus* st, BuildFilters bf) {
@@ -73,9 +115,11 @@ __global__ void __launch_bounds__(256)
     const uint64_t h = hash_key(k);
     const uint32_t tag = key32 ? static_cast<uint32_t>(k) : static_cast<uint32_t>(h >> 32);
     const uint64_t packed = (static_cast<uint64_t>(tag) << 32) | static_cast<uint32_t>(r);
-    uint64_t slot = h & mask;
-    uint64_t probe = 0;
+    const uint64_t turn = h >> 62;  // the same for equal keys: the later one meets the earlier
+    uint64_t grp = group_start(h, mask);
+    uint64_t probe = 0;  // slots passed
     for (; probe <= mask; ++probe) {
+      const uint64_t slot = grp + ((probe + turn) & 3);
       const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long*>(slots + slot),
                                                static_cast<unsigned long long>(kEmptySlot),
                                                static_cast<unsigned long long>(packed));
@@ -85,7 +129,7 @@ __global__ void __launch_bounds__(256)
       if (static_cast<uint32_t>(old >> 32) == tag &&
           (key32 || load_int(key, static_cast<uint32_t>(old)) == k))
         dup = true;
-      slot = (slot + 1) & mask;
+      if ((probe & 3) == 3) grp = (grp + 4) & mask;
     }
     if (probe > mask) raise_status(st, GFPDB_ENOMEM, 10);  // table full: cannot happen at load <= 1
     if (static_cast<int64_t>(probe) > my_max) my_max = static_cast<int64_t>(probe);
@@ -104,23 +148,12 @@ __global__ void __launch_bounds__(256)
 // memory, flushed to the output when fewer than 32 free places remain (one
 // staging round adds at most 32) and once at the end.
 constexpr int kProbeWarps = 8;  // 256-thread CTAs
-constexpr int kStage = 512;     // staged pairs per warp
+constexpr int kStage = 256;     // staged pairs per warp
 
 struct PairStage {
-  int32_t* p;
-  int32_t* b;
-  int n;  // staged pairs; the same in every lane
+  int2* pair;  // (probe row, build row)
+  int n;       // staged pairs; the same in every lane
 };
-
-__device__ __forceinline__ void stage_pairs(PairStage& sg, bool emit, int lane, int32_t prow, int32_t brow) {
-  const uint32_t em = __ballot_sync(0xffffffffu, emit);
-  if (emit) {
-    const int at = sg.n + __popc(em & ((1u << lane) - 1u));
-    sg.p[at] = prow;
-    sg.b[at] = brow;
-  }
-  sg.n += __popc(em);
-}
 
 // Claims sg.n output positions with one atomic and hands the stage to
 // write(first position, stage, lane).
@@ -135,14 +168,6 @@ __device__ __forceinline__ void flush_pairs(PairStage& sg, unsigned long long* c
   sg.n = 0;
 }
 
-// The slot value at index q (0..3) of a four-slot group held as two 16-byte
-// halves.
-__device__ __forceinline__ uint64_t group_slot(const ulonglong2& lo, const ulonglong2& hi, int q) {
-  const unsigned long long a = (q & 1) ? lo.y : lo.x;
-  const unsigned long long b = (q & 1) ? hi.y : hi.x;
-  return (q & 2) ? b : a;
-}
-
 // A probe key, streamed (evict-first): each probe row is read once, and the
 // L2 is better spent on the table.
 __device__ __forceinline__ int64_t load_key_stream(const DevCol& c, int64_t row) {
@@ -152,128 +177,125 @@ __device__ __forceinline__ int64_t load_key_stream(const DevCol& c, int64_t row)
 
 // The probe loop shared by the pair and the materialising probe.
 //
-// Each warp owns a contiguous range of probe rows and each lane walks one
-// row's run at a time; a lane whose run has ended takes the warp's next row
-// before the next step, so lanes do not sit idle behind the longest run of
-// a fixed tile. The keys of the next 128 rows of the range wait in four
-// registers per lane (a ring of 32-row batches, each loaded three batches
-// ahead of its use), so a new row's key comes from a shuffle rather than a
-// dependent load, and a step's only wait is its table read.
+// Each warp owns a contiguous range of probe rows and takes 64 lookups a
+// step, two per lane in flight: 64 new rows (their keys loaded a step ahead),
+// or, once 64 are waiting, rows whose group was full and whose run goes on.
+// Most rows are decided by their first group; the others wait on a stack with
+// the group to read next, so no lane idles behind another's longer run.
 //
-// A step reads the aligned group of four slots (one 32-byte sector) that
-// holds the run's next slot: the run is the same linear probe as the
-// build's, in about a quarter of the steps. In a run's first group the
-// slots before its start slot are not part of it; an empty slot at or
-// after the start ends the run.
+// 20M rows against 2M keys, half of them matching, four columns out: 328 us
+// (374 us with one lookup per lane at a time and two 16-byte reads a group).
+// Neither issue (50%) nor DRAM (20%) holds it: a request a lane from the L1
+// to the L2 for each lookup and each build value, at half that path's peak.
+constexpr int kProbeFlight = 2;  // lookups in flight per lane
+constexpr int kProbeStep = 32 * kProbeFlight;
+
 template <class Write>
 __device__ __forceinline__ void probe_rows(const DevCol& pkey, int64_t n, const uint64_t* __restrict__ slots,
                                            uint64_t mask, const DevCol& bkey, int key32, unsigned long long* cursor,
                                            Write& write) {
-  __shared__ int32_t s_p[kProbeWarps][kStage], s_b[kProbeWarps][kStage];
-  const int lane = threadIdx.x & 31;
+  __shared__ int2 s_pair[kProbeWarps][kStage];
+  __shared__ uint2 s_wait[kProbeWarps][2 * kProbeStep];  // (row, next group's first slot / 4: fewer than 2^34 slots)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t below = (1u << lane) - 1u;
-  PairStage sg{s_p[threadIdx.x >> 5], s_b[threadIdx.x >> 5], 0};
+  PairStage sg{s_pair[warp], 0};
+  int waiting = 0;  // the same in every lane
   const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const int64_t per = ((n + n_warps - 1) / n_warps + 31) & ~static_cast<int64_t>(31);
-  const int64_t begin = warp_global * per < n ? warp_global * per : n;
-  const int64_t end = begin + per < n ? begin + per : n;
-  // A table always keeps empty slots (load factor <= 0.9), so every run
-  // ends within one pass over the groups; the bound only guards the loop.
-  const uint64_t n_groups = (mask + 1) >> 2;
+  const int64_t per = ((n + n_warps - 1) / n_warps + kProbeStep - 1) / kProbeStep * kProbeStep;
+  int64_t base = warp_global * per < n ? warp_global * per : n;
+  const int64_t end = base + per < n ? base + per : n;
 
-  int64_t ring[4];  // keys of rows ring_base + 32 * b + lane
-  int64_t ring_base = begin;
+  int64_t ahead[kProbeFlight];  // keys of rows base + 32 * u + lane
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int64_t r = begin + 32 * b + lane;
-    ring[b] = r < end ? load_key_stream(pkey, r) : 0;
-  }
-  int taken = 0;  // rows of the ring's first batch already handed out (< 32 between steps)
-
-  bool active = false;
-  int32_t row = 0;
-  int64_t k = 0;
-  uint32_t tag = 0, valid = 0;
-  uint64_t grp = 0, steps = 0;
-  while (true) {
-    // Hand the next rows of the range to the lanes without one, in lane
-    // order: the lane of rank i among them takes row ring_base + taken + i.
-    const uint32_t idle = __ballot_sync(0xffffffffu, !active);
-    const int64_t left = end - (ring_base + taken);
-    if (idle == 0xffffffffu && left <= 0) break;
-    if (idle != 0 && left > 0) {
-      const int idx = taken + __popc(idle & below);  // < 64: in the ring's first two batches
-      const int64_t v0 = __shfl_sync(0xffffffffu, ring[0], idx & 31);
-      const int64_t v1 = __shfl_sync(0xffffffffu, ring[1], idx & 31);
-      if (!active && idx - taken < left) {
-        active = true;
-        row = static_cast<int32_t>(ring_base + idx);
-        k = idx < 32 ? v0 : v1;
-        const uint64_t h = hash_key(k);
-        tag = key32 ? static_cast<uint32_t>(k) : static_cast<uint32_t>(h >> 32);
-        const uint64_t slot = h & mask;
-        grp = slot & ~3ull;
-        valid = (0xFu << (slot & 3)) & 0xFu;
-        steps = 0;
+  for (int u = 0; u < kProbeFlight; ++u)
+    ahead[u] = base + 32 * u + lane < end ? load_key_stream(pkey, base + 32 * u + lane) : 0;
+  while (base < end || waiting > 0) {
+    int32_t row[kProbeFlight];
+    int64_t key[kProbeFlight];
+    uint64_t grp[kProbeFlight];
+    uint32_t tag[kProbeFlight];
+    bool active[kProbeFlight];
+    const bool resume = waiting >= kProbeStep || base >= end;
+    if (resume) {
+      const int take = waiting < kProbeStep ? waiting : kProbeStep;
+      waiting -= take;
+#pragma unroll
+      for (int u = 0; u < kProbeFlight; ++u) {
+        const int i = 32 * u + lane;
+        active[u] = i < take;
+        const uint2 w = active[u] ? s_wait[warp][waiting + i] : make_uint2(0, 0);
+        row[u] = static_cast<int32_t>(w.x);
+        grp[u] = static_cast<uint64_t>(w.y) << 2;
+        key[u] = active[u] ? load_int(pkey, row[u]) : 0;
       }
-      const int handed = static_cast<int64_t>(__popc(idle)) < left ? __popc(idle) : static_cast<int>(left);
-      taken += handed;
-      if (taken >= 32) {  // the first batch is used up: shift, fetch the batch after the last
-        ring[0] = ring[1];
-        ring[1] = ring[2];
-        ring[2] = ring[3];
-        const int64_t r = ring_base + 128 + lane;
-        ring[3] = r < end ? load_key_stream(pkey, r) : 0;
-        ring_base += 32;
-        taken -= 32;
+      __syncwarp();  // read before this step queues again
+    } else {
+#pragma unroll
+      for (int u = 0; u < kProbeFlight; ++u) {
+        active[u] = base + 32 * u + lane < end;
+        row[u] = static_cast<int32_t>(base + 32 * u + lane);
+        key[u] = ahead[u];
+      }
+      base += kProbeStep;
+#pragma unroll
+      for (int u = 0; u < kProbeFlight; ++u)
+        if (base + 32 * u + lane < end) ahead[u] = load_key_stream(pkey, base + 32 * u + lane);
+    }
+    uint64_t start[kProbeFlight];
+    ulonglong2 lo[kProbeFlight], hi[kProbeFlight];
+#pragma unroll
+    for (int u = 0; u < kProbeFlight; ++u) {
+      const uint64_t h = hash_key(key[u]);
+      tag[u] = key32 ? static_cast<uint32_t>(key[u]) : static_cast<uint32_t>(h >> 32);
+      start[u] = group_start(h, mask);
+      if (!resume) grp[u] = start[u];
+      if (active[u]) {
+        load_group(slots, grp[u], lo[u], hi[u]);
       }
     }
-
-    uint32_t mm = 0;  // matching slots of this step's group that lie on the run
-    ulonglong2 lo{0, 0}, hi{0, 0};
-    if (active) {
-      const ulonglong2* g = reinterpret_cast<const ulonglong2*>(slots + grp);
-      lo = __ldg(g);
-      hi = __ldg(g + 1);
-      uint32_t eb = 0, tb = 0;
+    uint32_t mm[kProbeFlight];  // matching slots of the groups
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint64_t v = group_slot(lo, hi, q);
-        if (v == kEmptySlot)
-          eb |= 1u << q;
-        else if (static_cast<uint32_t>(v >> 32) == tag)
-          tb |= 1u << q;
-      }
-      eb &= valid;
-      const int stop = eb ? __ffs(eb) - 1 : 4;
-      mm = tb & valid & ((1u << stop) - 1u);
+    for (int u = 0; u < kProbeFlight; ++u) {
+      bool ends = true;
+      mm[u] = active[u] ? group_matches(lo[u], hi[u], tag[u], &ends) : 0u;
       if (!key32) {
-        for (uint32_t t = mm; t != 0; t &= t - 1) {
-          const int q = __ffs(t) - 1;
-          if (load_int(bkey, static_cast<int32_t>(static_cast<uint32_t>(group_slot(lo, hi, q)))) != k)
-            mm &= ~(1u << q);
+        for (uint32_t t = mm[u]; t != 0; t &= t - 1) {
+          const int q = __ffs(static_cast<int>(t)) - 1;
+          if (load_int(bkey, static_cast<int32_t>(static_cast<uint32_t>(group_slot(lo[u], hi[u], q)))) != key[u])
+            mm[u] &= ~(1u << q);
         }
       }
-      if (eb != 0 || ++steps > n_groups) {
-        active = false;
-      } else {
-        grp = (grp + 4) & mask;
-        valid = 0xFu;
+      // A table always keeps empty slots (load factor <= 0.9), so every run
+      // ends; coming round to its start only guards the loop.
+      const uint64_t next = (grp[u] + 4) & mask;
+      const bool on = !ends && next != start[u];
+      const uint32_t cont = __ballot_sync(0xffffffffu, on);
+      if (on) {
+        const int at = waiting + __popc(cont & below);  // fewer than kProbeStep waited, at most as many join
+        s_wait[warp][at] = make_uint2(static_cast<uint32_t>(row[u]), static_cast<uint32_t>(next >> 2));
       }
+      waiting += __popc(cont);
     }
-    // One staged match per lane per round; a group can hold several copies
-    // of a repeated build key.
-    while (__any_sync(0xffffffffu, mm != 0)) {
-      int32_t brow = 0;
-      const bool emit = mm != 0;
-      if (emit) {
-        brow = static_cast<int32_t>(static_cast<uint32_t>(group_slot(lo, hi, __ffs(mm) - 1)));
-        mm &= mm - 1;
+    // One match per lookup and round (a group can hold several copies of a
+    // repeated build key).
+    bool more;
+    do {
+      if (sg.n > kStage - kProbeStep) flush_pairs(sg, cursor, lane, write);
+      more = false;
+#pragma unroll
+      for (int u = 0; u < kProbeFlight; ++u) {
+        const uint32_t em = __ballot_sync(0xffffffffu, mm[u] != 0);
+        if (mm[u] != 0) {
+          const uint64_t v = group_slot(lo[u], hi[u], __ffs(static_cast<int>(mm[u])) - 1);
+          s_pair[warp][sg.n + __popc(em & below)] = make_int2(row[u], static_cast<int32_t>(static_cast<uint32_t>(v)));
+          mm[u] &= mm[u] - 1;
+          more = more || mm[u] != 0;
+        }
+        sg.n += __popc(em);
       }
-      stage_pairs(sg, emit, lane, row, brow);
-      if (sg.n > kStage - 32) flush_pairs(sg, cursor, lane, write);
-    }
+    } while (__any_sync(0xffffffffu, more));
+    __syncwarp();  // what this step queued is seen by every lane
   }
   if (sg.n > 0) flush_pairs(sg, cursor, lane, write);
 }
@@ -286,8 +308,8 @@ __global__ void __launch_bounds__(256)
   auto write = [&](int64_t at, const PairStage& sg, int lane) {
     for (int i = lane; i < sg.n; i += 32)
       if (at + i < cap) {
-        __stcs(out_p + at + i, sg.p[i]);
-        __stcs(out_b + at + i, sg.b[i]);
+        __stcs(out_p + at + i, sg.pair[i].x);
+        __stcs(out_b + at + i, sg.pair[i].y);
       }
   };
   probe_rows(pkey, n, slots, mask, bkey, key32, reinterpret_cast<unsigned long long*>(&st->value), write);
@@ -320,38 +342,42 @@ struct JoinEmitParams {
 // which stream (evict-first): the output is written once and read by later
 // kernels, while the L2 should keep the hash table and the build columns
 // that the probes and gathers revisit.
-template <class T>
+// kStep: words from one row's index to the next.
+template <int kStep, class T>
 __device__ __forceinline__ void copy_staged(const T* __restrict__ src, T* __restrict__ dst, const int32_t* idx,
                                             int n, int64_t at, int64_t cap, int lane, bool stream_src) {
   constexpr int kU = 4;
+  if (at >= cap) return;
+  if (n > cap - at) n = static_cast<int>(cap - at);
+  dst += at;
   for (int i0 = 0; i0 < n; i0 += 32 * kU) {
     T v[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int i = i0 + u * 32 + lane;
-      if (i < n) v[u] = stream_src ? __ldcs(src + idx[i]) : __ldg(src + idx[i]);
+      if (i < n) v[u] = stream_src ? __ldcs(src + idx[i * kStep]) : __ldg(src + idx[i * kStep]);
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int i = i0 + u * 32 + lane;
-      if (i < n && at + i < cap) __stcs(dst + at + i, v[u]);
+      if (i < n) __stcs(dst + i, v[u]);
     }
   }
 }
 
-__global__ void __launch_bounds__(256) join_probe_emit_kernel(const __grid_constant__ JoinEmitParams p) {
+__global__ void __launch_bounds__(256, 4) join_probe_emit_kernel(const __grid_constant__ JoinEmitParams p) {
   const int64_t n = clamp_rows(p.n_dev, p.n_cap);
   auto write = [&](int64_t at, const PairStage& sg, int lane) {
     for (int c = 0; c < p.n_out; ++c) {
-      const int32_t* idx = p.from_build[c] ? sg.b : sg.p;
+      const int32_t* idx = &sg.pair[0].x + (p.from_build[c] ? 1 : 0);
       // probe rows are read once (streamed); build rows are revisited
       const bool stream_src = !p.from_build[c];
       if (p.width[c] == 8)
-        copy_staged(static_cast<const long long*>(p.src[c]), static_cast<long long*>(p.dst[c]), idx, sg.n, at, p.cap,
-                    lane, stream_src);
+        copy_staged<2>(static_cast<const long long*>(p.src[c]), static_cast<long long*>(p.dst[c]), idx, sg.n, at, p.cap,
+                       lane, stream_src);
       else
-        copy_staged(static_cast<const int*>(p.src[c]), static_cast<int*>(p.dst[c]), idx, sg.n, at, p.cap, lane,
-                    stream_src);
+        copy_staged<2>(static_cast<const int*>(p.src[c]), static_cast<int*>(p.dst[c]), idx, sg.n, at, p.cap, lane,
+                       stream_src);
     }
   };
   probe_rows(p.pkey, n, p.slots, p.mask, p.bkey, p.key32, reinterpret_cast<unsigned long long*>(&p.st->value), write);
@@ -419,10 +445,10 @@ __global__ void __launch_bounds__(256) join_chain_kernel(const __grid_constant__
       const int32_t* idx = s_rows[warp][p.from[c]];
       const bool stream_src = p.from[c] == 0;  // the input row: read once
       if (p.width[c] == 8)
-        copy_staged(static_cast<const long long*>(p.src[c]), static_cast<long long*>(p.dst[c]), idx, staged,
+        copy_staged<1>(static_cast<const long long*>(p.src[c]), static_cast<long long*>(p.dst[c]), idx, staged,
                     static_cast<int64_t>(at), p.cap, lane, stream_src);
       else
-        copy_staged(static_cast<const int*>(p.src[c]), static_cast<int*>(p.dst[c]), idx, staged,
+        copy_staged<1>(static_cast<const int*>(p.src[c]), static_cast<int*>(p.dst[c]), idx, staged,
                     static_cast<int64_t>(at), p.cap, lane, stream_src);
     }
     __syncwarp();
@@ -446,7 +472,7 @@ __global__ void __launch_bounds__(256) join_chain_kernel(const __grid_constant__
       const uint64_t h = hash_key(k);
       key[l] = k;
       tag[l] = L.key32 ? static_cast<uint32_t>(k) : static_cast<uint32_t>(h >> 32);
-      slot[l] = h & L.mask;
+      slot[l] = group_start(h, L.mask);
       steps[l] = 0;
       ended &= ~(1u << l);
     };
@@ -458,12 +484,12 @@ __global__ void __launch_bounds__(256) join_chain_kernel(const __grid_constant__
         bool run_over = (ended >> lvl & 1u) != 0;
         if (!run_over) {
           // the aligned four-slot group (one sector) holding the run's next
-          // slot: the first match at or after it that precedes an empty slot
+          // slot: the first match at or after it
           const uint64_t s0 = slot[lvl];
           const int q0 = static_cast<int>(s0 & 3);
           const uint64_t g = s0 & ~3ull;
-          const ulonglong2* gp = reinterpret_cast<const ulonglong2*>(L.slots + g);
-          const ulonglong2 lo = __ldg(gp), hi = __ldg(gp + 1);
+          ulonglong2 lo, hi;
+          load_group(L.slots, g, lo, hi);
           uint32_t eb = 0, tb = 0;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -473,10 +499,7 @@ __global__ void __launch_bounds__(256) join_chain_kernel(const __grid_constant__
             else if (static_cast<uint32_t>(v >> 32) == tag[lvl])
               tb |= 1u << q;
           }
-          const uint32_t from = (0xFu << q0) & 0xFu;
-          eb &= from;
-          const int stop = eb ? __ffs(eb) - 1 : 4;
-          tb &= from & ((1u << stop) - 1u);
+          tb &= (0xFu << q0) & 0xFu;  // the slots not yet looked at
           int m = -1;
           int32_t brow = 0;
           for (; tb != 0; tb &= tb - 1) {
@@ -491,9 +514,9 @@ __global__ void __launch_bounds__(256) join_chain_kernel(const __grid_constant__
           steps[lvl] += static_cast<uint64_t>(4 - q0);
           if (m >= 0) {
             slot[lvl] = (g + m + 1) & L.mask;
-            // the run ends in this group when an empty slot follows the
-            // match with no other candidate (a repeated key) before it; tb
-            // still holds the match and the candidates after it
+            // the run ends in this group when it has an empty slot and no
+            // other candidate (a repeated key); tb still holds the match and
+            // the candidates after it
             if (eb != 0 && (tb >> (m + 1)) == 0) ended |= 1u << lvl;
             rows[lvl + 1] = brow;
             if (lvl == p.n_levels - 1) {
@@ -579,7 +602,7 @@ int probe_grid(Kernel kernel, int64_t n) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 256, 0) != cudaSuccess || b < 1) b = 4;
     return b;
   }();
-  return grid_for(n, per_sm, kProbeWarps * 256);  // at least 256 rows per warp
+  return grid_for(n, per_sm, kProbeWarps * 2 * kProbeStep);
 }
 
 }  // namespace
@@ -892,16 +915,18 @@ __device__ __forceinline__ int walk_matches(const MatchParams& p, int64_t r, F&&
   const int64_t k = load_int(p.pkey, r);
   const uint64_t h = hash_key(k);
   const uint32_t tag = p.key32 ? static_cast<uint32_t>(k) : static_cast<uint32_t>(h >> 32);
-  uint64_t slot = h & p.mask;
+  uint64_t grp = group_start(h, p.mask);
   int m = 0;
-  for (uint64_t i = 0; i <= p.mask; ++i, slot = (slot + 1) & p.mask) {
-    const uint64_t s = __ldg(p.slots + slot);
-    if (s == kEmptySlot) break;
-    if (static_cast<uint32_t>(s >> 32) != tag) continue;
-    const uint32_t b = static_cast<uint32_t>(s);
-    if (!p.key32 && load_int(p.bkey, b) != k) continue;
-    f(b, m);
-    ++m;
+  bool ends = false;
+  for (uint64_t i = 0; i <= p.mask && !ends; i += 4, grp = (grp + 4) & p.mask) {
+    ulonglong2 lo, hi;
+    load_group(p.slots, grp, lo, hi);
+    for (uint32_t t = group_matches(lo, hi, tag, &ends); t != 0; t &= t - 1) {
+      const uint32_t b = static_cast<uint32_t>(group_slot(lo, hi, __ffs(static_cast<int>(t)) - 1));
+      if (!p.key32 && load_int(p.bkey, b) != k) continue;
+      f(b, m);
+      ++m;
+    }
   }
   return m;
 }

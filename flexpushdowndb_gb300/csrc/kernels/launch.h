@@ -48,6 +48,14 @@ struct CopySpan {
 };
 void pack_spans(const std::vector<CopySpan>& spans, void* dst, cudaStream_t s);
 
+// Copies between device buffers, all of them in one launch per 64.
+struct DeviceCopy {
+  void* dst;
+  const void* src;
+  int64_t bytes;
+};
+void copy_device(const std::vector<DeviceCopy>& copies, cudaStream_t s);
+
 // Fill up to two regions (16-byte aligned, sizes multiples of 16) with one
 // byte value each, in one kernel launch.
 struct FillSpan {
