@@ -12,25 +12,23 @@
 // key lands in does not change any query's result, only that equal keys land
 // in the same slot.
 //
-// Three launches, all stable and without global atomics, over tiles of
-// 512 rows per warp of a block (4096 rows for 8 warps):
-//   shuffle_count_kernel   the slots of a tile's rows (several key loads in
-//                          flight per thread), counted by shared-memory
-//                          atomics; the counts land slot-major in a
-//                          [slots][tiles] matrix;
-//   scan_i32_kernel        one exclusive prefix sum over the matrix gives each
-//                          (slot, tile) its first output row;
-//   shuffle_scatter_kernel the tile's rows ranked in shared memory (a lane's
-//                          peers with the same slot from one ballot per slot
-//                          bit): per-warp counts of each slot, scanned across warps and
-//                          slots, give every row its place in the tile's
-//                          slot order (input order kept); then each column
-//                          leaves in that order, consecutive threads writing
-//                          consecutive rows of one slot's run, so the writes
-//                          are whole sectors rather than one value per
-//                          sector. utf8 columns are gathered afterwards
-//                          through the inverse permutation the same kernel
-//                          writes.
+// Three launches, all stable and without global atomics, over tiles of 256
+// rows per warp of a block (4096 rows for 16 warps, 2048 for 8):
+//   shuffle_count_kernel   hashes the tile's rows (several key loads in flight
+//                          per thread), keeps each row's slot in 16 bits and
+//                          counts the slots by shared-memory atomics; the
+//                          counts land slot-major in a [slots][tiles] matrix;
+//   shuffle_scan_kernel    one block per slot: its tiles' counts become
+//                          offsets within the slot, and the slot's total;
+//   shuffle_scatter_kernel ranks the tile's rows (a lane's peers with the same
+//                          slot from one ballot per slot bit) and gives every
+//                          row its place in the tile's slot order (input order
+//                          kept); then each column is read in row order, put
+//                          into shared memory in slot order and written from
+//                          there, so reads are whole lines and writes whole
+//                          sectors of one slot's run. utf8 columns are
+//                          gathered afterwards through the inverse permutation
+//                          that the same kernel writes.
 #include <algorithm>
 #include <cstring>
 
@@ -41,8 +39,9 @@ namespace gfpdb {
 namespace {
 
 constexpr int kShufMaxFixed = 24;   // fixed-width columns scattered per launch
-constexpr int kShufRowsPerWarp = 512;
-constexpr int kShufUnroll = 4;      // key loads in flight per thread
+constexpr int kShufRowsPerWarp = 256;
+constexpr int kShufPerLane = kShufRowsPerWarp / 32;
+constexpr int kShufUnroll = 8;      // key loads in flight per thread
 
 struct ShufKeys {
   DevCol keys[kMaxKeyColumns];
@@ -50,7 +49,7 @@ struct ShufKeys {
   uint32_t slots;
   int64_t n;       // rows
   int32_t tile;    // rows per block: warps * kShufRowsPerWarp
-  int32_t slot_bits;  // bits of a slot number (0 for one slot)
+  int32_t pad;
   int64_t ntiles;
 };
 
@@ -60,8 +59,10 @@ struct ShufScatter {
   int8_t width[kShufMaxFixed];
   int32_t n_fixed;
   int32_t pad;
-  const int32_t* starts;  // scanned counts, [slots][ntiles]
-  int32_t* inverse;       // inverse[out row] = input row (utf8 columns), or null
+  const uint16_t* row_slot;  // slot of each row
+  const int32_t* starts;     // [slots][ntiles] rows of the slot in earlier tiles
+  const int32_t* totals;     // [slots] rows of the slot
+  int32_t* inverse;          // inverse[out row] = input row (utf8 columns), or null
 };
 
 __device__ __forceinline__ uint32_t slot_of(uint64_t h, uint32_t slots) {
@@ -69,204 +70,228 @@ __device__ __forceinline__ uint32_t slot_of(uint64_t h, uint32_t slots) {
   return static_cast<uint32_t>(((g >> 32) * slots) >> 32);
 }
 
-// Slots of rows [begin, begin + rows) into out[0, rows): each thread takes
-// rows tid, tid + blockDim, ..., kShufUnroll of them per round.
-__device__ __forceinline__ void tile_slots(const ShufKeys& p, int64_t begin, int rows, uint16_t* out) {
-  if (p.n_keys == 1 && p.keys[0].type != CT_UTF8) {  // one integer key: the loads first, then the hashes
-    for (int base = 0; base < rows; base += kShufUnroll * blockDim.x) {
-      int64_t v[kShufUnroll];
-#pragma unroll
-      for (int u = 0; u < kShufUnroll; ++u) {
-        const int i = base + u * blockDim.x + threadIdx.x;
-        v[u] = i < rows ? load_int(p.keys[0], begin + i) : 0;
-      }
-#pragma unroll
-      for (int u = 0; u < kShufUnroll; ++u) {
-        const int i = base + u * blockDim.x + threadIdx.x;
-        if (i < rows) out[i] = static_cast<uint16_t>(slot_of(row_key_combine(kRowKeySeed, hash_key(v[u])), p.slots));
-      }
-    }
-    return;
-  }
-  for (int base = 0; base < rows; base += kShufUnroll * blockDim.x) {
-    uint64_t h[kShufUnroll];
-#pragma unroll
-    for (int u = 0; u < kShufUnroll; ++u) {
-      const int i = base + u * blockDim.x + threadIdx.x;
-      h[u] = i < rows ? row_key_hash(p.keys, p.n_keys, begin + i) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < kShufUnroll; ++u) {
-      const int i = base + u * blockDim.x + threadIdx.x;
-      if (i < rows) out[i] = static_cast<uint16_t>(slot_of(h[u], p.slots));
-    }
-  }
-}
-
 // Lanes of the warp whose slot equals this lane's (the lane itself
 // included), from one ballot per slot bit: the live lanes agreeing with this
 // lane on every bit.
-__device__ __forceinline__ unsigned slot_peers(uint32_t s, bool live, int bits) {
+template <int kBits>
+__device__ __forceinline__ unsigned slot_peers(uint32_t s, bool live) {
   unsigned peers = __ballot_sync(0xffffffffu, live);
-  for (int b = 0; b < bits; ++b) {
+#pragma unroll
+  for (int b = 0; b < kBits; ++b) {
     const unsigned ones = __ballot_sync(0xffffffffu, (s >> b) & 1u);
     peers &= ((s >> b) & 1u) ? ones : ~ones;
   }
   return peers;
 }
 
-__global__ void __launch_bounds__(256) shuffle_count_kernel(const __grid_constant__ ShufKeys p, int32_t* counts) {
+enum ShufKeyKind { kKeyI32, kKeyI64, kKeyAny };
+
+// The multiplies of three 64-bit mixes a row hold it (issue 68%, math pipe
+// throttle): 62 us for 20M int64 keys, as before it also wrote the slots. The
+// scatter reads the 2-byte slot instead of hashing the key again.
+template <int kKind>
+__global__ void __launch_bounds__(512)
+    shuffle_count_kernel(const __grid_constant__ ShufKeys p, uint16_t* row_slot, int32_t* counts) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   int32_t* hist = reinterpret_cast<int32_t*>(s_raw);
   const int64_t begin = static_cast<int64_t>(blockIdx.x) * p.tile;
   const int rows = static_cast<int>(begin + p.tile < p.n ? p.tile : p.n - begin);
-  for (uint32_t i = threadIdx.x; i < p.slots; i += blockDim.x) hist[i] = 0;
+  const int step = blockDim.x;
+  for (uint32_t i = threadIdx.x; i < p.slots; i += step) hist[i] = 0;
   __syncthreads();
-  const bool one_int_key = p.n_keys == 1 && p.keys[0].type != CT_UTF8;
-  for (int base = 0; base < rows; base += kShufUnroll * blockDim.x) {
+  row_slot += begin;
+  for (int base = threadIdx.x; base < rows; base += kShufUnroll * step) {
     uint64_t h[kShufUnroll];
-    if (one_int_key) {
-      int64_t v[kShufUnroll];
 #pragma unroll
-      for (int u = 0; u < kShufUnroll; ++u) {
-        const int i = base + u * blockDim.x + threadIdx.x;
-        v[u] = i < rows ? load_int(p.keys[0], begin + i) : 0;
-      }
-#pragma unroll
-      for (int u = 0; u < kShufUnroll; ++u) h[u] = row_key_combine(kRowKeySeed, hash_key(v[u]));
-    } else {
-#pragma unroll
-      for (int u = 0; u < kShufUnroll; ++u) {
-        const int i = base + u * blockDim.x + threadIdx.x;
-        h[u] = i < rows ? row_key_hash(p.keys, p.n_keys, begin + i) : 0;
+    for (int u = 0; u < kShufUnroll; ++u) {
+      const int i = base + u * step;
+      h[u] = 0;
+      if (i < rows) {
+        if (kKind == kKeyI32) h[u] = static_cast<uint64_t>(static_cast<int64_t>(__ldcs(static_cast<const int*>(p.keys[0].data) + begin + i)));
+        else if (kKind == kKeyI64) h[u] = static_cast<uint64_t>(__ldcs(static_cast<const long long*>(p.keys[0].data) + begin + i));
+        else h[u] = row_key_hash(p.keys, p.n_keys, begin + i);
       }
     }
 #pragma unroll
-    for (int u = 0; u < kShufUnroll; ++u)
-      if (base + u * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x) < rows)
-        atomicAdd(&hist[slot_of(h[u], p.slots)], 1);
+    for (int u = 0; u < kShufUnroll; ++u) {
+      const int i = base + u * step;
+      if (kKind != kKeyAny) h[u] = row_key_combine(kRowKeySeed, hash_key(static_cast<int64_t>(h[u])));
+      if (i < rows) {
+        const uint32_t s = slot_of(h[u], p.slots);
+        row_slot[i] = static_cast<uint16_t>(s);
+        atomicAdd(&hist[s], 1);
+      }
+    }
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < p.slots; i += blockDim.x)
+  for (uint32_t i = threadIdx.x; i < p.slots; i += step)
     counts[static_cast<int64_t>(i) * p.ntiles + blockIdx.x] = hist[i];
 }
 
-// Exclusive prefix sum of v[0, n) in shared memory by the whole block.
-__device__ __forceinline__ void block_exclusive_scan(int32_t* v, int n, int32_t* warp_sums) {
-  const int per = (n + blockDim.x - 1) / blockDim.x;
-  const int lo = threadIdx.x * per;
-  const int hi = lo + per < n ? lo + per : n;
-  int32_t sum = 0;
-  for (int k = lo; k < hi; ++k) sum += v[k];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t incl = sum;
+// Inclusive prefix sum of one value per thread over the block; *total is the
+// block's sum. warp_sums: 32 words that no thread uses when it is called.
+template <class T>
+__device__ __forceinline__ T block_inclusive_scan(T v, T* warp_sums, T* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const int32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += t;
+    const T t = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= d) v += t;
   }
-  if (lane == 31) warp_sums[warp] = incl;
+  if (lane == 31) warp_sums[warp] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int32_t run = 0;
-    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
-      const int32_t t = warp_sums[w];
-      warp_sums[w] = run;
-      run += t;
-    }
+  T w = lane < nw ? warp_sums[lane] : T{0};
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const T t = __shfl_up_sync(0xffffffffu, w, d);
+    if (lane >= d) w += t;
   }
+  *total = __shfl_sync(0xffffffffu, w, 31);
+  const T before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
   __syncthreads();
-  int32_t excl = warp_sums[warp] + incl - sum;
-  for (int k = lo; k < hi; ++k) {
-    const int32_t t = v[k];
-    v[k] = excl;
-    excl += t;
-  }
+  return warp > 0 ? v + before : v;
 }
 
-__global__ void __launch_bounds__(256) shuffle_scatter_kernel(const __grid_constant__ ShufKeys p,
-                                                              const __grid_constant__ ShufScatter q) {
-  extern __shared__ __align__(16) unsigned char s_raw[];
+// Block s: counts[s][0, ntiles) becomes its exclusive prefix sum, in place.
+__global__ void __launch_bounds__(1024) shuffle_scan_kernel(int32_t* counts, int64_t ntiles, int32_t* totals) {
   __shared__ int32_t warp_sums[32];
+  int32_t* row = counts + static_cast<int64_t>(blockIdx.x) * ntiles;
+  int32_t run = 0;
+  for (int64_t at = 0; at < ntiles; at += blockDim.x) {
+    const int64_t i = at + threadIdx.x;
+    const int32_t v = i < ntiles ? row[i] : 0;
+    int32_t sum;
+    const int32_t incl = block_inclusive_scan(v, warp_sums, &sum);
+    if (i < ntiles) row[i] = run + incl - v;
+    run += sum;
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = run;
+}
+
+// Dynamic shared memory of the scatter: a column of the tile in slot order,
+// the output row of each of its places, per-slot words, per-warp counts.
+constexpr int64_t shuf_scatter_smem(int64_t tile, int64_t slots) {
+  return tile * 12 + slots * 4 + (tile / kShufRowsPerWarp) * slots * 2;
+}
+
+// Bound by latency: a tile goes through a chain of barriers (rank, scan, and
+// two a column), so what counts is how many tiles an SM has in flight. 8 rows
+// a lane keep it to 40 registers, three blocks of 16 warps an SM. 20M rows of
+// 20 bytes over 256 slots: 197 us (237 us with 16 rows a lane and 32 warps an
+// SM, 228 us with the next column's loads ahead of the writes at 64
+// registers, 246 us with tiles of 2048 rows). Reading the rows in slot order
+// straight from memory, a lookup per lane in the L1, and ranking them twice
+// took 305 us.
+template <int kBits>
+__global__ void __launch_bounds__(512, 3) shuffle_scatter_kernel(const __grid_constant__ ShufKeys p,
+                                                                 const __grid_constant__ ShufScatter q) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  __shared__ int64_t warp_sums[32];
   const int tile = p.tile;
   const int nw = blockDim.x >> 5;
-  const uint32_t slots = p.slots;
-  int32_t* sdest = reinterpret_cast<int32_t*>(s_raw);  // [tile] output row of the tile's i-th row in slot order
-  int32_t* tbase = sdest + tile;                         // [slots] first position of a slot in the tile's order
-  int32_t* tstart = tbase + slots;                       // [slots] the slot's first output row for this tile
-  uint16_t* srow = reinterpret_cast<uint16_t*>(tstart + slots);  // [tile] tile row at each position
-  uint16_t* sslot = srow + tile;                                  // [tile] slot of each tile row
-  uint16_t* wcnt = sslot + tile;                                  // [warps][slots]
+  const int slots = static_cast<int>(p.slots);
+  uint64_t* stage8 = reinterpret_cast<uint64_t*>(s_raw);  // [tile]
+  uint32_t* stage4 = reinterpret_cast<uint32_t*>(s_raw);
+  int32_t* sdest = reinterpret_cast<int32_t*>(stage8 + tile);     // [tile] output row of each place
+  int32_t* delta = sdest + tile;                                  // [slots] output row less place
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(delta + slots);    // [warps][slots]
   const int64_t begin = static_cast<int64_t>(blockIdx.x) * tile;
   const int rows = static_cast<int>(begin + tile < p.n ? tile : p.n - begin);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r0 = warp * kShufRowsPerWarp + lane;  // this lane's rows: r0 + 32 j
 
-  for (uint32_t i = threadIdx.x; i < nw * slots; i += blockDim.x) wcnt[i] = 0;
-  for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x)
-    tstart[i] = q.starts[static_cast<int64_t>(i) * p.ntiles + blockIdx.x];
-  tile_slots(p, begin, rows, sslot);
-  __syncthreads();
-
-  // Per-warp counts over the warp's rows [warp * R, (warp + 1) * R).
-  const int r0 = warp * kShufRowsPerWarp;
-  uint16_t* mine = wcnt + static_cast<int64_t>(warp) * slots;
-  for (int j = r0; j < r0 + kShufRowsPerWarp; j += 32) {
-    const int i = j + lane;
-    const bool live = i < rows;
-    const uint32_t s = live ? sslot[i] : 0u;
-    const unsigned peers = slot_peers(s, live, p.slot_bits);
-    if (live && lane == __ffs(peers) - 1) mine[s] = static_cast<uint16_t>(mine[s] + __popc(peers));
-    __syncwarp();
-  }
-  __syncthreads();
-  // Exclusive across warps per slot (in place), the tile's count per slot.
-  for (uint32_t s = threadIdx.x; s < slots; s += blockDim.x) {
-    int32_t run = 0;
-    for (int w = 0; w < nw; ++w) {
-      const int32_t c = wcnt[static_cast<int64_t>(w) * slots + s];
-      wcnt[static_cast<int64_t>(w) * slots + s] = static_cast<uint16_t>(run);
-      run += c;
-    }
-    tbase[s] = run;
-  }
-  __syncthreads();
-  block_exclusive_scan(tbase, static_cast<int>(slots), warp_sums);
+  uint32_t at[kShufPerLane];  // slot | rank among the warp's rows of the slot << 16, later the row's place
+#pragma unroll
+  for (int j = 0; j < kShufPerLane; ++j)
+    at[j] = r0 + 32 * j < rows ? __ldcs(q.row_slot + begin + r0 + 32 * j) : 0u;
+  for (int i = threadIdx.x; i < nw * slots; i += blockDim.x) wcnt[i] = 0;
   __syncthreads();
 
-  // Each row's position in the tile's slot order, and its output row.
+  uint16_t* mine = wcnt + warp * slots;
   const unsigned below = (1u << lane) - 1u;
-  for (int j = r0; j < r0 + kShufRowsPerWarp; j += 32) {
-    const int i = j + lane;
-    const bool live = i < rows;
-    const uint32_t s = live ? sslot[i] : 0u;
-    const unsigned peers = slot_peers(s, live, p.slot_bits);
-    if (live) {
-      const int32_t within = mine[s] + __popc(peers & below);
-      const int32_t lp = tbase[s] + within;
-      srow[lp] = static_cast<uint16_t>(i);
-      sdest[lp] = tstart[s] + within;
-    }
+#pragma unroll
+  for (int j = 0; j < kShufPerLane; ++j) {
+    const bool live = r0 + 32 * j < rows;
+    const uint32_t s = at[j];
+    const unsigned peers = slot_peers<kBits>(s, live);
+    const uint32_t had = mine[s];
     __syncwarp();
-    if (live && lane == __ffs(peers) - 1) mine[s] = static_cast<uint16_t>(mine[s] + __popc(peers));
+    if (live && (peers & below) == 0) mine[s] = static_cast<uint16_t>(had + __popc(peers));
     __syncwarp();
+    at[j] = s | (had + __popc(peers & below)) << 16;
   }
   __syncthreads();
 
-  // The columns, in the tile's slot order.
+  // Slots in order, a block's width at a time: where the slot begins in the
+  // tile's order and in the output, and where each warp's rows of it begin.
+  // One scan carries both sums: a tile's rows in the low 14 bits.
+  int64_t run = 0;
+  for (int s0 = 0; s0 < slots; s0 += blockDim.x) {
+    const int s = s0 + threadIdx.x;
+    int32_t mid = 0;
+    int64_t both = 0;
+    if (s < slots) {
+      for (int w = 0; w < nw; ++w) mid += wcnt[w * slots + s];
+      both = static_cast<int64_t>(q.totals[s]) << 14 | mid;
+    }
+    int64_t sum;
+    const int64_t excl = run + block_inclusive_scan(both, warp_sums, &sum) - both;
+    run += sum;
+    if (s < slots) {
+      int32_t place = static_cast<int32_t>(excl & 0x3FFF);
+      delta[s] = static_cast<int32_t>(excl >> 14) + q.starts[static_cast<int64_t>(s) * p.ntiles + blockIdx.x] - place;
+      for (int w = 0; w < nw; ++w) {
+        const int32_t c = wcnt[w * slots + s];
+        wcnt[w * slots + s] = static_cast<uint16_t>(place);
+        place += c;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kShufPerLane; ++j) {
+    const uint32_t s = at[j] & 0xFFFFu;
+    at[j] = mine[s] + (at[j] >> 16);
+    if (r0 + 32 * j < rows) sdest[at[j]] = static_cast<int32_t>(at[j]) + delta[s];
+  }
+
   for (int c = 0; c < q.n_fixed; ++c) {
     if (q.width[c] == 8) {
       const long long* src = static_cast<const long long*>(q.src[c]) + begin;
-      int64_t* dst = static_cast<int64_t*>(q.dst[c]);
-      for (int i = threadIdx.x; i < rows; i += blockDim.x) dst[sdest[i]] = __ldg(src + srow[i]);
+      long long* dst = static_cast<long long*>(q.dst[c]);
+      long long v[kShufPerLane];
+#pragma unroll
+      for (int j = 0; j < kShufPerLane; ++j) v[j] = r0 + 32 * j < rows ? __ldcs(src + r0 + 32 * j) : 0;
+      __syncthreads();  // the column before it has left the stage
+#pragma unroll
+      for (int j = 0; j < kShufPerLane; ++j)
+        if (r0 + 32 * j < rows) stage8[at[j]] = static_cast<uint64_t>(v[j]);
+      __syncthreads();
+#pragma unroll 4
+      for (int i = threadIdx.x; i < rows; i += blockDim.x) dst[sdest[i]] = static_cast<long long>(stage8[i]);
     } else {
       const int* src = static_cast<const int*>(q.src[c]) + begin;
-      int32_t* dst = static_cast<int32_t*>(q.dst[c]);
-      for (int i = threadIdx.x; i < rows; i += blockDim.x) dst[sdest[i]] = __ldg(src + srow[i]);
+      int* dst = static_cast<int*>(q.dst[c]);
+      int v[kShufPerLane];
+#pragma unroll
+      for (int j = 0; j < kShufPerLane; ++j) v[j] = r0 + 32 * j < rows ? __ldcs(src + r0 + 32 * j) : 0;
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < kShufPerLane; ++j)
+        if (r0 + 32 * j < rows) stage4[at[j]] = static_cast<uint32_t>(v[j]);
+      __syncthreads();
+#pragma unroll 4
+      for (int i = threadIdx.x; i < rows; i += blockDim.x) dst[sdest[i]] = static_cast<int>(stage4[i]);
     }
   }
-  if (q.inverse != nullptr)
-    for (int i = threadIdx.x; i < rows; i += blockDim.x)
-      q.inverse[sdest[i]] = static_cast<int32_t>(begin + srow[i]);
+  if (q.inverse != nullptr) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kShufPerLane; ++j)
+      if (r0 + 32 * j < rows) stage4[at[j]] = static_cast<uint32_t>(begin + r0 + 32 * j);
+    __syncthreads();
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) q.inverse[sdest[i]] = static_cast<int32_t>(stage4[i]);
+  }
 }
 
 }  // namespace
@@ -300,30 +325,35 @@ ShuffleResult shuffle_rows(const TupleSetPtr& in_ts, const std::vector<std::stri
     return r;
   }
 
-  // Tiles of 8 warps x 512 rows; the [slots][tiles] count matrix then holds
-  // at most a quarter as many cells as rows (slots <= 1024).
-  constexpr int kWarps = 8;
-  p.tile = kWarps * kShufRowsPerWarp;
+  // 16 warps a tile: runs of one slot are twice as long as with 8. Inputs that
+  // would leave an SM with less than two such tiles take 8.
+  const int warps = n >= static_cast<int64_t>(num_sms()) * 2 * 16 * kShufRowsPerWarp ? 16 : 8;
+  p.tile = warps * kShufRowsPerWarp;
   p.ntiles = (n + p.tile - 1) / p.tile;
   const int blocks = static_cast<int>(p.ntiles);
-  p.slot_bits = num_slots > 1 ? 64 - __builtin_clzll(static_cast<unsigned long long>(num_slots - 1)) : 0;
-  const int64_t smem_count = num_slots * 4;
-  const int64_t smem_scatter = static_cast<int64_t>(p.tile) * 4 + num_slots * 8 + static_cast<int64_t>(p.tile) * 4 +
-                               kWarps * num_slots * 2;
-  if (smem_scatter > 48 * 1024)
-    GF_CUDA(cudaFuncSetAttribute(shuffle_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem_scatter)));
+  const int64_t smem_scatter = shuf_scatter_smem(p.tile, num_slots);
+  const auto scatter = num_slots <= 32    ? shuffle_scatter_kernel<5>
+                       : num_slots <= 256 ? shuffle_scatter_kernel<8>
+                                          : shuffle_scatter_kernel<10>;
+  GF_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_scatter)));
 
   const int64_t cells = num_slots * p.ntiles;
-  auto counts = make_buffer(cells * 4, s);
-  auto starts = make_buffer((cells + 1) * 4, s);
+  auto row_slot = make_buffer(n * 2, s);
+  auto starts = make_buffer((cells + num_slots) * 4, s);
+  int32_t* totals = starts->as<int32_t>() + cells;
   {
     ProfScope prof("shuffle_count_kernel", s);
-    shuffle_count_kernel<<<blocks, kWarps * 32, smem_count, s>>>(p, counts->as<int32_t>());
+    const auto count = p.n_keys == 1 && p.keys[0].type == CT_I64    ? shuffle_count_kernel<kKeyI64>
+                       : p.n_keys == 1 && p.keys[0].type != CT_UTF8 ? shuffle_count_kernel<kKeyI32>
+                                                                    : shuffle_count_kernel<kKeyAny>;
+    count<<<blocks, warps * 32, num_slots * 4, s>>>(p, row_slot->as<uint16_t>(), starts->as<int32_t>());
     after_launch("shuffle_count_kernel");
-    prof.stop(static_cast<double>(n) * 4.0 * p.n_keys + static_cast<double>(cells) * 4.0);
+    prof.stop(static_cast<double>(n) * (4.0 * p.n_keys + 2.0) + static_cast<double>(cells) * 4.0);
   }
-  exclusive_scan_i32(counts->as<int32_t>(), starts->as<int32_t>(), cells, s);
+  const int64_t scan_threads = std::min<int64_t>(1024, (p.ntiles + 31) / 32 * 32);
+  shuffle_scan_kernel<<<static_cast<int>(num_slots), static_cast<int>(scan_threads), 0, s>>>(starts->as<int32_t>(),
+                                                                                             p.ntiles, totals);
+  after_launch("shuffle_scan_kernel");
 
   // Output columns: fixed-width ones scattered by the kernel (in groups of
   // kShufMaxFixed, the ranking repeated per group), utf8 ones gathered
@@ -337,7 +367,9 @@ ShuffleResult shuffle_rows(const TupleSetPtr& in_ts, const std::vector<std::stri
   do {
     ShufScatter q;
     std::memset(&q, 0, sizeof(q));
+    q.row_slot = row_slot->as<uint16_t>();
     q.starts = starts->as<int32_t>();
+    q.totals = totals;
     const size_t take = std::min<size_t>(kShufMaxFixed, fixed.size() - at);
     for (size_t j = 0; j < take; ++j) {
       const auto& c = in->column(fixed[at + j]);
@@ -351,9 +383,9 @@ ShuffleResult shuffle_rows(const TupleSetPtr& in_ts, const std::vector<std::stri
     q.n_fixed = static_cast<int32_t>(take);
     if (at == 0 && inverse) q.inverse = inverse->as<int32_t>();
     ProfScope prof("shuffle_scatter_kernel", s);
-    shuffle_scatter_kernel<<<blocks, kWarps * 32, smem_scatter, s>>>(p, q);
+    scatter<<<blocks, warps * 32, smem_scatter, s>>>(p, q);
     after_launch("shuffle_scatter_kernel");
-    double bytes = static_cast<double>(n) * 4.0 * p.n_keys + (q.inverse ? n * 4.0 : 0.0);
+    double bytes = static_cast<double>(n) * 2.0 + (q.inverse ? n * 4.0 : 0.0);
     for (size_t j = 0; j < take; ++j) bytes += 2.0 * n * q.width[j];
     prof.stop(bytes);
     at += take;
@@ -365,12 +397,10 @@ ShuffleResult shuffle_rows(const TupleSetPtr& in_ts, const std::vector<std::stri
     for (size_t j = 0; j < utf8.size(); ++j) out[utf8[j]] = g[j];
   }
 
-  // Slot boundaries: the scanned count of each slot's first sub-range.
-  std::vector<int32_t> first(num_slots);
-  GF_CUDA(cudaMemcpy2DAsync(first.data(), 4, starts->as<int32_t>(), static_cast<size_t>(p.ntiles) * 4, 4,
-                            static_cast<size_t>(num_slots), cudaMemcpyDeviceToHost, s));
+  std::vector<int32_t> rows(num_slots);
+  GF_CUDA(cudaMemcpyAsync(rows.data(), totals, static_cast<size_t>(num_slots) * 4, cudaMemcpyDeviceToHost, s));
   sync(s);
-  for (int64_t i = 0; i < num_slots; ++i) r.offsets[i] = first[i];
+  for (int64_t i = 0; i < num_slots; ++i) r.offsets[i + 1] = r.offsets[i] + rows[i];
   r.rows = TupleSet::make(in->fields(), std::move(out), n);
   return r;
 }
