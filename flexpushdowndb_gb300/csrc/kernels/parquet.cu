@@ -210,7 +210,8 @@ constexpr int kPqRuns = 256;  // run headers read per round
 // per page left most SMs without a warp (a 4M-row, 7-column file of
 // 131,072-row pages is 237 pages; the pass took 460 us at 12% occupancy) and
 // the longest page set its length; with parts, word-wide index reads and one
-// copy per span of chunks the whole read of that file went from 1,118 to 680 us.
+// copy per span of chunks the whole read of that file went from 1,118 to 680 us
+// (653 with copying and decoding overlapped, see kPqBatch).
 constexpr int kPqPart = 8192;
 
 struct PagePart {
@@ -469,9 +470,10 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
   }
 }
 
-// blockIdx.y: a data page (index into `list`); values over x.
-__global__ void __launch_bounds__(256) parquet_values_kernel(const PageDev* pages, const int32_t* list, DictArrays dicts,
-                                                             DevStatus* st) {
+// blockIdx.y: a data page (index into `list`, whose first is the read's
+// first-th); values over x.
+__global__ void __launch_bounds__(256) parquet_values_kernel(const PageDev* pages, const int32_t* list, int32_t first,
+                                                             DictArrays dicts, DevStatus* st) {
   const PageDev& pg = pages[list[blockIdx.y]];
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const bool dict = pg.encoding != parquet::ENC_PLAIN;
@@ -483,7 +485,7 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const PageDev* page
       // plain values only: a fixed-width dictionary page is decoded to its
       // values by the page pass and never listed here
       if (dict || (i + 1) * pg.width > pg.values_len) {
-        raise_status(st, GFPDB_EINVAL, 600000 + static_cast<int32_t>(blockIdx.y));
+        raise_status(st, GFPDB_EINVAL, 600000 + first + static_cast<int32_t>(blockIdx.y));
         continue;
       }
       // the value's 4-byte words from the two aligned words around each
@@ -496,7 +498,7 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const PageDev* page
     } else if (dict) {
       const int32_t e = pg.idx[row];
       if (e < 0 || e >= dp->num_values) {
-        raise_status(st, GFPDB_EINVAL, 600000 + static_cast<int32_t>(blockIdx.y));
+        raise_status(st, GFPDB_EINVAL, 600000 + first + static_cast<int32_t>(blockIdx.y));
         pg.row_ptr[row] = 0;
         pg.row_len[row] = 0;
         continue;
@@ -519,6 +521,36 @@ __global__ void parquet_bytes_kernel(const uint64_t* __restrict__ ptr, const int
 
 constexpr int64_t kPqCopyGap = 64 * 1024;
 
+// A read's chunks are copied and decoded in batches of about kPqBatch bytes:
+// while one batch is decoded on the caller's stream the next ones are copied
+// on a stream of the read's own. Reads of a single batch use the caller's
+// stream alone. (72.6 MB, 4M rows: 558 us of copying and then decoding as one
+// batch, 496 us in batches.)
+constexpr int64_t kPqBatch = 8 << 20;
+
+// The copies' stream; nothing it started is left running when it goes.
+struct CopyStream {
+  cudaStream_t s = nullptr;
+  cudaEvent_t ev = nullptr;
+  ~CopyStream() {
+    if (s != nullptr) {
+      (void)cudaStreamSynchronize(s);
+      (void)cudaStreamDestroy(s);
+    }
+    if (ev != nullptr) (void)cudaEventDestroy(ev);
+  }
+  void open(cudaStream_t after) {
+    GF_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    GF_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    order(after, s);
+  }
+  // `to` goes on after what `from` holds now.
+  void order(cudaStream_t from, cudaStream_t to) {
+    GF_CUDA(cudaEventRecord(ev, from));
+    GF_CUDA(cudaStreamWaitEvent(to, ev, 0));
+  }
+};
+
 int grid_parquet(int64_t n) {
   int64_t b = (n + 255) / 256;
   const int64_t cap = static_cast<int64_t>(num_sms()) * 8;
@@ -535,26 +567,48 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   if (rows > INT32_MAX) fail(GFPDB_EUNSUPPORTED, "a Parquet read of more than 2^31 - 1 rows");
   const int nc = static_cast<int>(L.columns.size());
 
-  // the column chunks' bytes on the device: chunks that follow each other in
-  // the file with at most kPqCopyGap bytes between them share one copy (a
-  // copy costs about 3 us besides its bytes)
+  // the column chunks' bytes on the device, in batches; within one, chunks
+  // that follow each other in the file with at most kPqCopyGap bytes between
+  // them share one copy (a copy costs about 3 us besides its bytes)
   struct Span {
     int64_t begin, end, at;  // file bytes [begin, end) at byte `at` of the arena
   };
+  struct Batch {
+    size_t chunk_end, span_end;              // its last chunk and span, plus one
+    size_t item_end = 0, snappy_end = 0, data_end = 0;  // the same in the lists below
+    int64_t bytes = 0;
+  };
   std::vector<Span> spans;
+  std::vector<Batch> batches;
   std::vector<int64_t> chunk_at(L.chunks.size());
   int64_t arena_bytes = 0;
   for (size_t c = 0; c < L.chunks.size(); ++c) {
     const auto& ch = L.chunks[c];
-    if (!spans.empty() && ch.begin >= spans.back().end && ch.begin - spans.back().end <= kPqCopyGap)
+    const bool fresh = batches.empty() || batches.back().bytes >= kPqBatch;
+    if (fresh) batches.push_back(Batch{c, spans.size()});
+    Batch& b = batches.back();
+    if (!fresh && ch.begin >= spans.back().end && ch.begin - spans.back().end <= kPqCopyGap)
       spans.back().end = ch.end;
     else
       spans.push_back(Span{ch.begin, ch.end, arena_bytes});
     chunk_at[c] = spans.back().at + (ch.begin - spans.back().begin);
     arena_bytes = (chunk_at[c] + (ch.end - ch.begin) + 15) / 16 * 16;
+    b.bytes += ch.end - ch.begin;
+    b.chunk_end = c + 1;
+    b.span_end = spans.size();
   }
   auto arena = make_buffer(arena_bytes + 16, s);  // tail padding: 4-byte word reads past a value's end
-  for (const Span& sp : spans) copy_h2d(arena->as<uint8_t>() + sp.at, file + sp.begin, sp.end - sp.begin, s);
+  CopyStream copies;
+  if (batches.size() > 1) copies.open(s);
+  size_t copied = 0;  // spans
+  auto copy_to = [&](size_t end) {
+    for (; copied < end; ++copied)
+      copy_h2d(arena->as<uint8_t>() + spans[copied].at, file + spans[copied].begin,
+               spans[copied].end - spans[copied].begin, copies.s != nullptr ? copies.s : s);
+  };
+  // the first copies run while the host lays the pages out; the others come
+  // after the page descriptors, which would wait behind them
+  if (!batches.empty()) copy_to(batches[std::min<size_t>(1, batches.size() - 1)].span_end);
 
   // per-column outputs and working arrays
   std::vector<BufferPtr> fixed(nc), row_ptr(nc), row_len(nc), idx(nc);
@@ -577,8 +631,16 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   std::vector<int32_t> snappy_list, data_list, item_list;  // item_list: (page, first value) pairs
   int64_t inflate_bytes = 0, dict_entries = 0;
   std::vector<int64_t> inflate_at(L.pages.size(), -1);
+  size_t batch = 0;  // pages come in the order of their chunks
+  auto end_batch = [&] {
+    batches[batch].item_end = item_list.size() / 2;
+    batches[batch].snappy_end = snappy_list.size();
+    batches[batch].data_end = data_list.size();
+    ++batch;
+  };
   for (size_t p = 0; p < L.pages.size(); ++p) {
     const auto& pg = L.pages[p];
+    while (static_cast<size_t>(pg.chunk) >= batches[batch].chunk_end) end_batch();
     const bool v2 = pg.type == parquet::PAGE_DATA_V2;
     const bool snappy = pg.codec == parquet::CODEC_SNAPPY && !(v2 && !pg.v2_compressed);
     if (snappy) {
@@ -600,6 +662,7 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
       item_list.push_back(static_cast<int32_t>(first));
     }
   }
+  while (batch < batches.size()) end_batch();
   auto inflated = make_buffer(inflate_bytes + 16, s);
   for (size_t p = 0; p < L.pages.size(); ++p) {
     const auto& pg = L.pages[p];
@@ -641,7 +704,6 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   DevStatus* st = status->as<DevStatus>();
   const int64_t np = static_cast<int64_t>(pd.size());
   auto pages_dev = make_buffer((np > 0 ? np : 1) * static_cast<int64_t>(sizeof(PageDev)), s);
-  const int64_t n_items = static_cast<int64_t>(item_list.size() / 2);
   std::vector<int32_t> all_lists(item_list);
   all_lists.insert(all_lists.end(), snappy_list.begin(), snappy_list.end());
   all_lists.insert(all_lists.end(), data_list.begin(), data_list.end());
@@ -653,33 +715,41 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   const int32_t* snappy_dev = lists->as<int32_t>() + item_list.size();
   const int32_t* data_dev = snappy_dev + snappy_list.size();
 
-  if (!snappy_list.empty()) {
-    ProfScope prof("parquet_snappy_kernel", s);
-    parquet_snappy_kernel<<<grid_parquet(static_cast<int64_t>(snappy_list.size()) * 32), 256, 0, s>>>(
-        pages, snappy_dev, static_cast<int32_t>(snappy_list.size()), st);
-    after_launch("parquet_snappy_kernel");
-    prof.stop(static_cast<double>(inflate_bytes));
-  }
-  if (np > 0) {
-    ProfScope prof("parquet_pages_kernel", s);
-    const int64_t most = static_cast<int64_t>(num_sms()) * 8;
-    parquet_pages_kernel<<<static_cast<int>(std::min(n_items, most)), kPqThreads, 0, s>>>(
-        pages, static_cast<int32_t>(np), lists->as<PagePart>(), n_items, dicts, st);
-    after_launch("parquet_pages_kernel");
-    prof.stop(0.0);
-  }
-  if (!data_list.empty()) {
+  const PagePart* items = lists->as<PagePart>();
+  Batch from{};
+  for (const Batch& b : batches) {
+    copy_to(b.span_end);
+    if (copies.s != nullptr) copies.order(copies.s, s);
+    if (b.snappy_end > from.snappy_end) {
+      const int64_t n = static_cast<int64_t>(b.snappy_end - from.snappy_end);
+      ProfScope prof("parquet_snappy_kernel", s);
+      parquet_snappy_kernel<<<grid_parquet(n * 32), 256, 0, s>>>(pages, snappy_dev + from.snappy_end,
+                                                                 static_cast<int32_t>(n), st);
+      after_launch("parquet_snappy_kernel");
+      double bytes = 0;
+      for (size_t k = from.snappy_end; k < b.snappy_end; ++k) bytes += pd[snappy_list[k]].inflated_len;
+      prof.stop(bytes);
+    }
+    if (b.item_end > from.item_end) {
+      ProfScope prof("parquet_pages_kernel", s);
+      const int64_t n = static_cast<int64_t>(b.item_end - from.item_end), most = static_cast<int64_t>(num_sms()) * 8;
+      parquet_pages_kernel<<<static_cast<int>(std::min(n, most)), kPqThreads, 0, s>>>(
+          pages, static_cast<int32_t>(np), items + from.item_end, n, dicts, st);
+      after_launch("parquet_pages_kernel");
+      prof.stop(0.0);
+    }
     // each data page's values over up to 64 blocks of 256 threads
     int64_t most = 0;
-    for (int32_t p : data_list) most = std::max<int64_t>(most, L.pages[p].num_values);
+    for (size_t k = from.data_end; k < b.data_end; ++k) most = std::max<int64_t>(most, L.pages[data_list[k]].num_values);
     const int gx = static_cast<int>(std::min<int64_t>(64, std::max<int64_t>(1, (most + 255) / 256)));
-    for (size_t at = 0; at < data_list.size(); at += 65535) {  // grid y limit
-      const int gy = static_cast<int>(std::min<size_t>(65535, data_list.size() - at));
+    for (size_t at = from.data_end; at < b.data_end; at += 65535) {  // grid y limit
+      const int gy = static_cast<int>(std::min<size_t>(65535, b.data_end - at));
       ProfScope prof("parquet_values_kernel", s);
-      parquet_values_kernel<<<dim3(gx, gy), 256, 0, s>>>(pages, data_dev + at, dicts, st);
+      parquet_values_kernel<<<dim3(gx, gy), 256, 0, s>>>(pages, data_dev + at, static_cast<int32_t>(at), dicts, st);
       after_launch("parquet_values_kernel");
       prof.stop(0.0);
     }
+    from = b;
   }
   DevStatus h;
   GF_CUDA(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
