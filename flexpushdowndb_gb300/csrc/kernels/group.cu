@@ -399,7 +399,9 @@ __global__ void __launch_bounds__(NT) group_update_kernel(const __grid_constant_
 // in flight, and rows that miss the shared table queue up until they fill
 // two rounds of a warp. 1024 threads with two rows each: 512 with four took
 // 1.6 times as long, 768 with two or three 1.25 times. 20M rows, SUM, COUNT and
-// MAX: 0.9M groups (Zipf) 375 us against 621, 1000 groups 227 against 347.
+// MAX: 0.9M groups (Zipf) 384 us against 621, 1000 groups 193 against 347. A
+// row reads its set's four one-byte tags and then one key: with the four keys
+// read instead the random 16-byte reads' bank conflicts made it 403 and 228.
 struct PlainAcc {
   const void* col;   // null: a count
   int32_t wide;      // int64 column
@@ -423,7 +425,7 @@ struct PlainParams {
 };
 
 constexpr int64_t plain_smem(int64_t slots, int n_acc) {
-  return slots * (8 + 8 * n_acc) + kGroupSeenBits / 8 + kPlainThreads / 32 * kPlainQueue * 12;
+  return slots * (8 + 8 * n_acc + 1) + kGroupSeenBits / 8 + kPlainThreads / 32 * kPlainQueue * 12;
 }
 
 __device__ __forceinline__ void red_add(unsigned long long* at, unsigned long long v) {
@@ -558,6 +560,7 @@ __global__ void __launch_bounds__(kPlainThreads) group_update_plain_kernel(const
   uint64_t* q_key = reinterpret_cast<uint64_t*>(s_acc) + static_cast<int64_t>(S) * A;
   uint32_t* q_row = reinterpret_cast<uint32_t*>(q_key + kPlainThreads / 32 * kPlainQueue);
   unsigned* s_seen = q_row + kPlainThreads / 32 * kPlainQueue;
+  uint32_t* s_tags = s_seen + kGroupSeenBits / 32;  // a byte per slot, 0 while it is empty
   q_key += warp * kPlainQueue;
   q_row += warp * kPlainQueue;
   unsigned head = 0, tail = 0;  // the same in every lane
@@ -568,6 +571,7 @@ __global__ void __launch_bounds__(kPlainThreads) group_update_plain_kernel(const
     for (int a = 0; a < A; ++a) s_acc[a * S + i] = a < pp.n_add ? 0ull : static_cast<unsigned long long>(INT64_MIN);
   }
   for (int i = threadIdx.x; i < kGroupSeenBits / 32; i += kPlainThreads) s_seen[i] = 0;
+  for (int i = threadIdx.x; i < S / kPlainWays; i += kPlainThreads) s_tags[i] = 0;
   __syncthreads();
 
   // Rows past the end stand for the last row and are not live: every load is
@@ -648,20 +652,29 @@ __global__ void __launch_bounds__(kPlainThreads) group_update_plain_kernel(const
     for (int u = 0; u < U; ++u) {
       h[u] = hash_key(static_cast<int64_t>(key[u]));
       const bool is_row = base + lane + 32 * u < pp.n;
-      const int at = kPlainWays * static_cast<int>(__umulhi(static_cast<unsigned>(h[u] >> 32),
-                                                            static_cast<unsigned>(S / kPlainWays)));
-      const ulonglong2 ka = *reinterpret_cast<const ulonglong2*>(s_keys + at);
-      const ulonglong2 kb = *reinterpret_cast<const ulonglong2*>(s_keys + at + 2);
+      const int set = static_cast<int>(__umulhi(static_cast<unsigned>(h[u] >> 32), static_cast<unsigned>(S / kPlainWays)));
+      const int at = kPlainWays * set;
+      const uint32_t tag = (static_cast<uint32_t>(h[u]) >> 24) | 1u;  // not a bit of the seen bits' index
+      const uint32_t tags = *reinterpret_cast<const volatile uint32_t*>(s_tags + set);
+      const uint32_t same = __vcmpeq4(tags, tag * 0x01010101u);
       const bool can = is_row && key[u] != kEmptySlot;
-      int way = ka.x == key[u] ? 0 : ka.y == key[u] ? 1 : kb.x == key[u] ? 2 : kb.y == key[u] ? 3 : -1;
-      if (!can) way = -1;
-      if (can && way < 0 && kb.y == kEmptySlot) {  // slots fill in order: the last one is empty while any is
+      int way = -1;
+      if (can && same != 0) {
+        way = (__ffs(static_cast<int>(same)) - 1) >> 3;
+        if (*reinterpret_cast<const volatile uint64_t*>(s_keys + at + way) != key[u]) {  // another key's tag
+          way = -1;
+          for (int j = 0; j < kPlainWays; ++j)
+            if (*reinterpret_cast<const volatile uint64_t*>(s_keys + at + j) == key[u]) way = j;
+        }
+      }
+      if (can && way < 0 && (tags >> 24) == 0) {  // slots fill in order: the last one is empty while any is
         const unsigned bit = static_cast<unsigned>(h[u]) & (kGroupSeenBits - 1);
         if (atomicOr(s_seen + (bit >> 5), 1u << (bit & 31)) >> (bit & 31) & 1u)  // not its first sight
           for (int j = 0; j < kPlainWays && way < 0; ++j) {
             const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long*>(s_keys + at + j),
                                                      static_cast<unsigned long long>(kEmptySlot),
                                                      static_cast<unsigned long long>(key[u]));
+            if (old == kEmptySlot) reinterpret_cast<uint8_t*>(s_tags)[at + j] = static_cast<uint8_t>(tag);
             if (old == kEmptySlot || old == key[u]) way = j;
           }
       }
@@ -1594,7 +1607,7 @@ class GroupTable {
                                                     group_update_plain_kernel<3, false>, group_update_plain_kernel<4, false>};
       const bool beside = p.n_acc == 3 && p.key_stride == 4;
       const PlainKernel fn = beside ? group_update_plain_kernel<3, true> : table[p.n_acc - 1];
-      p.sm_slots = static_cast<int32_t>((max_smem_optin() - 1024 - plain_smem(0, 0)) / per_slot) / kPlainWays * kPlainWays;
+      p.sm_slots = static_cast<int32_t>((max_smem_optin() - 1024 - plain_smem(0, 0)) / (per_slot + 1)) / kPlainWays * kPlainWays;
       const int64_t dyn = plain_smem(p.sm_slots, p.n_acc);
       GF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn)));
       fn<<<num_sms(), kPlainThreads, dyn, s>>>(p, plain);
