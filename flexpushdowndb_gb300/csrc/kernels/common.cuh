@@ -161,47 +161,70 @@ constexpr uint64_t kFlagAgg = 1ull << 62;
 constexpr uint64_t kFlagIncl = 2ull << 62;
 constexpr uint64_t kValueMask = (1ull << 62) - 1;
 
+// A status word carries its own value, so its loads and stores order nothing
+// else.
+__device__ __forceinline__ uint64_t ld_status(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void st_status(uint64_t* p, uint64_t v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 // Called by all 32 lanes of one warp. Publishes `tile_total` for `tile` and
 // returns the exclusive prefix (sum of all earlier tiles). Tiles must be
 // handed out in increasing order (atomic ticket) so that every earlier tile
 // belongs to a CTA that is already running; each wait is still bounded.
+// When all tiles run at once the last ones walk back over all others, a round
+// trip to the L2 a window: windows of 128 tiles (four words a lane) instead of
+// 32, and no wait for words behind the nearest inclusive one.
 __device__ __forceinline__ uint64_t lookback_exclusive(uint64_t* status, int64_t tile, uint64_t tile_total,
                                                        DevStatus* st) {
+  constexpr int kWords = 4;
   const int lane = threadIdx.x & 31;
   if (tile == 0) {
-    if (lane == 0) st_release(&status[0], kFlagIncl | tile_total);
+    if (lane == 0) st_status(&status[0], kFlagIncl | tile_total);
     return 0;
   }
-  if (lane == 0) st_release(&status[tile], kFlagAgg | tile_total);
-  uint64_t excl = 0;
-  int64_t window = tile - 1;
-  for (;;) {
-    const int64_t j = window - lane;
-    uint64_t v;
-    uint32_t spins = 0;
-    for (;;) {
-      v = j >= 0 ? ld_acquire(&status[j]) : kFlagIncl;
-      const bool missing = (v & ~kValueMask) == 0;
-      if (!__any_sync(0xffffffffu, missing)) break;
-      if (++spins > kSpinLimit) {
+  if (lane == 0) st_status(&status[tile], kFlagAgg | tile_total);
+  uint64_t excl = 0;  // this lane's part of it
+  bool done = false;
+  for (int64_t window = tile - 1; !done; window -= 32 * kWords) {
+    uint64_t v[kWords];
+    for (uint32_t spins = 0;; ++spins) {
+#pragma unroll
+      for (int w = 0; w < kWords; ++w) {
+        const int64_t j = window - 32 * w - lane;
+        v[w] = j >= 0 ? ld_status(&status[j]) : kFlagIncl;
+      }
+      // words from the nearest on, up to an inclusive one
+      bool wait = false;
+      done = false;
+#pragma unroll
+      for (int w = 0; w < kWords; ++w) {
+        const uint32_t incl = __ballot_sync(0xffffffffu, (v[w] & ~kValueMask) == kFlagIncl);
+        const uint32_t missing = __ballot_sync(0xffffffffu, (v[w] & ~kValueMask) == 0);
+        const uint32_t upto = incl != 0 ? incl ^ (incl - 1) : 0xffffffffu;  // the first inclusive one and those before it
+        if (done || ((upto >> lane) & 1u) == 0) v[w] = 0;
+        if (!done && (missing & upto) != 0) wait = true;
+        done = done || incl != 0;
+      }
+      if (!wait) break;
+      if (spins > kSpinLimit) {
         if (lane == 0) raise_status(st, GFPDB_ETIMEDOUT, 1);
-        v = kFlagIncl;  // give up: the call reports the timeout
+        done = true;  // give up: the call reports the timeout
         break;
       }
-      __nanosleep(64);
+      __nanosleep(32);
     }
-    const uint32_t incl = __ballot_sync(0xffffffffu, (v & ~kValueMask) == kFlagIncl);
-    uint64_t mine = v & kValueMask;
-    if (incl != 0) {
-      const int first = __ffs(incl) - 1;
-      if (lane > first) mine = 0;
-    }
-    for (int d = 16; d > 0; d >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, d);
-    excl += __shfl_sync(0xffffffffu, mine, 0);
-    if (incl != 0) break;
-    window -= 32;
+#pragma unroll
+    for (int w = 0; w < kWords; ++w) excl += v[w] & kValueMask;
   }
-  if (lane == 0) st_release(&status[tile], kFlagIncl | (excl + tile_total));
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) excl += __shfl_xor_sync(0xffffffffu, excl, d);
+  if (lane == 0) st_status(&status[tile], kFlagIncl | (excl + tile_total));
   return excl;
 }
 
