@@ -737,8 +737,8 @@ def _operator_case(args):
 
         prof = _kernel_profile(_abi.lib(), _abi, fn, args.steps)
         kern = {k: v["ms"] / args.steps for k, v in prof.items()}
-        ms = sum(kern.get(k, 0.0) for k in ("shuffle_count_kernel", "scan_i32_kernel", "shuffle_scatter_kernel"))
-        # the key read twice (count, scatter), every column read and written once
+        ms = sum(kern.get(k, 0.0) for k in ("shuffle_count_kernel", "shuffle_scan_kernel", "shuffle_scatter_kernel"))
+        # the key and 8 B for the slots, every column read and written once
         algo = n * (8 + 8 + 2 * (8 + 8 + 4))
         print(json.dumps({"case": "shuffle", "rows": n, "slots": args.slots, "kernels_ms": kern, "shuffle_ms": ms,
                           "algorithmic_gbs": algo / (ms * 1e6), "rows_per_s": n / (ms * 1e-3)}))
@@ -817,7 +817,7 @@ def _operator_case(args):
         for _ in range(max(3, args.warmup)):
             fn()
         ms = _kernel_ms(lambda: f.evaluate(dt, project=["c", "d"]),
-                        ("select_kernel", "select_probe_kernel", "select_gather_kernel"), args.steps)
+                        ("select_kernel", "select_scan_kernel", "select_probe_kernel", "select_gather_kernel"), args.steps)
         algo = n * 12 + sel * 24  # a, b over every row; c, d read and written for the selected rows
         print(json.dumps({"case": "filter", "rows": n, "selected": sel, "kernel_ms": ms,
                           "algorithmic_gbs": algo / (ms * 1e6)}))

@@ -350,10 +350,14 @@ ShuffleResult shuffle_rows(const TupleSetPtr& in_ts, const std::vector<std::stri
     after_launch("shuffle_count_kernel");
     prof.stop(static_cast<double>(n) * (4.0 * p.n_keys + 2.0) + static_cast<double>(cells) * 4.0);
   }
-  const int64_t scan_threads = std::min<int64_t>(1024, (p.ntiles + 31) / 32 * 32);
-  shuffle_scan_kernel<<<static_cast<int>(num_slots), static_cast<int>(scan_threads), 0, s>>>(starts->as<int32_t>(),
-                                                                                             p.ntiles, totals);
-  after_launch("shuffle_scan_kernel");
+  {
+    ProfScope prof("shuffle_scan_kernel", s);
+    const int64_t threads = std::min<int64_t>(1024, (p.ntiles + 31) / 32 * 32);
+    shuffle_scan_kernel<<<static_cast<int>(num_slots), static_cast<int>(threads), 0, s>>>(starts->as<int32_t>(),
+                                                                                          p.ntiles, totals);
+    after_launch("shuffle_scan_kernel");
+    prof.stop(2.0 * static_cast<double>(cells) * 4.0);
+  }
 
   // Output columns: fixed-width ones scattered by the kernel (in groups of
   // kShufMaxFixed, the ranking repeated per group), utf8 ones gathered
