@@ -392,14 +392,17 @@ __global__ void __launch_bounds__(NT) group_update_kernel(const __grid_constant_
     atomicAdd(reinterpret_cast<unsigned long long*>(&p.st->aux[0]), static_cast<unsigned long long>(s_claims));
 }
 
-// Large exact batches whose aggregates are counts and sums, minima or maxima
-// of plain integer columns. Bound by issue and by the lanes that wait: the
+// Exact batches of kGroupPlainRows rows and more whose aggregates are counts
+// and sums, minima or maxima of plain integer columns. Bound by issue and by the lanes that wait: the
 // code is straight where the kernel above interprets each accumulator of each
 // row (606 instructions per 32 rows there, 373 here), two rows of a lane are
 // in flight, and rows that miss the shared table queue up until they fill
 // two rounds of a warp. 1024 threads with two rows each: 512 with four took
 // 1.6 times as long, 768 with two or three 1.25 times. 20M rows, SUM, COUNT and
-// MAX: 0.9M groups (Zipf) 384 us against 621, 1000 groups 193 against 347. A
+// MAX: 0.9M groups (Zipf) 384 us against 621, 1000 groups 193 against 347; 1M
+// rows of 10, 1000, 20k and 500k keys 23, 28, 32 and 38 us against 39, 51, 58
+// and 66, 250k rows 16 to 22 against 20 to 31, 100k rows 18 to 24 both ways,
+// so batches from about 200k rows on take it. A
 // row reads its set's four one-byte tags and then one key: with the four keys
 // read instead the random 16-byte reads' bank conflicts made it 403 and 228.
 struct PlainAcc {
@@ -409,6 +412,7 @@ struct PlainAcc {
   int64_t flip;      // -1 for a minimum, which is kept as the maximum of ~x
 };
 
+constexpr int64_t kGroupPlainRows = 3 << 16;
 constexpr int kPlainAccs = 4;
 constexpr int kPlainThreads = 1024;
 constexpr int kPlainRows = 2;  // rows of a lane in flight
@@ -1601,7 +1605,7 @@ class GroupTable {
     p.use_smem = (hint == 0 || hint <= 4096) ? 1 : 0;
     ProfScope prof("group_update_kernel", s);
     PlainParams plain;
-    if (p.use_smem && ts.exact() && n >= kGroupLargeRows && plain_params(p, &plain)) {
+    if (p.use_smem && ts.exact() && n >= kGroupPlainRows && plain_params(p, &plain)) {
       using PlainKernel = void (*)(GroupParams, PlainParams);
       static const PlainKernel table[kPlainAccs] = {group_update_plain_kernel<1, false>, group_update_plain_kernel<2, false>,
                                                     group_update_plain_kernel<3, false>, group_update_plain_kernel<4, false>};
@@ -1610,7 +1614,8 @@ class GroupTable {
       p.sm_slots = static_cast<int32_t>((max_smem_optin() - 1024 - plain_smem(0, 0)) / (per_slot + 1)) / kPlainWays * kPlainWays;
       const int64_t dyn = plain_smem(p.sm_slots, p.n_acc);
       GF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn)));
-      fn<<<num_sms(), kPlainThreads, dyn, s>>>(p, plain);
+      const int64_t step = kPlainThreads * kPlainRows;
+      fn<<<static_cast<int>(std::min<int64_t>(num_sms(), (n + step - 1) / step)), kPlainThreads, dyn, s>>>(p, plain);
     } else if (p.use_smem && ts.exact() && n >= kGroupLargeRows) {
       static std::once_flag configured;
       std::call_once(configured, [] {

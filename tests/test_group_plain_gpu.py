@@ -72,3 +72,13 @@ def test_kinds(gpu, aggs, groups):
 @pytest.mark.parametrize("rows", [LARGE, LARGE + 1, LARGE + 31, LARGE + 32, LARGE + 33, LARGE + 63, LARGE + 2047, 5_000_001])
 def test_keys_and_rows(gpu, keys, rows):
     check(table(rows, 200_000, rows % 97), keys, [("SUM", "v"), ("COUNT", None), ("MAX", "q")])
+
+
+@pytest.mark.parametrize("aggs", [[("SUM", "v"), ("COUNT", None), ("MAX", "q")], [("MIN", "v"), ("SUM", "q")]],
+                         ids=["3", "2"])
+@pytest.mark.parametrize("groups", [1, 7, 5000, 150_000])
+@pytest.mark.parametrize("rows", [(3 << 16) - 1, 3 << 16, (3 << 16) + 1, 152 * 2048 - 1, 152 * 2048, 152 * 2048 + 1])
+def test_smallest_batches(gpu, rows, groups, aggs):
+    """Batches around the size from which they take the plain kernel, and
+    around one step of every block."""
+    check(table(rows, groups, rows % 89), ["w"], aggs)
