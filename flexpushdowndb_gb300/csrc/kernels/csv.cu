@@ -329,7 +329,7 @@ __device__ __forceinline__ unsigned div_fields(const CsvParams& p, unsigned j) {
   return p.inv_fields == 0 ? j : __umulhi(j, p.inv_fields);  // exact for j * n_fields < 2^32
 }
 
-// The 16 KiB tile and the kCsvFront bytes before it into `text`, without a barrier.
+// The 32 KiB tile and the kCsvFront bytes before it into `text`, without a barrier.
 __device__ __forceinline__ void stage_tile(const CsvParams& p, uint4* text) {
   constexpr int kEach = kCsvTile / 16 / kCsvThreads;
   const int64_t tile0 = static_cast<int64_t>(blockIdx.x) * kCsvTile;
