@@ -228,32 +228,32 @@ __device__ __forceinline__ uint64_t lookback_exclusive(uint64_t* status, int64_t
   return excl;
 }
 
-// Block-wide exclusive sum of one int per thread (blockDim.x <= 1024).
+// Block-wide exclusive sum of one value per thread (blockDim.x <= 1024).
 // Returns the thread's exclusive prefix; *total gets the block sum.
-template <int THREADS>
-__device__ __forceinline__ int block_exclusive_sum(int x, int* total, int* s_warp) {
+template <int THREADS, class T>
+__device__ __forceinline__ T block_exclusive_sum(T x, T* total, T* s_warp) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   constexpr int NW = THREADS / 32;
-  int incl = x;
+  T incl = x;
   for (int d = 1; d < 32; d <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, incl, d);
+    T y = __shfl_up_sync(0xffffffffu, incl, d);
     if (lane >= d) incl += y;
   }
   if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    int w = lane < NW ? s_warp[lane] : 0;
-    int wi = w;
+    T w = lane < NW ? s_warp[lane] : 0;
+    T wi = w;
     for (int d = 1; d < 32; d <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, wi, d);
+      T y = __shfl_up_sync(0xffffffffu, wi, d);
       if (lane >= d) wi += y;
     }
     if (lane < NW) s_warp[lane] = wi - w;
     if (lane == NW - 1) s_warp[NW] = wi;
   }
   __syncthreads();
-  int r = incl - x + s_warp[warp];
+  T r = incl - x + s_warp[warp];
   *total = s_warp[NW];
   return r;
 }

@@ -104,7 +104,7 @@ template <int kItems>
 __global__ void __launch_bounds__(kScanThreads)
     scan_i32_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, int64_t n, int64_t n_tiles,
                     uint64_t* tile_status, uint32_t* ticket, DevStatus* st) {
-  __shared__ int s_warp[kScanThreads / 32 + 1];
+  __shared__ int64_t s_warp[kScanThreads / 32 + 1];
   __shared__ uint32_t s_tile;
   __shared__ uint64_t s_base;
   const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
@@ -129,11 +129,13 @@ __global__ void __launch_bounds__(kScanThreads)
 #pragma unroll
       for (int k = 0; k < kItems; ++k) v[k] = row0 + k < n ? in[row0 + k] : 0;
     }
-    int sum = 0;
+    // 64 bits: a tile's values can sum to more than 2^31, and the total says
+    // so to the caller, who then stores nothing by these offsets
+    int64_t sum = 0;
 #pragma unroll
     for (int k = 0; k < kItems; ++k) sum += v[k];
-    int total;
-    int excl = block_exclusive_sum<kScanThreads>(sum, &total, s_warp);
+    int64_t total;
+    const int64_t excl = block_exclusive_sum<kScanThreads>(sum, &total, s_warp);
     if (threadIdx.x < 32) {
       uint64_t b = lookback_exclusive(tile_status, tile, static_cast<uint64_t>(total), st);
       if (threadIdx.x == 0) s_base = b;
@@ -380,7 +382,7 @@ int64_t exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, cudaStrea
   GF_CUDA(cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, s));
   sync(s);
   raise_device_status(hs, "prefix sum");
-  if (hs.value > INT32_MAX) fail(GFPDB_EUNSUPPORTED, "utf8 column exceeds 2 GiB of bytes");
+  if (hs.value > INT32_MAX || hs.value < 0) fail(GFPDB_EUNSUPPORTED, "utf8 column exceeds 2 GiB of bytes");
   return hs.value;
 }
 
