@@ -1,5 +1,7 @@
 #include "runtime.h"
 
+#include "shared_limits.h"
+
 #include <mutex>
 #include <vector>
 
@@ -93,6 +95,13 @@ void ensure_device() {
 
 int num_sms() { return info_for(current_device()).sms; }
 int max_smem_optin() { return info_for(current_device()).smem_optin; }
+
+void allow_shared(const void* kernel, int64_t bytes) {
+  static SharedLimits limits;
+  limits.raise(current_device(), kernel, static_cast<int>(bytes), [&](int b) {
+    GF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
+  });
+}
 
 namespace {
 thread_local Arena* g_thread_arena = nullptr;

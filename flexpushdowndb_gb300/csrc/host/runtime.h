@@ -81,6 +81,13 @@ int current_device();
 void ensure_device();            // gfpdb_device_init on first use
 int num_sms();                   // SM count of the current device
 int max_smem_optin();            // opt-in shared memory per block
+// Lets launches of `kernel` on the current device have `bytes` of dynamic
+// shared memory (shared_limits.h).
+void allow_shared(const void* kernel, int64_t bytes);
+template <class... Args>
+void allow_shared(void (*kernel)(Args...), int64_t bytes) {
+  allow_shared(reinterpret_cast<const void*>(kernel), bytes);
+}
 
 // Stream-ordered device allocation. Memory comes from the device's default
 // memory pool with an unbounded release threshold, so repeated queries reuse

@@ -335,7 +335,7 @@ ShuffleResult shuffle_rows(const TupleSetPtr& in_ts, const std::vector<std::stri
   const auto scatter = num_slots <= 32    ? shuffle_scatter_kernel<5>
                        : num_slots <= 256 ? shuffle_scatter_kernel<8>
                                           : shuffle_scatter_kernel<10>;
-  GF_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_scatter)));
+  allow_shared(scatter, smem_scatter);
 
   const int64_t cells = num_slots * p.ntiles;
   auto row_slot = make_buffer(n * 2, s);
