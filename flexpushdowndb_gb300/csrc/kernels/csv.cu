@@ -40,7 +40,6 @@
 // of a tile fill more of its last warp step, and per-tile work halves.
 #include <algorithm>
 #include <cstring>
-#include <mutex>
 
 #include "common.cuh"
 #include "launch.h"
@@ -827,13 +826,8 @@ TupleSetPtr csv_parse(const char* device_text, int64_t n_bytes, char delimiter, 
   if (static_cast<int>(fields.size()) > 256) fail(GFPDB_EUNSUPPORTED, "too many CSV fields per line");
   if (n_bytes >= (int64_t{1} << 40)) fail(GFPDB_EUNSUPPORTED, "CSV text too large");
   const uint8_t* text = reinterpret_cast<const uint8_t*>(device_text);
-  static std::once_flag configured;  // above 48 KB of shared memory a block
-  std::call_once(configured, [] {
-    GF_CUDA(cudaFuncSetAttribute(csv_fields_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 csv_fields_smem(1)));  // the most
-    GF_CUDA(cudaFuncSetAttribute(csv_strings_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 csv_strings_smem(kCsvWarps)));
-  });
+  allow_shared(csv_fields_kernel, csv_fields_smem(1));  // the most
+  allow_shared(csv_strings_kernel, csv_strings_smem(kCsvWarps));
   if ((reinterpret_cast<uintptr_t>(text) & 15u) != 0) fail(GFPDB_EINVAL, "CSV text must be 16-byte aligned");
 
   if (static_cast<int>(fields.size()) > kCsvMaxFields) fail(GFPDB_EUNSUPPORTED, "too many CSV fields per line");

@@ -36,7 +36,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "eval.cuh"
@@ -1613,16 +1612,12 @@ class GroupTable {
       const PlainKernel fn = beside ? group_update_plain_kernel<3, true> : table[p.n_acc - 1];
       p.sm_slots = static_cast<int32_t>((max_smem_optin() - 1024 - plain_smem(0, 0)) / (per_slot + 1)) / kPlainWays * kPlainWays;
       const int64_t dyn = plain_smem(p.sm_slots, p.n_acc);
-      GF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn)));
+      allow_shared(fn, dyn);
       const int64_t step = kPlainThreads * kPlainRows;
       fn<<<static_cast<int>(std::min<int64_t>(num_sms(), (n + step - 1) / step)), kPlainThreads, dyn, s>>>(p, plain);
     } else if (p.use_smem && ts.exact() && n >= kGroupLargeRows) {
-      static std::once_flag configured;
-      std::call_once(configured, [] {
-        GF_CUDA(cudaFuncSetAttribute(group_update_kernel<kGroupLargeThreads>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 2048));
-      });
       // the opt-in limit less the kernel's static shared memory
+      allow_shared(group_update_kernel<kGroupLargeThreads>, max_smem_optin() - 2048);
       p.sm_slots = static_cast<int32_t>((max_smem_optin() - 2048 - group_smem(kGroupLargeThreads, 0, 0)) / per_slot);
       group_update_kernel<kGroupLargeThreads>
           <<<num_sms(), kGroupLargeThreads, group_smem(kGroupLargeThreads, p.sm_slots, p.n_acc), s>>>(p);

@@ -23,7 +23,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <set>
+#include <tuple>
 #include <type_traits>
 
 #include "../host/handles.h"
@@ -353,27 +353,28 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(const __grid_consta
   }
 }
 
-// Resident CTAs per SM for a variant and dynamic shared-memory size, cached
-// (the occupancy query is not free and the answer never changes).
-int select_blocks_per_sm(bool with_pred, size_t dyn) {
+// Resident CTAs per SM of a kernel on the current device for a dynamic
+// shared-memory size (`most`: the largest it is launched with), cached: the
+// occupancy query is not free and the answer never changes.
+int resident_blocks(const void* fn, int threads, size_t dyn, int64_t most) {
   static std::mutex mu;
-  static std::map<std::pair<bool, size_t>, int> cache;
-  static bool attr_set[2] = {false, false};
+  static std::map<std::tuple<int, const void*, size_t>, int> cache;
   std::lock_guard<std::mutex> lk(mu);
-  auto key = std::make_pair(with_pred, dyn);
+  const auto key = std::make_tuple(current_device(), fn, dyn);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
-  const void* fn = with_pred ? reinterpret_cast<const void*>(select_kernel<true>)
-                             : reinterpret_cast<const void*>(select_kernel<false>);
-  if (!attr_set[with_pred]) {
-    GF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kBloomSmemBudget));
-    attr_set[with_pred] = true;
-  }
+  allow_shared(fn, most);
   int per_sm = 0;
-  GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSelThreads, dyn));
+  GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn));
   if (per_sm < 1) per_sm = 1;
   cache[key] = per_sm;
   return per_sm;
+}
+
+int select_blocks_per_sm(bool with_pred, size_t dyn) {
+  const void* fn = with_pred ? reinterpret_cast<const void*>(select_kernel<true>)
+                             : reinterpret_cast<const void*>(select_kernel<false>);
+  return resident_blocks(fn, kSelThreads, dyn, kBloomSmemBudget);
 }
 
 // A predicate leaf of the simple form: an integer column against an integer
@@ -956,23 +957,7 @@ ProbeKernel select_probe_fn(bool with_pred, int n_later) {
   return table[with_pred ? 1 : 0][k];
 }
 
-int two_pass_blocks_per_sm(const void* f, size_t dyn) {
-  static std::mutex mu;
-  static std::map<std::pair<const void*, size_t>, int> cache;
-  static std::set<const void*> attr_set;
-  std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_pair(f, dyn);
-  auto it = cache.find(key);
-  if (it != cache.end()) return it->second;
-  if (!attr_set.count(f)) {
-    GF_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSpMaxDynamic)));
-    attr_set.insert(f);
-  }
-  int per_sm = 0;
-  GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kPwThreads, dyn));
-  cache[key] = per_sm;
-  return per_sm;
-}
+int two_pass_blocks_per_sm(const void* fn, size_t dyn) { return resident_blocks(fn, kPwThreads, dyn, kSpMaxDynamic); }
 
 // ---------------------------------------------------------------------------
 // Compact selection for small inputs (dimension tables, small partitions).
@@ -1370,7 +1355,7 @@ TupleSetPtr select_rows(const TupleSet& in, const CompiledPredicate* pred, const
         const size_t dyn = static_cast<size_t>(p.smem_words) * 4;
         const ProbeKernel fn = select_probe_fn(spred.n_leaves > 0, p.n_probes - 1);
         const int per_sm = two_pass_blocks_per_sm(reinterpret_cast<const void*>(fn), dyn);
-        const int64_t cap = static_cast<int64_t>(num_sms()) * (per_sm > 0 ? per_sm : 1);
+        const int64_t cap = static_cast<int64_t>(num_sms()) * per_sm;
         fn<<<static_cast<int>(want < cap ? want : cap), kPwThreads, dyn, s>>>(p, spred, rowlist->as<int32_t>(),
                                                                              counts, range_totals);
       } else {
@@ -1382,7 +1367,7 @@ TupleSetPtr select_rows(const TupleSet& in, const CompiledPredicate* pred, const
         q.range_totals = range_totals;
         const size_t dyn = static_cast<size_t>(kPwThreads / 32) * kScanStages * q.row_bytes * kPwRows;
         const int per_sm = two_pass_blocks_per_sm(reinterpret_cast<const void*>(select_scan_kernel), dyn);
-        const int64_t cap = static_cast<int64_t>(num_sms()) * (per_sm > 0 ? per_sm : 1);
+        const int64_t cap = static_cast<int64_t>(num_sms()) * per_sm;
         select_scan_kernel<<<static_cast<int>(want < cap ? want : cap), kPwThreads, dyn, s>>>(q);
       }
       after_launch(name);

@@ -23,7 +23,6 @@
 // keys); a repeated key is reported as an error.
 #include <algorithm>
 #include <cstring>
-#include <mutex>
 
 #include "common.cuh"
 #include "launch.h"
@@ -1893,13 +1892,9 @@ void StarBatchState::prepare(cudaStream_t s) {
 // finish its stripe after everyone else.
 template <int ITEMS, typename M>
 static void launch_fact_items(const SBFactParams& p, size_t smem, int grid, cudaStream_t s) {
-  // Opt in once to the largest dynamic size this engine asks for (static
-  // plus dynamic shared memory above 48 KB needs it).
-  static std::once_flag configured;
-  std::call_once(configured, [] {
-    GF_CUDA(cudaFuncSetAttribute(sb_fact_kernel<ITEMS, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kSBSmemMaxDynamic)));
-  });
+  // The largest dynamic size this engine asks for (static plus dynamic shared
+  // memory above 48 KB needs it).
+  allow_shared(sb_fact_kernel<ITEMS, M>, kSBSmemMaxDynamic);
   int per_sm = 0;
   GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sb_fact_kernel<ITEMS, M>, kSBFactThreads, smem));
   if (per_sm < 1) fail(GFPDB_EUNSUPPORTED, "the batched fact stage does not fit on an SM with these settings");
@@ -1919,11 +1914,7 @@ static void launch_fact_mask(const SBFactParams& p, size_t smem, int grid, cudaS
 
 template <int ITEMS, typename M>
 static void launch_direct_items(const SBFactParams& p, size_t smem, int64_t tiles, cudaStream_t s) {
-  static std::once_flag configured;
-  std::call_once(configured, [] {
-    GF_CUDA(cudaFuncSetAttribute(sb_fact_direct_kernel<ITEMS, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kSBSmemMaxDynamic)));
-  });
+  allow_shared(sb_fact_direct_kernel<ITEMS, M>, kSBSmemMaxDynamic);
   int per_sm = 0;
   GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sb_fact_direct_kernel<ITEMS, M>, kSBDirectThreads,
                                                         smem));

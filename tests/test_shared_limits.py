@@ -65,6 +65,14 @@ def test_limits_only_rise(tmp_path):
     assert subprocess.run([str(tmp_path / "limits")], capture_output=True, text=True, check=True).stdout == f"0 0 0 1 {1 << 20}"
 
 
+def test_every_limit_is_kept_per_device():
+    """A process may use several devices, and each has its own limits: no
+    source sets one but allow_shared."""
+    sources = [p for kind in ("*.cu", "*.cuh", "*.cpp", "*.h") for p in HOST.parent.rglob(kind)]
+    assert len(sources) > 10
+    assert [p.name for p in sources if "MaxDynamicSharedMemorySize" in p.read_text()] == ["runtime.cpp"]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("slots", [(256, 256), (1000, 300), (20, 32)])
 def test_shuffles_from_two_threads(gpu, slots):
