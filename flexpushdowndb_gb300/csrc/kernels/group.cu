@@ -45,24 +45,12 @@ namespace gfpdb {
 
 namespace {
 
-// Two block shapes. Batches of kGroupLargeRows rows and more, counted on the
-// host, run one CTA of 1,024 threads per SM whose shared-memory table takes
-// most of the SM (6,000 slots at three accumulators): a frequent key is then
-// kept once per SM and not once per 256-thread CTA, and the table holds more
-// of them. Smaller and device-counted batches run CTAs of 256 threads with
-// 1,024 slots, whose tables are quicker to clear and merge. Measured with 20M
-// rows of Zipf(1.1) int64 keys over 10M values and three aggregates: 609 us
-// and about 40% of the rows in the global table, against 1,126 us and 69% with
-// 760 small CTAs (rows that missed not queued, 64-bit shared-memory atomics);
-// with 200,000 rows of five keys the small CTAs take 17 us (66 us before).
 constexpr int kGroupThreads = 256;
-constexpr int kGroupLargeThreads = 1024;
-constexpr int64_t kGroupLargeRows = 2 << 20;
-constexpr int kGroupSmemSlotsMax = 1024;  // slots of a small CTA's shared-memory table
+constexpr int kGroupSmemSlotsMax = 1024;  // slots of a CTA's shared-memory table
 constexpr int kGroupQueue = 64;           // rows of a warp waiting for the global table (two rounds of 32)
-// A large CTA's table takes in a key on its second sight: a bit per hash
-// value remembers the first. Keys seen once would otherwise fill the table
-// before the frequent ones have all come by.
+// group_update_plain_kernel's table takes in a key on its second sight: a bit
+// per hash value remembers the first. Keys seen once would otherwise fill the
+// table before the frequent ones have all come by.
 constexpr int kGroupSeenBits = 1 << 16;
 constexpr int kGroupSmemProbes = 4;       // shared-memory slots a row tries before the global table
 constexpr uint32_t kDictSpinLimit = 1u << 20;
@@ -88,8 +76,8 @@ struct GroupParams {
   unsigned long long* accs;
   uint64_t mask;
   int32_t key_stride, acc_stride;
-  int32_t use_smem;
   int32_t sm_slots;
+  int32_t float_sums;         // a float64 sum is among the accumulators
   DevStatus* st;  // aux[0]: groups claimed, aux[1]: special slot used
   Program prog;
 };
@@ -231,35 +219,18 @@ __device__ __forceinline__ unsigned long long row_value(const GroupParams& p, co
   return program_value(p, a, row);
 }
 
-// The accumulators of four aggregates at a time: their inputs are loaded
-// together before the first is combined.
-template <class Combine>
-__device__ __forceinline__ void add_row(const GroupParams& p, int64_t row, Combine&& combine) {
-  for (int a0 = 0; a0 < p.n_acc; a0 += 4) {
-    unsigned long long v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = a0 + u < p.n_acc ? row_value(p, p.acc[a0 + u], row) : 0ull;
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (a0 + u < p.n_acc) combine(a0 + u, v[u]);
-  }
-}
-
-// A warp's rows waiting for the global table: a ring of kGroupQueue.
-struct GroupQueue {
-  uint64_t* key;
-  int32_t* row;
-  unsigned head, tail;
-};
-
-// The first n (at most 32) waiting rows into the global table, one per lane.
-__device__ __forceinline__ void drain_queue(const GroupParams& p, GroupQueue& q, int n, int lane, unsigned* claims) {
-  if (lane < n) {
-    const unsigned e = (q.head + lane) & (kGroupQueue - 1);
-    const uint64_t key = q.key[e];
-    const int64_t row = q.row[e];
-    uint64_t g = UINT64_MAX;
-    for (int a0 = 0; a0 == 0 || a0 < p.n_acc; a0 += 4) {
+// A row into the global table; the first values are asked for before the slot.
+template <int A>
+__device__ __forceinline__ void add_global(const GroupParams& p, uint64_t key, int64_t row, unsigned* claims) {
+  uint64_t g = UINT64_MAX;
+  if constexpr (A == 0) {
+    global_slot(p, key, claims);
+  } else if constexpr (A == 1) {
+    const unsigned long long v = row_value(p, p.acc[0], row);
+    g = global_slot(p, key, claims);
+    if (g != UINT64_MAX) acc_combine(p.accs + g * p.acc_stride, p.acc[0].fn, p.acc[0].vt, v);
+  } else {
+    for (int a0 = 0; a0 < p.n_acc; a0 += 4) {
       unsigned long long v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) v[u] = a0 + u < p.n_acc ? row_value(p, p.acc[a0 + u], row) : 0ull;
@@ -273,32 +244,60 @@ __device__ __forceinline__ void drain_queue(const GroupParams& p, GroupQueue& q,
           acc_combine(p.accs + g * p.acc_stride + a0 + u, p.acc[a0 + u].fn, p.acc[a0 + u].vt, v[u]);
     }
   }
-  __syncwarp();
-  q.head += n;
 }
 
-// Bytes of a CTA's dynamic shared memory: the table, the large shape's seen
-// bits, the warps' queues.
-constexpr int64_t group_smem(int threads, int64_t slots, int n_acc) {
-  return slots * (8 + 8 * n_acc) + (threads == kGroupLargeThreads ? kGroupSeenBits / 8 : 0) +
-         static_cast<int64_t>(threads / 32) * kGroupQueue * 12;
+// Bytes of a CTA's dynamic shared memory: the table and the warps' queues.
+constexpr int64_t group_smem(int64_t slots, int n_acc) {
+  return slots * (8 + 8 * n_acc) + kGroupThreads / 32 * kGroupQueue * 12;
 }
 
-// Any accumulators, any batch: each row's are interpreted one by one, and
-// issue holds it. Large exact batches of plain aggregates take
-// group_update_plain_kernel.
-template <int NT>
-__global__ void __launch_bounds__(NT) group_update_kernel(const __grid_constant__ GroupParams p) {
-  constexpr bool kLarge = NT == kGroupLargeThreads;
+// Every row straight to the global table (the caller expects many groups).
+// Bound by the latency of its atomics, so registers count: 40 to 48 of them,
+// five to six CTAs an SM. With the first four values loaded before the slot is
+// looked up (62 registers) 4M rows of 200k keys took 17 us more (175, call).
+template <int A>
+__global__ void __launch_bounds__(kGroupThreads) group_update_global_kernel(const __grid_constant__ GroupParams p) {
+  __shared__ unsigned s_claims;
+  const int64_t n_rows = clamp_rows(p.n_dev, p.n_rows);
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * kGroupThreads;
+  if (first >= n_rows) return;
+  if (threadIdx.x == 0) s_claims = 0;
+  __syncthreads();
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kGroupThreads;
+  for (int64_t r = first + threadIdx.x; r < n_rows; r += stride) {
+    const uint64_t g = global_slot(p, pack_key(p, r), &s_claims);
+    if (A == 0 || g == UINT64_MAX) continue;
+    for (int a = 0; a < (A < 2 ? A : p.n_acc); ++a)
+      acc_combine(p.accs + g * p.acc_stride + a, p.acc[a].fn, p.acc[a].vt, row_value(p, p.acc[a], r));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_claims != 0)
+    atomicAdd(reinterpret_cast<unsigned long long*>(&p.st->aux[0]), static_cast<unsigned long long>(s_claims));
+}
+
+// Any accumulators, any batch; large exact batches of plain aggregates take
+// group_update_plain_kernel. A: the accumulators, 2 for any number. Issue and
+// the latency of shared-memory atomics hold it, so five CTAs an SM, which 48
+// registers allow: with the next key loaded a step ahead (63 registers, four
+// CTAs) 20M rows of 100 keys took 572 us instead of 533 for a computed sum and
+// a count, 645 instead of 586 for six aggregates. One accumulator's value and
+// the next key are loaded ahead all the same (100 keys 331 us, 351 without).
+// One CTA of 1,024 threads an SM with a table of most of its shared memory,
+// tried for batches of 2M rows and more, took 31 ms instead of 8 for 20M rows
+// of a float64 sum: one address for all of an SM's rows.
+template <int A>
+__global__ void __launch_bounds__(kGroupThreads, 5) group_update_kernel(const __grid_constant__ GroupParams p) {
+  constexpr int NT = kGroupThreads;
+  constexpr bool kAhead = A == 1;
   extern __shared__ unsigned long long s_mem[];
   __shared__ int s_scan[NT / 32 + 1];
   __shared__ unsigned s_claims;
-  const int S = p.use_smem ? p.sm_slots : 0;
+  const int S = p.sm_slots;  // a power of two
+  const int n_acc = A < 2 ? A : p.n_acc;
   uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_mem);
   unsigned long long* s_acc = s_mem + S;  // [accumulator][slot]
-  uint64_t* s_qkey = reinterpret_cast<uint64_t*>(s_acc + static_cast<int64_t>(S) * p.n_acc);
+  uint64_t* s_qkey = reinterpret_cast<uint64_t*>(s_acc + static_cast<int64_t>(S) * n_acc);
   int32_t* s_qrow = reinterpret_cast<int32_t*>(s_qkey + (NT / 32) * kGroupQueue);
-  unsigned* s_seen = reinterpret_cast<unsigned*>(s_qrow + (NT / 32) * kGroupQueue);
   const int64_t n_rows = clamp_rows(p.n_dev, p.n_rows);
   // A grid sized for a capacity can be far larger than the rows that arrive:
   // CTAs without rows leave before touching shared memory (uniform per CTA).
@@ -306,36 +305,42 @@ __global__ void __launch_bounds__(NT) group_update_kernel(const __grid_constant_
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_claims = 0;
   for (int i = threadIdx.x; i < S; i += NT) s_keys[i] = kEmptySlot;
-  for (int a = 0; a < p.n_acc; ++a) {
+  for (int a = 0; a < n_acc; ++a) {
     const unsigned long long v = acc_identity(p.acc[a].fn, p.acc[a].vt);
     for (int i = threadIdx.x; i < S; i += NT) s_acc[a * S + i] = v;
   }
-  if (kLarge)
-    for (int i = threadIdx.x; i < kGroupSeenBits / 32; i += NT) s_seen[i] = 0;
   __syncthreads();
-  GroupQueue q{s_qkey + warp * kGroupQueue, s_qrow + warp * kGroupQueue, 0, 0};
+  // the warp's rows waiting for the global table, a ring of kGroupQueue; the
+  // first n (at most 32) go into it together, one per lane
+  uint64_t* q_key = s_qkey + warp * kGroupQueue;
+  int32_t* q_row = s_qrow + warp * kGroupQueue;
+  unsigned head = 0, tail = 0;  // the same in every lane
+  auto drain = [&](int n) {
+    if (lane < n) {
+      const unsigned e = (head + lane) & (kGroupQueue - 1);
+      add_global<A>(p, q_key[e], q_row[e], &s_claims);
+    }
+    __syncwarp();
+    head += n;
+  };
   const int64_t stride = static_cast<int64_t>(gridDim.x) * NT;
   int64_t base = static_cast<int64_t>(blockIdx.x) * NT + warp * 32;
-  uint64_t next = base + lane < n_rows ? pack_key(p, base + lane) : 0;
+  uint64_t next = kAhead && base + lane < n_rows ? pack_key(p, base + lane) : 0;
   for (; base < n_rows; base += stride) {
     const int64_t r = base + lane;
-    const uint64_t key = next;
-    if (r + stride < n_rows) next = pack_key(p, r + stride);  // a step ahead of its use
+    const uint64_t key = kAhead ? next : r < n_rows ? pack_key(p, r) : 0;
+    if (kAhead && r + stride < n_rows) next = pack_key(p, r + stride);
+    const unsigned long long v0 = kAhead && r < n_rows ? row_value(p, p.acc[0], r) : 0ull;
     int found = -1;
-    if (r < n_rows && S > 0 && key != kEmptySlot) {
+    if (r < n_rows && key != kEmptySlot) {
       // A short probe run: with few groups the table is sparse and a key is
       // found or placed in a step or two; with many groups (high-cardinality
       // keys) the table is soon full and a longer run only delays the row's
       // trip to the global table.
-      const uint64_t h = hash_key(static_cast<int64_t>(key));
-      int slot = static_cast<int>(__umulhi(static_cast<unsigned>(h >> 32), static_cast<unsigned>(S)));
+      int slot = static_cast<int>(hash_key(static_cast<int64_t>(key))) & (S - 1);
       for (int i = 0; i < kGroupSmemProbes; ++i) {
         uint64_t k = *reinterpret_cast<volatile uint64_t*>(s_keys + slot);
         if (k == kEmptySlot) {
-          if (kLarge) {
-            const unsigned bit = static_cast<unsigned>(h) & (kGroupSeenBits - 1);
-            if ((atomicOr(s_seen + (bit >> 5), 1u << (bit & 31)) >> (bit & 31) & 1u) == 0) break;  // first sight
-          }
           k = atomicCAS(reinterpret_cast<unsigned long long*>(s_keys + slot),
                         static_cast<unsigned long long>(kEmptySlot), static_cast<unsigned long long>(key));
           if (k == kEmptySlot) k = key;
@@ -344,47 +349,62 @@ __global__ void __launch_bounds__(NT) group_update_kernel(const __grid_constant_
           found = slot;
           break;
         }
-        if (++slot == S) slot = 0;
+        slot = (slot + 1) & (S - 1);
       }
     }
-    if (found >= 0)
-      add_row(p, r, [&](int a, unsigned long long v) { smem_combine(s_acc + a * S + found, p.acc[a].fn, p.acc[a].vt, v); });
-    const bool miss = r < n_rows && found < 0;
-    const unsigned m = __ballot_sync(0xffffffffu, miss);
-    if (miss) {
-      const unsigned e = (q.tail + __popc(m & ((1u << lane) - 1u))) & (kGroupQueue - 1);
-      q.key[e] = key;
-      q.row[e] = static_cast<int32_t>(r);
+    // The warp's rows all go to one slot: their float64 sum is added up in
+    // registers. A double has no native shared-memory addition, and 32 lanes'
+    // compare-and-swap loops on one address go round 32 times (a float64 sum
+    // without keys over 20M rows: 790 us, 8,600 with a loop a row).
+    int same = 0;
+    if (A > 0 && p.float_sums && __all_sync(0xffffffffu, found >= 0)) __match_all_sync(0xffffffffu, found, &same);
+    if (found >= 0) {
+      auto combine = [&](int a, unsigned long long v) {
+        unsigned long long* to = s_acc + a * S + found;
+        if (same && p.acc[a].fn == AGG_SUM && p.acc[a].vt == VT_F64) {
+          double x = __longlong_as_double(static_cast<long long>(v));
+#pragma unroll
+          for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+          if (lane == 0) atomicAdd(reinterpret_cast<double*>(to), x);
+        } else {
+          smem_combine(to, p.acc[a].fn, p.acc[a].vt, v);
+        }
+      };
+      if (A == 1) combine(0, v0);
+      else for (int a = 0; a < n_acc; ++a) combine(a, row_value(p, p.acc[a], r));
     }
-    q.tail += __popc(m);
-    __syncwarp();
-    if (q.tail - q.head >= 32) drain_queue(p, q, 32, lane, &s_claims);
+    const unsigned m = __ballot_sync(0xffffffffu, r < n_rows && found < 0);
+    if (m != 0) {
+      if (m >> lane & 1u) {
+        const unsigned e = (tail + __popc(m & ((1u << lane) - 1u))) & (kGroupQueue - 1);
+        q_key[e] = key;
+        q_row[e] = static_cast<int32_t>(r);
+      }
+      tail += __popc(m);
+      __syncwarp();
+      if (tail - head >= 32) drain(32);
+    }
   }
-  if (q.tail != q.head) drain_queue(p, q, static_cast<int>(q.tail - q.head), lane, &s_claims);
-  auto merge = [&](int i) {
-    const uint64_t g = global_slot(p, s_keys[i], &s_claims);
-    if (g == UINT64_MAX) return;
-    for (int a = 0; a < p.n_acc; ++a)
-      acc_combine(p.accs + g * p.acc_stride + a, p.acc[a].fn, p.acc[a].vt, s_acc[a * S + i]);
-  };
+  if (tail != head) drain(static_cast<int>(tail - head));
   __syncthreads();
-  if (kLarge) {
-    for (int i = threadIdx.x; i < S; i += NT)
-      if (s_keys[i] != kEmptySlot) merge(i);
-  } else if (S > 0) {
-    // Merge into the global table: the occupied slots are listed first (a
-    // block scan), so each thread merges about one group, and every group's
-    // global insert and atomics run in the same round instead of one after
-    // another on the threads that hold several.
-    int c = 0;
-    for (int i = threadIdx.x; i < S; i += NT) c += s_keys[i] != kEmptySlot ? 1 : 0;
-    uint16_t* s_occ = reinterpret_cast<uint16_t*>(s_qkey);  // the queues are empty: at most kGroupSmemSlotsMax entries
-    int occupied;
-    int o = block_exclusive_sum<NT>(c, &occupied, s_scan);
-    for (int i = threadIdx.x; i < S; i += NT)
-      if (s_keys[i] != kEmptySlot) s_occ[o++] = static_cast<uint16_t>(i);
-    __syncthreads();
-    for (int j = threadIdx.x; j < occupied; j += NT) merge(s_occ[j]);
+  // Merge into the global table: the occupied slots are listed first (a
+  // block scan), so each thread merges about one group, and every group's
+  // global insert and atomics run in the same round instead of one after
+  // another on the threads that hold several.
+  int c = 0;
+  for (int i = threadIdx.x; i < S; i += NT) c += s_keys[i] != kEmptySlot ? 1 : 0;
+  uint16_t* s_occ = reinterpret_cast<uint16_t*>(s_qkey);  // the queues are empty: at most kGroupSmemSlotsMax entries
+  int occupied;
+  int o = block_exclusive_sum<NT>(c, &occupied, s_scan);
+  for (int i = threadIdx.x; i < S; i += NT)
+    if (s_keys[i] != kEmptySlot) s_occ[o++] = static_cast<uint16_t>(i);
+  __syncthreads();
+  for (int j = threadIdx.x; j < occupied; j += NT) {
+    const int i = s_occ[j];
+    const uint64_t g = global_slot(p, s_keys[i], &s_claims);
+    if (g == UINT64_MAX) continue;
+    for (int a = 0; a < n_acc; ++a)
+      acc_combine(p.accs + g * p.acc_stride + a, p.acc[a].fn, p.acc[a].vt, s_acc[a * S + i]);
   }
   __syncthreads();
   if (threadIdx.x == 0 && s_claims != 0)
@@ -392,18 +412,19 @@ __global__ void __launch_bounds__(NT) group_update_kernel(const __grid_constant_
 }
 
 // Exact batches of kGroupPlainRows rows and more whose aggregates are counts
-// and sums, minima or maxima of plain integer columns. Bound by issue and by the lanes that wait: the
-// code is straight where the kernel above interprets each accumulator of each
-// row (606 instructions per 32 rows there, 373 here), two rows of a lane are
-// in flight, and rows that miss the shared table queue up until they fill
-// two rounds of a warp. 1024 threads with two rows each: 512 with four took
-// 1.6 times as long, 768 with two or three 1.25 times. 20M rows, SUM, COUNT and
-// MAX: 0.9M groups (Zipf) 384 us against 621, 1000 groups 193 against 347; 1M
-// rows of 10, 1000, 20k and 500k keys 23, 28, 32 and 38 us against 39, 51, 58
-// and 66, 250k rows 16 to 22 against 20 to 31, 100k rows 18 to 24 both ways,
-// so batches from about 200k rows on take it. A
-// row reads its set's four one-byte tags and then one key: with the four keys
-// read instead the random 16-byte reads' bank conflicts made it 403 and 228.
+// and sums, minima or maxima of plain integer columns. Bound by issue and by
+// the lanes that wait: the code is straight where the kernel above interprets
+// each accumulator of each row (373 instructions per 32 rows here), two rows
+// of a lane are in flight, and rows that miss the shared table queue up until
+// they fill two rounds of a warp. 1024 threads with two rows each: 512 with
+// four took 1.6 times as long, 768 with two or three 1.25 times. SUM, COUNT
+// and MAX, the whole call, against the kernel above: 20M rows of 1000 keys 348
+// against 568 us, of Zipf(1.1) keys over 10M values 605 against 811; 1M rows
+// of 10, 1000, 20k and 500k keys 104 to 152 against 125 to 201, 250k rows 87 to
+// 124 against 91 to 146, 100k rows the same both ways, so batches from about
+// 200k rows on take it. A row reads its set's four one-byte tags and then one
+// key: with the four keys read instead the random 16-byte reads' bank
+// conflicts cost 20M rows of 1000 keys 35 us more.
 struct PlainAcc {
   const void* col;   // null: a count
   int32_t wide;      // int64 column
@@ -1581,9 +1602,13 @@ class GroupTable {
       const int64_t b2 = known + fresh;
       // at most 5/8 full with the spare quarter taken, half full without: a
       // table half the size costs the update a little and saves more around
-      // it (0.9M groups of 20M rows, 2M slots against 4M: init 23 against 43
-      // us, update 396 against 371, finalize 44 against 74)
-      const int64_t slots = b2 + b2 * 3 / 5;
+      // it (three accumulators, 0.9M groups of 20M rows, 2M slots against 4M:
+      // init 23 against 43 us, update 396 against 371, finalize 44 against
+      // 74; six, 20M rows of 1M keys: the call 1,150 against 1,225 us). With
+      // fewer accumulators there is less around it, and longer runs cost
+      // more: half full at most (20M rows of 1M keys: no accumulators 520
+      // against 654 us, one 619 against 761, two 923 against 998).
+      const int64_t slots = accs.size() < 3 ? 2 * b2 : b2 + b2 * 3 / 5;
       const uint64_t w2 = next_pow2(static_cast<uint64_t>(slots < 1024 ? 1024 : slots));
       if (w2 < want) want = w2 > cap ? w2 : cap;
     }
@@ -1601,10 +1626,11 @@ class GroupTable {
     p.st = status->as<DevStatus>();
     // Shared-memory pre-aggregation unless the caller expects many groups.
     const int per_slot = 8 + 8 * p.n_acc;
-    p.use_smem = (hint == 0 || hint <= 4096) ? 1 : 0;
+    const bool use_smem = hint == 0 || hint <= 4096;
+    for (int a = 0; a < p.n_acc; ++a) p.float_sums |= accs[a].fn == AGG_SUM && accs[a].vt == VT_F64;
     ProfScope prof("group_update_kernel", s);
     PlainParams plain;
-    if (p.use_smem && ts.exact() && n >= kGroupPlainRows && plain_params(p, &plain)) {
+    if (use_smem && ts.exact() && n >= kGroupPlainRows && plain_params(p, &plain)) {
       using PlainKernel = void (*)(GroupParams, PlainParams);
       static const PlainKernel table[kPlainAccs] = {group_update_plain_kernel<1, false>, group_update_plain_kernel<2, false>,
                                                     group_update_plain_kernel<3, false>, group_update_plain_kernel<4, false>};
@@ -1615,33 +1641,29 @@ class GroupTable {
       allow_shared(fn, dyn);
       const int64_t step = kPlainThreads * kPlainRows;
       fn<<<static_cast<int>(std::min<int64_t>(num_sms(), (n + step - 1) / step)), kPlainThreads, dyn, s>>>(p, plain);
-    } else if (p.use_smem && ts.exact() && n >= kGroupLargeRows) {
-      // the opt-in limit less the kernel's static shared memory
-      allow_shared(group_update_kernel<kGroupLargeThreads>, max_smem_optin() - 2048);
-      p.sm_slots = static_cast<int32_t>((max_smem_optin() - 2048 - group_smem(kGroupLargeThreads, 0, 0)) / per_slot);
-      group_update_kernel<kGroupLargeThreads>
-          <<<num_sms(), kGroupLargeThreads, group_smem(kGroupLargeThreads, p.sm_slots, p.n_acc), s>>>(p);
     } else {
+      using Kernel = void (*)(GroupParams);
+      static const Kernel table[2][3] = {{group_update_global_kernel<0>, group_update_global_kernel<1>, group_update_global_kernel<2>},
+                                         {group_update_kernel<0>, group_update_kernel<1>, group_update_kernel<2>}};
+      const Kernel fn = table[use_smem ? 1 : 0][std::min(p.n_acc, 2)];
       int sm_slots = kGroupSmemSlotsMax;
       // dynamic plus static shared memory stays within the 48 KB a launch
       // gets without opting in to more
-      while (group_smem(kGroupThreads, sm_slots, p.n_acc) > 47 * 1024) sm_slots >>= 1;
+      while (group_smem(sm_slots, p.n_acc) > 47 * 1024) sm_slots >>= 1;
       p.sm_slots = sm_slots;
-      const size_t dyn = static_cast<size_t>(group_smem(kGroupThreads, p.use_smem ? sm_slots : 0, p.n_acc));
+      const size_t dyn = static_cast<size_t>(use_smem ? group_smem(sm_slots, p.n_acc) : 0);
       // 16 rows a thread amortise a CTA's table, but while that leaves SMs
       // without a CTA four rows do
       int64_t blocks = (n + kGroupThreads * 16 - 1) / (kGroupThreads * 16);
       blocks = std::max(blocks, std::min<int64_t>(num_sms(), (n + kGroupThreads * 4 - 1) / (kGroupThreads * 4)));
       // one wave: as many CTAs as fit on every SM at once
       int per_sm = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, group_update_kernel<kGroupThreads>, kGroupThreads,
-                                                        dyn) != cudaSuccess ||
-          per_sm < 1)
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kGroupThreads, dyn) != cudaSuccess || per_sm < 1)
         per_sm = 1;
       int64_t max_blocks = static_cast<int64_t>(num_sms()) * per_sm;
       if (blocks > max_blocks) blocks = max_blocks;
       if (blocks < 1) blocks = 1;
-      group_update_kernel<kGroupThreads><<<static_cast<int>(blocks), kGroupThreads, dyn, s>>>(p);
+      fn<<<static_cast<int>(blocks), kGroupThreads, dyn, s>>>(p);
     }
     after_launch("group_update_kernel");
     double w = 0;
