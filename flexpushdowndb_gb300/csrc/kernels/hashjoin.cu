@@ -17,8 +17,8 @@
 // occupy separate slots (multimap semantics). A build may test up to four
 // bloom filters on its key (a bloom selection folded into the join) and leave
 // out the rows that fail one. Probing: a warp
-// makes 64 lookups a step, two in flight per lane; rows whose group was full
-// wait on the warp's stack and go on 64 at a time. Matches collect per warp in
+// makes 32 lookups a step; rows whose group was full wait on the warp's stack
+// and go on 32 at a time. Matches collect per warp in
 // shared memory and leave in runs of up to kStage pairs, each run taking its
 // output positions with one atomic on the shared cursor: the cursor is a
 // single address whose atomics the L2 serialises, so one atomic per warp step
@@ -57,10 +57,28 @@ __device__ __forceinline__ uint64_t group_slot(const ulonglong2& lo, const ulong
 
 // One group, in one 32-byte load: lanes read groups at random, so a load
 // costs the L1 about a cycle a lane, and two 16-byte halves cost it twice.
+// kL1: kept in the L1, for tables of fewer than kSlotsInL1 slots (128 KB).
+// Lookups of a few hundred keys otherwise all meet at a few sectors of the L2
+// (500 keys: 20M rows 850 us, 280 through the L1; 2,000 keys 366 and 281),
+// while groups of a larger table would only push others out (10,000 keys 264
+// us, 277 through the L1; 5,000 keys the same both ways).
+constexpr uint64_t kSlotsInL1 = 16384;
+
+template <bool kL1>
 __device__ __forceinline__ void load_group(const uint64_t* slots, uint64_t grp, ulonglong2& lo, ulonglong2& hi) {
-  asm("ld.global.nc.L1::no_allocate.v4.u64 {%0, %1, %2, %3}, [%4];"
-      : "=l"(lo.x), "=l"(lo.y), "=l"(hi.x), "=l"(hi.y)
-      : "l"(slots + grp));
+  if (kL1)
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(lo.x), "=l"(lo.y), "=l"(hi.x), "=l"(hi.y)
+        : "l"(slots + grp));
+  else
+    asm("ld.global.nc.L1::no_allocate.v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(lo.x), "=l"(lo.y), "=l"(hi.x), "=l"(hi.y)
+        : "l"(slots + grp));
+}
+
+__device__ __forceinline__ void load_group(const uint64_t* slots, uint64_t grp, uint64_t mask, ulonglong2& lo, ulonglong2& hi) {
+  if (mask < kSlotsInL1) load_group<true>(slots, grp, lo, hi);
+  else load_group<false>(slots, grp, lo, hi);
 }
 
 // Bits of the group's slots that hold `tag`, and whether it has an empty slot
@@ -148,7 +166,7 @@ __global__ void __launch_bounds__(256)
 // memory, flushed to the output when fewer than 32 free places remain (one
 // staging round adds at most 32) and once at the end.
 constexpr int kProbeWarps = 8;  // 256-thread CTAs
-constexpr int kStage = 256;     // staged pairs per warp
+constexpr int kStage = 512;     // staged pairs per warp
 
 struct PairStage {
   int2* pair;  // (probe row, build row)
@@ -177,129 +195,108 @@ __device__ __forceinline__ int64_t load_key_stream(const DevCol& c, int64_t row)
 
 // The probe loop shared by the pair and the materialising probe.
 //
-// Each warp owns a contiguous range of probe rows and takes 64 lookups a
-// step, two per lane in flight: 64 new rows (their keys loaded a step ahead),
-// or, once 64 are waiting, rows whose group was full and whose run goes on.
-// Most rows are decided by their first group; the others wait on a stack with
-// the group to read next, so no lane idles behind another's longer run.
+// Each warp owns a contiguous range of probe rows and takes 32 lookups a
+// step: 32 new rows (their keys loaded a step ahead), or, once 32 are waiting,
+// rows whose group was full and whose run goes on. Most rows are decided by
+// their first group; the others wait on a stack with their key and the group
+// to read next, so no lane idles behind another's longer run.
 //
-// 20M rows against 2M keys, half of them matching, four columns out: 328 us
-// (374 us with one lookup per lane at a time and two 16-byte reads a group).
+// 20M rows against 2M keys, half of them matching, three columns out: 341 us
+// the call (400 us with a run walked slot by slot to its end by each lane).
 // Neither issue (50%) nor DRAM (20%) holds it: a request a lane from the L1
 // to the L2 for each lookup and each build value, at half that path's peak.
-constexpr int kProbeFlight = 2;  // lookups in flight per lane
-constexpr int kProbeStep = 32 * kProbeFlight;
-
-template <class Write>
+// Two lookups a lane in flight at 64 registers, waiting rows' keys read again
+// and 256 staged pairs took 352 us there, and with tables and columns past the
+// L2 much more, where DRAM's pages hold it and the stage's length is that of
+// the output's runs (16M int32 keys 885 us, 688 now; 8M int64 keys 896, 679).
+template <bool kL1, class Write>
 __device__ __forceinline__ void probe_rows(const DevCol& pkey, int64_t n, const uint64_t* __restrict__ slots,
                                            uint64_t mask, const DevCol& bkey, int key32, unsigned long long* cursor,
                                            Write& write) {
   __shared__ int2 s_pair[kProbeWarps][kStage];
-  __shared__ uint2 s_wait[kProbeWarps][2 * kProbeStep];  // (row, next group's first slot / 4: fewer than 2^34 slots)
+  __shared__ uint2 s_wait[kProbeWarps][64];  // (row, next group's first slot / 4: fewer than 2^34 slots)
+  __shared__ int64_t s_wait_key[kProbeWarps][64];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t below = (1u << lane) - 1u;
   PairStage sg{s_pair[warp], 0};
   int waiting = 0;  // the same in every lane
   const int64_t warp_global = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const int64_t per = ((n + n_warps - 1) / n_warps + kProbeStep - 1) / kProbeStep * kProbeStep;
+  const int64_t per = ((n + n_warps - 1) / n_warps + 31) / 32 * 32;
   int64_t base = warp_global * per < n ? warp_global * per : n;
   const int64_t end = base + per < n ? base + per : n;
 
-  int64_t ahead[kProbeFlight];  // keys of rows base + 32 * u + lane
-#pragma unroll
-  for (int u = 0; u < kProbeFlight; ++u)
-    ahead[u] = base + 32 * u + lane < end ? load_key_stream(pkey, base + 32 * u + lane) : 0;
+  int64_t ahead = base + lane < end ? load_key_stream(pkey, base + lane) : 0;  // the key of row base + lane
   while (base < end || waiting > 0) {
-    int32_t row[kProbeFlight];
-    int64_t key[kProbeFlight];
-    uint64_t grp[kProbeFlight];
-    uint32_t tag[kProbeFlight];
-    bool active[kProbeFlight];
-    const bool resume = waiting >= kProbeStep || base >= end;
+    int32_t row;
+    int64_t key;
+    uint64_t grp = 0;
+    bool active;
+    const bool resume = waiting >= 32 || base >= end;
     if (resume) {
-      const int take = waiting < kProbeStep ? waiting : kProbeStep;
+      const int take = waiting < 32 ? waiting : 32;
       waiting -= take;
-#pragma unroll
-      for (int u = 0; u < kProbeFlight; ++u) {
-        const int i = 32 * u + lane;
-        active[u] = i < take;
-        const uint2 w = active[u] ? s_wait[warp][waiting + i] : make_uint2(0, 0);
-        row[u] = static_cast<int32_t>(w.x);
-        grp[u] = static_cast<uint64_t>(w.y) << 2;
-        key[u] = active[u] ? load_int(pkey, row[u]) : 0;
-      }
+      active = lane < take;
+      const uint2 w = active ? s_wait[warp][waiting + lane] : make_uint2(0, 0);
+      row = static_cast<int32_t>(w.x);
+      grp = static_cast<uint64_t>(w.y) << 2;
+      key = active ? s_wait_key[warp][waiting + lane] : 0;
       __syncwarp();  // read before this step queues again
     } else {
-#pragma unroll
-      for (int u = 0; u < kProbeFlight; ++u) {
-        active[u] = base + 32 * u + lane < end;
-        row[u] = static_cast<int32_t>(base + 32 * u + lane);
-        key[u] = ahead[u];
-      }
-      base += kProbeStep;
-#pragma unroll
-      for (int u = 0; u < kProbeFlight; ++u)
-        if (base + 32 * u + lane < end) ahead[u] = load_key_stream(pkey, base + 32 * u + lane);
+      active = base + lane < end;
+      row = static_cast<int32_t>(base + lane);
+      key = ahead;
+      base += 32;
+      if (base + lane < end) ahead = load_key_stream(pkey, base + lane);
     }
-    uint64_t start[kProbeFlight];
-    ulonglong2 lo[kProbeFlight], hi[kProbeFlight];
-#pragma unroll
-    for (int u = 0; u < kProbeFlight; ++u) {
-      const uint64_t h = hash_key(key[u]);
-      tag[u] = key32 ? static_cast<uint32_t>(key[u]) : static_cast<uint32_t>(h >> 32);
-      start[u] = group_start(h, mask);
-      if (!resume) grp[u] = start[u];
-      if (active[u]) {
-        load_group(slots, grp[u], lo[u], hi[u]);
-      }
-    }
-    uint32_t mm[kProbeFlight];  // matching slots of the groups
-#pragma unroll
-    for (int u = 0; u < kProbeFlight; ++u) {
-      bool ends = true;
-      mm[u] = active[u] ? group_matches(lo[u], hi[u], tag[u], &ends) : 0u;
+    const uint64_t h = hash_key(key);
+    const uint32_t tag = key32 ? static_cast<uint32_t>(key) : static_cast<uint32_t>(h >> 32);
+    const uint64_t start = group_start(h, mask);
+    if (!resume) grp = start;
+    ulonglong2 lo, hi;
+    uint32_t mm = 0;  // matching slots of the group
+    bool ends = true;
+    if (active) {
+      load_group<kL1>(slots, grp, lo, hi);
+      mm = group_matches(lo, hi, tag, &ends);
       if (!key32) {
-        for (uint32_t t = mm[u]; t != 0; t &= t - 1) {
+        for (uint32_t t = mm; t != 0; t &= t - 1) {
           const int q = __ffs(static_cast<int>(t)) - 1;
-          if (load_int(bkey, static_cast<int32_t>(static_cast<uint32_t>(group_slot(lo[u], hi[u], q)))) != key[u])
-            mm[u] &= ~(1u << q);
+          if (load_int(bkey, static_cast<int32_t>(static_cast<uint32_t>(group_slot(lo, hi, q)))) != key)
+            mm &= ~(1u << q);
         }
       }
-      // A table always keeps empty slots (load factor <= 0.9), so every run
-      // ends; coming round to its start only guards the loop.
-      const uint64_t next = (grp[u] + 4) & mask;
-      const bool on = !ends && next != start[u];
-      const uint32_t cont = __ballot_sync(0xffffffffu, on);
-      if (on) {
-        const int at = waiting + __popc(cont & below);  // fewer than kProbeStep waited, at most as many join
-        s_wait[warp][at] = make_uint2(static_cast<uint32_t>(row[u]), static_cast<uint32_t>(next >> 2));
-      }
-      waiting += __popc(cont);
     }
+    // A table always keeps empty slots (load factor <= 0.9), so every run
+    // ends; coming round to its start only guards the loop.
+    const uint64_t next = (grp + 4) & mask;
+    const bool on = !ends && next != start;
+    const uint32_t cont = __ballot_sync(0xffffffffu, on);
+    if (on) {
+      const int at = waiting + __popc(cont & below);  // fewer than 32 waited, at most 32 join
+      s_wait[warp][at] = make_uint2(static_cast<uint32_t>(row), static_cast<uint32_t>(next >> 2));
+      s_wait_key[warp][at] = key;
+    }
+    waiting += __popc(cont);
     // One match per lookup and round (a group can hold several copies of a
     // repeated build key).
-    bool more;
-    do {
-      if (sg.n > kStage - kProbeStep) flush_pairs(sg, cursor, lane, write);
-      more = false;
-#pragma unroll
-      for (int u = 0; u < kProbeFlight; ++u) {
-        const uint32_t em = __ballot_sync(0xffffffffu, mm[u] != 0);
-        if (mm[u] != 0) {
-          const uint64_t v = group_slot(lo[u], hi[u], __ffs(static_cast<int>(mm[u])) - 1);
-          s_pair[warp][sg.n + __popc(em & below)] = make_int2(row[u], static_cast<int32_t>(static_cast<uint32_t>(v)));
-          mm[u] &= mm[u] - 1;
-          more = more || mm[u] != 0;
-        }
-        sg.n += __popc(em);
+    uint32_t em = __ballot_sync(0xffffffffu, mm != 0);
+    while (em != 0) {
+      if (sg.n > kStage - 32) flush_pairs(sg, cursor, lane, write);
+      if (mm != 0) {
+        const uint64_t v = group_slot(lo, hi, __ffs(static_cast<int>(mm)) - 1);
+        s_pair[warp][sg.n + __popc(em & below)] = make_int2(row, static_cast<int32_t>(static_cast<uint32_t>(v)));
+        mm &= mm - 1;
       }
-    } while (__any_sync(0xffffffffu, more));
+      sg.n += __popc(em);
+      em = __ballot_sync(0xffffffffu, mm != 0);
+    }
     __syncwarp();  // what this step queued is seen by every lane
   }
   if (sg.n > 0) flush_pairs(sg, cursor, lane, write);
 }
 
+template <bool kL1>
 __global__ void __launch_bounds__(256)
     join_probe_kernel(DevCol pkey, int64_t n_cap, const int64_t* n_dev, const uint64_t* __restrict__ slots,
                       uint64_t mask, DevCol bkey, int key32, int32_t* __restrict__ out_p,
@@ -312,7 +309,7 @@ __global__ void __launch_bounds__(256)
         __stcs(out_b + at + i, sg.pair[i].y);
       }
   };
-  probe_rows(pkey, n, slots, mask, bkey, key32, reinterpret_cast<unsigned long long*>(&st->value), write);
+  probe_rows<kL1>(pkey, n, slots, mask, bkey, key32, reinterpret_cast<unsigned long long*>(&st->value), write);
 }
 
 // Probe and materialise in one pass: every staged match becomes an output
@@ -365,6 +362,7 @@ __device__ __forceinline__ void copy_staged(const T* __restrict__ src, T* __rest
   }
 }
 
+template <bool kL1>
 __global__ void __launch_bounds__(256, 4) join_probe_emit_kernel(const __grid_constant__ JoinEmitParams p) {
   const int64_t n = clamp_rows(p.n_dev, p.n_cap);
   auto write = [&](int64_t at, const PairStage& sg, int lane) {
@@ -380,7 +378,7 @@ __global__ void __launch_bounds__(256, 4) join_probe_emit_kernel(const __grid_co
                        stream_src);
     }
   };
-  probe_rows(p.pkey, n, p.slots, p.mask, p.bkey, p.key32, reinterpret_cast<unsigned long long*>(&p.st->value), write);
+  probe_rows<kL1>(p.pkey, n, p.slots, p.mask, p.bkey, p.key32, reinterpret_cast<unsigned long long*>(&p.st->value), write);
 }
 
 // A chain of joins in one pass. Each lane walks its input row through the
@@ -489,7 +487,7 @@ __global__ void __launch_bounds__(256) join_chain_kernel(const __grid_constant__
           const int q0 = static_cast<int>(s0 & 3);
           const uint64_t g = s0 & ~3ull;
           ulonglong2 lo, hi;
-          load_group(L.slots, g, lo, hi);
+          load_group(L.slots, g, L.mask, lo, hi);
           uint32_t eb = 0, tb = 0;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -595,14 +593,14 @@ int grid_for(int64_t n, int per_sm = 4, int64_t rows_per_block = 256) {
 
 // The probes' warps wait on table loads, so their grids fill every SM with
 // as many CTAs as fit at once (one wave, no tail).
-template <class Kernel>
-int probe_grid(Kernel kernel, int64_t n) {
-  static const int per_sm = [kernel] {
+template <auto Kernel>
+int probe_grid(int64_t n) {
+  static const int per_sm = [] {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 256, 0) != cudaSuccess || b < 1) b = 4;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, Kernel, 256, 0) != cudaSuccess || b < 1) b = 4;
     return b;
   }();
-  return grid_for(n, per_sm, kProbeWarps * 2 * kProbeStep);
+  return grid_for(n, per_sm, kProbeWarps * 64);  // at least 64 rows per warp
 }
 
 }  // namespace
@@ -700,7 +698,10 @@ std::vector<ColumnPtr> join_probe_materialize(const JoinTable& t, const TupleSet
     if (attempt > 0) GF_CUDA(cudaMemsetAsync(status->data(), 0, sizeof(DevStatus), s));
     if (n > 0 && t.build->num_rows() > 0) {
       ProfScope prof("join_probe_emit_kernel", s);
-      join_probe_emit_kernel<<<probe_grid(join_probe_emit_kernel, n), 256, 0, s>>>(p);
+      if (p.mask < kSlotsInL1)
+        join_probe_emit_kernel<true><<<probe_grid<join_probe_emit_kernel<true>>(n), 256, 0, s>>>(p);
+      else
+        join_probe_emit_kernel<false><<<probe_grid<join_probe_emit_kernel<false>>(n), 256, 0, s>>>(p);
       after_launch("join_probe_emit_kernel");
       prof.stop(0);
       double w_out = 0;
@@ -852,9 +853,11 @@ void join_probe_pairs(const JoinTable& t, const TupleSet& probe, int probe_key, 
     if (attempt > 0) GF_CUDA(cudaMemsetAsync(status->data(), 0, sizeof(DevStatus), s));
     if (n > 0 && t.build->num_rows() > 0) {
       ProfScope prof("join_probe_kernel", s);
-      join_probe_kernel<<<probe_grid(join_probe_kernel, n), 256, 0, s>>>(pk, n, probe.rows_dev(), t.slots->as<uint64_t>(),
-                                                   t.capacity - 1, bkc, key32 ? 1 : 0, (*probe_idx)->as<int32_t>(),
-                                                   (*build_idx)->as<int32_t>(), cap, status->as<DevStatus>());
+      const bool l1 = t.capacity <= kSlotsInL1;
+      (l1 ? join_probe_kernel<true> : join_probe_kernel<false>)<<<
+          l1 ? probe_grid<join_probe_kernel<true>>(n) : probe_grid<join_probe_kernel<false>>(n), 256, 0, s>>>(
+          pk, n, probe.rows_dev(), t.slots->as<uint64_t>(), t.capacity - 1, bkc, key32 ? 1 : 0,
+          (*probe_idx)->as<int32_t>(), (*build_idx)->as<int32_t>(), cap, status->as<DevStatus>());
       after_launch("join_probe_kernel");
       prof.stop(static_cast<double>(n) * dtype_width(pc->type));
       prof.set_bytes_model(probe.rows_dev(), n, dtype_width(pc->type), &status->as<DevStatus>()->value, 8.0, status,
@@ -920,7 +923,7 @@ __device__ __forceinline__ int walk_matches(const MatchParams& p, int64_t r, F&&
   bool ends = false;
   for (uint64_t i = 0; i <= p.mask && !ends; i += 4, grp = (grp + 4) & p.mask) {
     ulonglong2 lo, hi;
-    load_group(p.slots, grp, lo, hi);
+    load_group(p.slots, grp, p.mask, lo, hi);
     for (uint32_t t = group_matches(lo, hi, tag, &ends); t != 0; t &= t - 1) {
       const uint32_t b = static_cast<uint32_t>(group_slot(lo, hi, __ffs(static_cast<int>(t)) - 1));
       if (!p.key32 && load_int(p.bkey, b) != k) continue;
