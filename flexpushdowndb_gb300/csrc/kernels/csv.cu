@@ -690,21 +690,30 @@ __global__ void __launch_bounds__(kCsvThreads, 5) csv_fields_kernel(const __grid
     }
 }
 
-// (3) utf8 offsets and bytes. A warp takes a column of the tile, 32 rows at a
-// time: their lengths, a warp scan for the offsets, then each lane copies its
-// string into the warp's buffer in shared memory (words between a head and a
-// tail of at most three bytes), laid out as the output's 16-byte lines, and
-// the warp writes the buffer out in whole 16-byte stores with byte stores at
-// its two ends. Groups of strings too long for the buffer go out string by
-// string.
+// (3) utf8 offsets and bytes. A warp takes a column of the tile, or with up to
+// four columns a run of a column's rows (csv_share of them a column: a single
+// column by one warp of the eight took 372 us the call for 3M strings of 20
+// bytes, 221 with all eight), 32 rows at a time: their lengths, a warp scan for
+// the offsets, then each lane copies its string into the warp's buffer in
+// shared memory (words between a head and a tail of at most three bytes), laid
+// out as the output's 16-byte lines, and the warp writes the buffer out in
+// whole 16-byte stores with byte stores at its two ends. Groups of strings too
+// long for the buffer go out a word of the output per lane, whichever rows its
+// bytes are of (1.4M strings of 60 bytes: 251 us the call, 537 string by string
+// with a byte per lane and one warp).
 constexpr int kCsvStage = 1536;                            // bytes of a warp's buffer besides its alignment
 constexpr int kCsvOutLines = (kCsvStage + 32) / 16;        // 16-byte lines of a warp's buffer
+constexpr int csv_share(int columns) { return columns >= 1 && columns <= kCsvWarps / 2 ? kCsvWarps / columns : 1; }
 constexpr int csv_strings_smem(int columns) {
-  return (kCsvTextLines + (columns < kCsvWarps ? columns : kCsvWarps) * kCsvOutLines) * 16;
+  const int warps = columns * csv_share(columns);
+  return (kCsvTextLines + (warps < kCsvWarps ? warps : kCsvWarps) * kCsvOutLines) * 16;
 }
 
+// kRuns: warps share a column's rows.
+template <bool kRuns>
 __global__ void __launch_bounds__(kCsvThreads, 5) csv_strings_kernel(const __grid_constant__ CsvParams p) {
   extern __shared__ uint4 s_mem[];
+  __shared__ int32_t s_run[kCsvWarps];  // bytes of each warp's run of rows
   uint4* const s_text = s_mem;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // where this tile's separators begin and the next one's (the last tile's
@@ -719,7 +728,11 @@ __global__ void __launch_bounds__(kCsvThreads, 5) csv_strings_kernel(const __gri
   uint32_t* const ow = reinterpret_cast<uint32_t*>(s_out);
   uint16_t* const oh = reinterpret_cast<uint16_t*>(s_out);
   uint8_t* const ob = reinterpret_cast<uint8_t*>(s_out);
-  for (int u = warp; u < p.n_utf8; u += kCsvWarps) {
+  const int share = kRuns ? csv_share(p.n_utf8) : 1;
+  auto length = [&](uint32_t span) {
+    return (span & 0xFFFFu) == kCsvFar ? static_cast<int32_t>(p.far[2 * blockIdx.x + 1]) : static_cast<int32_t>(span >> 16);
+  };
+  for (int u = warp / share; u < p.n_utf8; u += kCsvWarps / share) {
     const CsvOut& o = p.out[p.utf8_out[u]];
     // the column's data rows whose separator lies in the tile
     int64_t row0 = (begin >> 8) + (o.field < (begin & 255) ? 1 : 0) - p.header;
@@ -728,6 +741,19 @@ __global__ void __launch_bounds__(kCsvThreads, 5) csv_strings_kernel(const __gri
     if (row1 > p.n_rows) row1 = p.n_rows;
     uint8_t* const out = static_cast<uint8_t*>(o.data);
     const uint32_t* const spans = p.spans + u * p.n_rows;
+    const int part = kRuns ? warp % share : 0;
+    if (kRuns && row1 > row0) {  // this warp's run of them
+      const int64_t run = (row1 - row0 + share - 1) / share;
+      row0 = row0 + part * run < row1 ? row0 + part * run : row1;
+      row1 = row0 + run < row1 ? row0 + run : row1;
+      int32_t bytes = 0;  // a column holds less than 2^31 bytes (checked before the launch)
+#pragma unroll 4
+      for (int64_t r = row0 + lane; r < row1; r += 32) bytes += length(__ldg(spans + r));
+      bytes = __reduce_add_sync(0xffffffffu, bytes);
+      if (lane == 0) s_run[warp] = bytes;
+    } else if (kRuns && lane == 0) {
+      s_run[warp] = 0;
+    }
     // a column's spans are loaded a group ahead of their use
     uint32_t ahead = row0 + lane < row1 ? __ldg(spans + row0 + lane) : 0u;
     int32_t base = static_cast<int32_t>(
@@ -736,14 +762,16 @@ __global__ void __launch_bounds__(kCsvThreads, 5) csv_strings_kernel(const __gri
       __syncthreads();
       staged = true;
     }
+    if (kRuns)
+      for (int w = warp - part; w < warp; ++w) base += s_run[w];
     for (int64_t r = row0 + lane; r - lane < row1; r += 32) {
       const bool have = r < row1;
       const uint32_t span = ahead;
       ahead = r + 32 < row1 ? __ldg(spans + r + 32) : 0u;
       const bool far = have && (span & 0xFFFFu) == kCsvFar;
       const int b = static_cast<int>(span & 0xFFFFu);
-      const int32_t len = far ? static_cast<int32_t>(p.far[2 * blockIdx.x + 1]) : static_cast<int32_t>(span >> 16);
-      int32_t incl = len;  // a column holds less than 2^31 bytes (checked before the launch)
+      const int32_t len = length(span);
+      int32_t incl = len;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const int32_t y = __shfl_up_sync(0xffffffffu, incl, d);
@@ -804,12 +832,63 @@ __global__ void __launch_bounds__(kCsvThreads, 5) csv_strings_kernel(const __gri
         }
         __syncwarp();  // the buffer is rewritten by the next group
       } else {
-        for (int l = 0; l < 32; ++l) {
-          const int32_t n = __shfl_sync(0xffffffffu, len, l), to = __shfl_sync(0xffffffffu, at, l);
-          const int from = __shfl_sync(0xffffffffu, b, l);
-          const uint8_t* src = from != static_cast<int>(kCsvFar) ? t + from : p.text + p.far[2 * blockIdx.x];
-          for (int32_t x = lane; x < n; x += 32) out[static_cast<int64_t>(to) + x] = src[x];
+        // word by word of the output: where each row's bytes begin in it, and
+        // what its text lies at from there, in the warp's buffer
+        int32_t* const off = reinterpret_cast<int32_t*>(s_out);
+        int32_t* const from = off + 33;
+        off[lane + 1] = at + len;
+        if (lane == 0) off[0] = base;
+        from[lane] = b - at;  // a far row's bytes are read from the text itself
+        const int far_row = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, far))) - 1;  // one at most
+        const uint8_t* const far_text = far_row >= 0 ? p.text + p.far[2 * blockIdx.x] : nullptr;
+        __syncwarp();
+        const int32_t far_at = far_row >= 0 ? off[far_row] : 0;
+        const int32_t end = base + total;
+        auto byte = [&](int row, int32_t q) { return row == far_row ? far_text[q - far_at] : t[from[row] + q]; };
+        const int32_t w0 = (base + 3) >> 2, w1 = end >> 2;  // whole words [w0, w1)
+        {  // the bytes before and after them, three at most each
+          const int32_t head = 4 * w0 < end ? 4 * w0 : end, tail = 4 * w1 > head ? 4 * w1 : head;
+          const int32_t q = lane < 4 ? base + lane : tail + lane - 4;
+          if (lane < 4 ? q < head : lane < 8 && q < end) {
+            int row = lane < 4 ? 0 : static_cast<int>(row1 - (r - lane) < 32 ? row1 - (r - lane) : 32) - 1;
+            while (off[row + 1] <= q) ++row;
+            while (off[row] > q) --row;
+            out[q] = byte(row, q);
+          }
         }
+        int row = 0;
+        int32_t row_end = off[1], place = from[0];
+        for (int32_t w = w0 + lane; w < w1; w += 32) {
+          const int32_t q = 4 * w;
+          if (q >= row_end) {
+            do ++row;
+            while (off[row + 1] <= q);  // q < end
+            row_end = off[row + 1];
+            place = from[row];
+          }
+          uint32_t x;
+          const bool one = q + 4 <= row_end;
+          if (row != far_row && (one || off[row + 2] >= q + 4)) {
+            x = text_word(s, place + q);
+            if (!one) {  // its last bytes are the next row's first ones
+              const uint32_t next = ~0u << (8 * (row_end - q));
+              x = (x & ~next) | (text_word(s, from[row + 1] + q) & next);
+            }
+          } else if (one) {
+            const uint8_t* const f = far_text + (q - far_at);
+            x = f[0] | f[1] << 8 | f[2] << 16 | static_cast<uint32_t>(f[3]) << 24;
+          } else {
+            x = 0;
+            int at_row = row;
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+              while (off[at_row + 1] <= q + k) ++at_row;
+              x |= static_cast<uint32_t>(byte(at_row, q + k)) << (8 * k);
+            }
+          }
+          reinterpret_cast<uint32_t*>(out)[w] = x;
+        }
+        __syncwarp();  // the buffer is rewritten by the next group
       }
       base += total;
     }
@@ -827,7 +906,8 @@ TupleSetPtr csv_parse(const char* device_text, int64_t n_bytes, char delimiter, 
   if (n_bytes >= (int64_t{1} << 40)) fail(GFPDB_EUNSUPPORTED, "CSV text too large");
   const uint8_t* text = reinterpret_cast<const uint8_t*>(device_text);
   allow_shared(csv_fields_kernel, csv_fields_smem(1));  // the most
-  allow_shared(csv_strings_kernel, csv_strings_smem(kCsvWarps));
+  allow_shared(csv_strings_kernel<true>, csv_strings_smem(kCsvWarps));  // the most
+  allow_shared(csv_strings_kernel<false>, csv_strings_smem(kCsvWarps));
   if ((reinterpret_cast<uintptr_t>(text) & 15u) != 0) fail(GFPDB_EINVAL, "CSV text must be 16-byte aligned");
 
   if (static_cast<int>(fields.size()) > kCsvMaxFields) fail(GFPDB_EUNSUPPORTED, "too many CSV fields per line");
@@ -970,7 +1050,8 @@ TupleSetPtr csv_parse(const char* device_text, int64_t n_bytes, char delimiter, 
   }
   if (n_rows > 0 && !utf8.empty()) {
     ProfScope prof("csv_strings_kernel", s);
-    csv_strings_kernel<<<static_cast<int>(n_tiles), kCsvThreads, csv_strings_smem(n_utf8), s>>>(p);
+    const auto strings = csv_share(n_utf8) > 1 ? csv_strings_kernel<true> : csv_strings_kernel<false>;
+    strings<<<static_cast<int>(n_tiles), kCsvThreads, csv_strings_smem(n_utf8), s>>>(p);
     after_launch("csv_strings_kernel");
     prof.stop(static_cast<double>(n_bytes) + string_bytes + 4.0 * static_cast<double>(n_rows) * n_utf8);
   }
