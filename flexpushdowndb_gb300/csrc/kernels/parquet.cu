@@ -15,8 +15,11 @@
 //                          4-byte offset) and the warp moves its bytes, 32 at
 //                          a time (copies whose source overlaps their output
 //                          go in steps of the offset);
-//   parquet_pages_kernel   one CTA per 8,192 values of a page: thread 0 skips
-//                          (and checks) the definition levels, walks
+//   parquet_runs_kernel    one warp per page of more than 8,192 dictionary
+//                          indices in several runs: skips (and checks) its
+//                          definition levels and finds the run that each
+//                          8,192nd index lies in;
+//   parquet_pages_kernel   one CTA per 8,192 values of a page: thread 0 walks
 //                          byte-array lengths (data and dictionary pages) and
 //                          reads the dictionary indices' run headers, up to
 //                          256 a round, and every thread then decodes the
@@ -42,7 +45,7 @@ namespace {
 struct PageDev {
   const uint8_t* body;    // page body on the device (after its header)
   uint8_t* inflated;      // snappy pages: the decompressed body (v2: the values part)
-  const uint8_t* values;  // set by parquet_pages_kernel: the first value byte
+  const uint8_t* values;  // set by parquet_runs_kernel or parquet_pages_kernel: the first value byte
   int32_t body_len;
   int32_t inflated_len;
   int32_t values_len;     // set with `values`
@@ -54,7 +57,11 @@ struct PageDev {
   int32_t v1_def;         // data page v1 of an optional column
   int32_t width;          // fixed-width bytes, 0 for byte arrays
   int32_t dict_page;      // data pages: their dictionary page's index, -1
-  int32_t pad;
+  int32_t n_parts;
+  int32_t walked;         // 1: parquet_runs_kernel has set values and the parts' runs
+  int32_t first_part;     // its first part in the read's list
+  int32_t late_from;      // the parts from this value on are decoded in the read's second round (kPqNever: none)
+  int32_t walk_at, walk_done;  // where the walk over the runs stopped: a header's place, the values before it
   int64_t first_row;
   int64_t dict_base;      // byte-array dictionary pages: first entry in dict_ptr / dict_len
   int32_t* idx;           // dictionary-encoded columns: per-row entry
@@ -213,18 +220,230 @@ constexpr int kPqRuns = 256;  // run headers read per round
 // copy per span of chunks the whole read of that file went from 1,118 to 680 us
 // (653 with copying and decoding overlapped, see kPqBatch).
 constexpr int kPqPart = 8192;
+constexpr int32_t kPqNever = INT32_MAX;
 
 struct PagePart {
   int32_t page;
-  int32_t first;  // the part's first value in the page
+  int32_t first;     // the part's first value in the page
+  int32_t at, done;  // the run it lies in: the header's place among the page's values, the values before the run
 };
+
+// The page's values, behind its levels. With definition levels, false (and an
+// error) where one says null or they are malformed. One thread.
+__device__ bool page_values(const PageDev& pg, int32_t w, DevStatus* st, const uint8_t** values, int32_t* values_len) {
+  const uint8_t* base;
+  int32_t blen;
+  if (pg.snappy) {
+    base = pg.inflated;
+    blen = pg.inflated_len;
+  } else {
+    const int32_t skip = pg.type == parquet::PAGE_DATA_V2 ? pg.v2_levels : 0;
+    base = pg.body + skip;
+    blen = pg.body_len - skip;
+  }
+  int ok = 1;
+  if (pg.v1_def) {  // 4-byte length, then the levels: every one must be 1 (no nulls)
+    ok = 0;
+    if (blen >= 4) {
+      const int32_t len = static_cast<int32_t>(le32(base));
+      if (len >= 0 && len <= blen - 4) {
+        const uint8_t* lv = base + 4;
+        int32_t at = 0, seen = 0;
+        ok = 1;
+        while (seen < pg.num_values && ok) {
+          uint32_t h;
+          if (!run_header(lv, len, &at, &h)) {
+            ok = 0;
+            break;
+          }
+          if (h & 1) {  // bit-packed: (h >> 1) groups of 8 one-bit levels
+            const int32_t bytes = static_cast<int32_t>(h >> 1);
+            if (bytes > len - at) {
+              ok = 0;
+              break;
+            }
+            for (int32_t b = 0; b < bytes && ok; ++b) {
+              const int32_t valid = pg.num_values - seen - 8 * b;
+              const uint32_t need = valid >= 8 ? 0xffu : ((1u << (valid > 0 ? valid : 0)) - 1u);
+              if ((lv[at + b] & need) != need) ok = 0;  // a 0 level: a null
+            }
+            at += bytes;
+            seen += 8 * bytes;
+          } else {  // RLE: (h >> 1) copies of a one-byte level
+            if (at >= len || lv[at] != 1) {
+              ok = 0;
+              break;
+            }
+            ++at;
+            seen += static_cast<int32_t>(h >> 1);
+          }
+        }
+        base += 4 + len;
+        blen -= 4 + len;
+      }
+    }
+    if (!ok) raise_status(st, GFPDB_EUNSUPPORTED, 200000 + w);  // nulls, or bad levels
+  }
+  *values = base;
+  *values_len = blen;
+  return ok != 0;
+}
+
+// One warp per page of several parts and runs: where each part's first run
+// begins, so that no part walks the headers of the ones before it (they did,
+// and 16M rows of four columns in 1M-value pages of 504-value runs, as Arrow
+// writes them, took 8.4 ms, of 8-value runs 211 ms; 6.4 and 35 with a CTA per
+// page). A header's place follows from the one before. The page goes through
+// shared memory kPqWindow bytes at a time, so that short runs cost no memory
+// round trip each, and runs of one length, the usual case, are taken up to 32 a
+// step: each lane looks for the same header where it would be.
+//
+// Batches are decoded one after the other, so a page of many runs that all
+// differ would hold up the ones behind it, each in turn: after `steps` steps
+// the walk stops, and the page's remaining parts wait for the read's second
+// round, in which the walks of all its pages go on together.
+constexpr int kPqWindow = 1024;
+constexpr int kPqWalkThreads = 128;
+
+__global__ void __launch_bounds__(kPqWalkThreads) parquet_runs_kernel(PageDev* pages, const int32_t* list, int32_t n,
+                                                                      PagePart* parts, int32_t steps, int32_t late,
+                                                                      DevStatus* st) {
+  __shared__ uint4 s_window[kPqWalkThreads / 32][kPqWindow / 16];
+  const int lane = threadIdx.x & 31;
+  uint4* const window = s_window[threadIdx.x >> 5];
+  const uint8_t* const bytes = reinterpret_cast<const uint8_t*>(window);
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t item = warp; item < n; item += warps) {
+    const int32_t w = list[item];
+    PageDev& pg = pages[w];
+    const int32_t num_values = pg.num_values, n_parts = pg.n_parts;
+    PagePart* const part = parts + pg.first_part;
+    int32_t at = 1, done = 0;
+    if (late) {
+      if (pg.late_from == kPqNever) continue;
+      at = pg.walk_at;
+      done = pg.walk_done;
+    } else {
+      if (lane == 0) {
+        const uint8_t* values = nullptr;
+        int32_t len = 0;
+        const bool ok = page_values(pg, w, st, &values, &len);
+        pg.values = ok ? values : nullptr;
+        pg.values_len = ok ? len : 0;
+      }
+      __syncwarp();
+    }
+    const uint8_t* const base = pg.values;
+    const int32_t blen = pg.values_len;
+    const int bw = blen > 0 ? base[0] : 99;
+    if (bw > 32) continue;  // the parts report it
+    int32_t next = done > kPqPart ? (done + kPqPart - 1) / kPqPart : 1;  // the first part that is not found yet
+    int64_t from = 0, to = 0;  // the window: bytes [from, to) of the values, all of them real ones
+    int pad = 0;               // bytes of the window before `from`
+    for (int32_t step = 0; next < n_parts; ++step) {
+      if (step == steps) {
+        if (lane == 0) {
+          pg.late_from = next * kPqPart;
+          pg.walk_at = at;
+          pg.walk_done = done;
+          st->aux[0] = 1;
+        }
+        break;
+      }
+      if (at + 5 > to && to < blen) {  // a header is 5 bytes at most
+        // whole 16-byte lines (the buffers start on one, and end 16 bytes
+        // after the last page)
+        __syncwarp();
+        const uintptr_t first = reinterpret_cast<uintptr_t>(base + at) & ~uintptr_t{15};
+        pad = static_cast<int>(reinterpret_cast<uintptr_t>(base + at) - first);
+        from = at;
+        to = at + kPqWindow - pad;
+        if (to > blen) to = blen;
+#pragma unroll
+        for (int k = 0; k < kPqWindow / 16 / 32; ++k) {
+          const uintptr_t line = first + 16 * static_cast<uintptr_t>(lane + 32 * k);
+          if (line < reinterpret_cast<uintptr_t>(base + blen)) window[lane + 32 * k] = __ldg(reinterpret_cast<const uint4*>(line));
+        }
+        __syncwarp();
+      }
+      // runs that all differ, with one-byte headers: one after the other
+      const int shift = pad - static_cast<int>(from);  // window byte of value byte 0
+      if (at < to) {
+        uint32_t h = bytes[at + shift];
+        for (; step != steps; ++step) {
+          const int32_t count = h & 1 ? static_cast<int32_t>(h >> 1) * 8 : static_cast<int32_t>(h >> 1);
+          const int32_t after = at + 1 + (h & 1 ? static_cast<int32_t>(h >> 1) * bw : (bw + 7) / 8);
+          if (h >= 0x80 || count == 0 || after + 5 > to) break;
+          const uint32_t h2 = bytes[after + shift];
+          if (h2 == h) break;
+          if (count > num_values - done) break;
+          done += count;
+          for (; next < n_parts && next * kPqPart < done; ++next)
+            if (lane == 0) {
+              part[next].at = at;
+              part[next].done = done - count;
+            }
+          at = after;
+          h = h2;
+        }
+        if (next >= n_parts) break;
+        if (step == steps) {
+          --step;  // the loop's head sees it again
+          continue;
+        }
+      }
+      const uint8_t* const here = bytes + at + shift;
+      int32_t head = 0;
+      uint32_t h = 0;
+      bool good = run_header(here, static_cast<int32_t>(to - at), &head, &h);
+      const int64_t body = h & 1 ? static_cast<int64_t>(h >> 1) * bw : (bw + 7) / 8;
+      const int64_t count = h & 1 ? static_cast<int64_t>(h >> 1) * 8 : h >> 1;
+      good = good && count > 0 && body <= blen - at - head;
+      if (!good) {  // the parts from here on meet it and report it
+        for (int32_t p = next + lane; p < n_parts; p += 32) {
+          part[p].at = at;
+          part[p].done = done;
+        }
+        break;
+      }
+      // the same header where this lane's run would be: in the window first,
+      // beyond it only if no lane's run there differs
+      const int64_t stride = head + body;
+      const int64_t mine = at + lane * stride, before = done + lane * count;
+      const bool fits = mine + stride <= blen, near = mine + head <= to;
+      auto same = [&](const uint8_t* there) {
+        for (int b = 0; b < head; ++b)
+          if (there[b] != here[b]) return false;
+        return true;
+      };
+      const int in_window = __popc(__ballot_sync(0xffffffffu, near));
+      uint32_t differs = __ballot_sync(0xffffffffu, !fits || (near && !same(bytes + mine + shift)));
+      if (differs == 0 || __ffs(static_cast<int>(differs)) - 1 >= in_window)
+        differs |= __ballot_sync(0xffffffffu, fits && !near && !same(base + mine));
+      const int runs = differs != 0 ? __ffs(static_cast<int>(differs)) - 1 : 32;  // 1 at least
+      if (lane < runs) {
+        int64_t p = (before + kPqPart - 1) / kPqPart;
+        for (p = p < 1 ? 1 : p; p < n_parts && p * kPqPart < before + count; ++p) {
+          part[p].at = static_cast<int32_t>(mine);
+          part[p].done = static_cast<int32_t>(before);
+        }
+      }
+      const int64_t reached = done + runs * count;
+      if (reached >= num_values) break;
+      at += static_cast<int32_t>(runs * stride);
+      done = static_cast<int32_t>(reached);
+      next = done > kPqPart ? (done + kPqPart - 1) / kPqPart : 1;
+    }
+  }
+}
 
 // One CTA per part of a page: kPqPart consecutive values where the page
 // holds dictionary indices, the whole of any other page. Thread 0
-// does the sequential parts (definition levels, byte-array lengths, run
-// headers, which every part of a page walks for itself up to its own end);
-// the dictionary indices of each round of up to kPqRuns runs that lie in the
-// part are then decoded by every thread, a value finding its run by binary
+// does the sequential parts (byte-array lengths, and the run headers from the
+// part's first run, or its page's, to its end; pages that are not walked have
+// their levels skipped here too); the dictionary indices of each round of up to kPqRuns runs that lie in
+// the part are then decoded by every thread, a value finding its run by binary
 // search over the runs' first values. A fixed-width column's
 // index is looked up in its dictionary page at once and the value written
 // to the output column (the dictionary page's body is read as the host laid
@@ -233,80 +452,40 @@ struct PagePart {
 // dictionary pages' entries are known.
 __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* pages, int32_t n_pages,
                                                                    const PagePart* __restrict__ items, int64_t n_items,
-                                                                   DictArrays dicts, DevStatus* st) {
+                                                                   int32_t late, DictArrays dicts, DevStatus* st) {
   __shared__ int32_t s_first[kPqRuns + 1];  // the page value index each run starts at; then the round's end
   __shared__ int32_t s_start[kPqRuns];      // bit-packed runs: first byte; RLE runs: -1
   __shared__ uint32_t s_value[kPqRuns];     // RLE runs: the value
   __shared__ int32_t s_n, s_ok, s_at, s_done, s_bw, s_blen;
   __shared__ const uint8_t* s_base;
+  __shared__ uint4 s_window[kPqWindow / 16];
   for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
     __syncthreads();  // the previous part's shared state is no longer read
-    const int32_t w = items[item].page;
+    const PagePart part = items[item];
+    const int32_t w = part.page;
     PageDev& pg = pages[w];
-    const int32_t part_lo = items[item].first;
+    const int32_t part_lo = part.first;
+    if ((part_lo >= pg.late_from) != (late != 0)) continue;  // the read's other round decodes it
     const int32_t num_values = pg.num_values;
     const int32_t part_hi = num_values - part_lo < kPqPart ? num_values : part_lo + kPqPart;
     const uint8_t* base;
     int32_t blen;
-    if (pg.snappy) {
-      base = pg.inflated;
-      blen = pg.inflated_len;
-    } else {
-      const int32_t skip = pg.type == parquet::PAGE_DATA_V2 ? pg.v2_levels : 0;
-      base = pg.body + skip;
-      blen = pg.body_len - skip;
-    }
     if (threadIdx.x == 0) {
       int ok = 1;
-      if (pg.v1_def) {  // 4-byte length, then the levels: every one must be 1 (no nulls)
-        ok = 0;
-        if (blen >= 4) {
-          const int32_t len = static_cast<int32_t>(le32(base));
-          if (len >= 0 && len <= blen - 4) {
-            const uint8_t* lv = base + 4;
-            int32_t at = 0, seen = 0;
-            ok = 1;
-            while (seen < pg.num_values && ok) {
-              uint32_t h;
-              if (!run_header(lv, len, &at, &h)) {
-                ok = 0;
-                break;
-              }
-              if (h & 1) {  // bit-packed: (h >> 1) groups of 8 one-bit levels
-                const int32_t bytes = static_cast<int32_t>(h >> 1);
-                if (bytes > len - at) {
-                  ok = 0;
-                  break;
-                }
-                for (int32_t b = 0; b < bytes && ok; ++b) {
-                  const int32_t valid = pg.num_values - seen - 8 * b;
-                  const uint32_t need = valid >= 8 ? 0xffu : ((1u << (valid > 0 ? valid : 0)) - 1u);
-                  if ((lv[at + b] & need) != need) ok = 0;  // a 0 level: a null
-                }
-                at += bytes;
-                seen += 8 * bytes;
-              } else {  // RLE: (h >> 1) copies of a one-byte level
-                if (at >= len || lv[at] != 1) {
-                  ok = 0;
-                  break;
-                }
-                ++at;
-                seen += static_cast<int32_t>(h >> 1);
-              }
-            }
-            base += 4 + len;
-            blen -= 4 + len;
-          }
+      if (pg.walked) {
+        base = pg.values;
+        blen = pg.values_len;
+        ok = base != nullptr;  // else parquet_runs_kernel has reported why
+      } else {
+        ok = page_values(pg, w, st, &base, &blen);
+        if (ok && part_lo == 0) {  // for parquet_values_kernel
+          pg.values = base;
+          pg.values_len = blen;
         }
-        if (!ok) raise_status(st, GFPDB_EUNSUPPORTED, 200000 + w);  // nulls, or bad levels
       }
       s_base = base;
       s_blen = blen;
       if (ok) {
-        if (part_lo == 0) {  // for parquet_values_kernel
-          pg.values = base;
-          pg.values_len = blen;
-        }
         // (a page walked or checked here has one part)
         const bool bytes_walk = pg.width == 0 && (pg.type == parquet::PAGE_DICTIONARY || pg.encoding == parquet::ENC_PLAIN);
         if (bytes_walk) {  // byte arrays: each value's address and length
@@ -345,8 +524,8 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
         ok = 0;
       }
       s_ok = indices ? ok : 0;
-      s_at = 1;
-      s_done = 0;
+      s_at = part.at;
+      s_done = part.done;
     }
     __syncthreads();
     if (!s_ok) continue;
@@ -371,14 +550,27 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
       dn = dp.num_values;
     }
     for (;;) {
+      // the next kPqWindow bytes: a header read from memory waits for the one
+      // before it, from shared memory it costs a tenth of that
+      const int32_t from = s_at;
+      const uintptr_t line = reinterpret_cast<uintptr_t>(base + from) & ~uintptr_t{15};
+      const int pad = static_cast<int>(reinterpret_cast<uintptr_t>(base + from) - line);
+      const int32_t to = blen - from < kPqWindow - pad ? blen : from + kPqWindow - pad;
+      if (threadIdx.x < kPqWindow / 16 && line + 16 * threadIdx.x < reinterpret_cast<uintptr_t>(base + to))
+        s_window[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(line) + threadIdx.x);
+      __syncthreads();
       if (threadIdx.x == 0) {
-        int32_t n = 0, at = s_at, done = s_done;
+        const uint8_t* const window = reinterpret_cast<const uint8_t*>(s_window) + pad;
+        int32_t n = 0, at = from, done = s_done;
         while (n < kPqRuns && done < part_hi) {
+          if (at + 9 > to && to < blen) break;  // a header or an RLE run may go past the window
           uint32_t h;
-          if (!run_header(base, blen, &at, &h)) {
+          int32_t head = 0;
+          if (!run_header(window + (at - from), to - at, &head, &h)) {
             s_ok = 0;
             break;
           }
+          at += head;
           int64_t count;
           if (h & 1) {
             const int64_t groups = h >> 1;
@@ -396,7 +588,7 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
               break;
             }
             uint32_t v = 0;
-            for (int k = 0; k < vb; ++k) v |= static_cast<uint32_t>(base[at + k]) << (8 * k);
+            for (int k = 0; k < vb; ++k) v |= static_cast<uint32_t>(window[at - from + k]) << (8 * k);
             at += vb;
             s_start[n] = -1;
             s_value[n] = v;
@@ -411,14 +603,14 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
           if (done > part_lo) ++n;  // a run wholly before the part is passed over
         }
         s_first[n] = done;
-        s_n = s_ok ? n : 0;
+        s_n = s_ok ? n : -1;
         s_at = at;
         s_done = done;
         if (!s_ok) raise_status(st, GFPDB_EINVAL, 500000 + w);
       }
       __syncthreads();
       const int32_t n = s_n;
-      if (n == 0) break;
+      if (n < 0) break;
       const int32_t v0 = s_first[0] > part_lo ? s_first[0] : part_lo, v1 = s_first[n] < part_hi ? s_first[n] : part_hi;
       // unrolled so that several values' loads are in flight together
 #pragma unroll 4
@@ -473,8 +665,9 @@ __global__ void __launch_bounds__(kPqThreads) parquet_pages_kernel(PageDev* page
 // blockIdx.y: a data page (index into `list`, whose first is the read's
 // first-th); values over x.
 __global__ void __launch_bounds__(256) parquet_values_kernel(const PageDev* pages, const int32_t* list, int32_t first,
-                                                             DictArrays dicts, DevStatus* st) {
+                                                             int32_t late, DictArrays dicts, DevStatus* st) {
   const PageDev& pg = pages[list[blockIdx.y]];
+  if ((pg.late_from != kPqNever) != (late != 0)) return;  // the read's other round has all its indices
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const bool dict = pg.encoding != parquet::ENC_PLAIN;
   const PageDev* dp = dict ? &pages[pg.dict_page] : nullptr;
@@ -527,28 +720,47 @@ constexpr int64_t kPqCopyGap = 64 * 1024;
 // stream alone. (72.6 MB, 4M rows: 558 us of copying and then decoding as one
 // batch, 496 us in batches.)
 constexpr int64_t kPqBatch = 8 << 20;
+// Steps that a batch's walk over a page's runs may take: runs of one length are
+// done before (a 1M-value page of 504-value runs takes 66).
+constexpr int32_t kPqWalkSteps = 256;
 
-// The copies' stream; nothing it started is left running when it goes.
+// Whether the file's bytes show that all of a page's indices lie in one run: its
+// parts then need no walk (a batch would wait about 8 us for it; a look at each
+// page of a file of small ones takes as long). Levels and compressed pages are
+// not looked into.
+bool one_run(const uint8_t* file, const parquet::PageInfo& pg) {
+  if (pg.codec != parquet::CODEC_UNCOMPRESSED || pg.v1_def_levels) return false;
+  const int64_t skip = pg.type == parquet::PAGE_DATA_V2 ? pg.v2_levels : 0;
+  uint64_t h = 0;
+  for (int k = 0; k < 5 && skip + 1 + k < pg.compressed; ++k) {
+    const uint8_t b = file[pg.data_offset + skip + 1 + k];
+    h |= static_cast<uint64_t>(b & 0x7f) << (7 * k);
+    if ((b & 0x80) == 0) return static_cast<int64_t>(h & 1 ? (h >> 1) * 8 : h >> 1) >= pg.num_values;
+  }
+  return false;
+}
+
+// The copies' stream, two batches ahead of the decoding; nothing it started is
+// left running when it goes.
 struct CopyStream {
   cudaStream_t s = nullptr;
-  cudaEvent_t ev = nullptr;
+  cudaEvent_t ev[2] = {nullptr, nullptr};  // behind the copies of the even and of the odd batches
   ~CopyStream() {
     if (s != nullptr) {
       (void)cudaStreamSynchronize(s);
       (void)cudaStreamDestroy(s);
     }
-    if (ev != nullptr) (void)cudaEventDestroy(ev);
+    for (cudaEvent_t e : ev)
+      if (e != nullptr) (void)cudaEventDestroy(e);
   }
   void open(cudaStream_t after) {
     GF_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    GF_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    order(after, s);
+    for (cudaEvent_t& e : ev) GF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    GF_CUDA(cudaEventRecord(ev[0], after));
+    GF_CUDA(cudaStreamWaitEvent(s, ev[0], 0));
   }
-  // `to` goes on after what `from` holds now.
-  void order(cudaStream_t from, cudaStream_t to) {
-    GF_CUDA(cudaEventRecord(ev, from));
-    GF_CUDA(cudaStreamWaitEvent(to, ev, 0));
-  }
+  void copied(size_t batch) { GF_CUDA(cudaEventRecord(ev[batch & 1], s)); }
+  void await(size_t batch, cudaStream_t by) { GF_CUDA(cudaStreamWaitEvent(by, ev[batch & 1], 0)); }
 };
 
 int grid_parquet(int64_t n) {
@@ -575,7 +787,7 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   };
   struct Batch {
     size_t chunk_end, span_end;              // its last chunk and span, plus one
-    size_t item_end = 0, snappy_end = 0, data_end = 0;  // the same in the lists below
+    size_t item_end = 0, walk_end = 0, snappy_end = 0, data_end = 0;  // the same in the lists below
     int64_t bytes = 0;
   };
   std::vector<Span> spans;
@@ -600,15 +812,17 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   auto arena = make_buffer(arena_bytes + 16, s);  // tail padding: 4-byte word reads past a value's end
   CopyStream copies;
   if (batches.size() > 1) copies.open(s);
-  size_t copied = 0;  // spans
-  auto copy_to = [&](size_t end) {
-    for (; copied < end; ++copied)
-      copy_h2d(arena->as<uint8_t>() + spans[copied].at, file + spans[copied].begin,
-               spans[copied].end - spans[copied].begin, copies.s != nullptr ? copies.s : s);
+  auto copy_batch = [&](size_t b) {
+    if (b >= batches.size()) return;
+    for (size_t k = b > 0 ? batches[b - 1].span_end : 0; k < batches[b].span_end; ++k)
+      copy_h2d(arena->as<uint8_t>() + spans[k].at, file + spans[k].begin, spans[k].end - spans[k].begin,
+               copies.s != nullptr ? copies.s : s);
+    if (copies.s != nullptr) copies.copied(b);
   };
   // the first copies run while the host lays the pages out; the others come
   // after the page descriptors, which would wait behind them
-  if (!batches.empty()) copy_to(batches[std::min<size_t>(1, batches.size() - 1)].span_end);
+  copy_batch(0);
+  copy_batch(1);
 
   // per-column outputs and working arrays
   std::vector<BufferPtr> fixed(nc), row_ptr(nc), row_len(nc), idx(nc);
@@ -628,12 +842,16 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
 
   // page descriptors
   std::vector<PageDev> pd(L.pages.size());
-  std::vector<int32_t> snappy_list, data_list, item_list;  // item_list: (page, first value) pairs
+  std::vector<int32_t> snappy_list, data_list, walk_list;
+  std::vector<PagePart> item_list;
   int64_t inflate_bytes = 0, dict_entries = 0;
   std::vector<int64_t> inflate_at(L.pages.size(), -1);
+  int32_t looked_at = -1;  // a chunk
+  bool walk = false;
   size_t batch = 0;  // pages come in the order of their chunks
   auto end_batch = [&] {
-    batches[batch].item_end = item_list.size() / 2;
+    batches[batch].item_end = item_list.size();
+    batches[batch].walk_end = walk_list.size();
     batches[batch].snappy_end = snappy_list.size();
     batches[batch].data_end = data_list.size();
     ++batch;
@@ -657,9 +875,20 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
     const bool fixed_dict = L.columns[pg.column].dtype != DType::Utf8 && pg.encoding != parquet::ENC_PLAIN;
     if (pg.type != parquet::PAGE_DICTIONARY && !fixed_dict) data_list.push_back(static_cast<int32_t>(p));
     const bool indices = pg.type != parquet::PAGE_DICTIONARY && pg.encoding != parquet::ENC_PLAIN;
-    for (int64_t first = 0; first == 0 || (indices && first < pg.num_values); first += kPqPart) {
-      item_list.push_back(static_cast<int32_t>(p));
-      item_list.push_back(static_cast<int32_t>(first));
+    pd[p].first_part = static_cast<int32_t>(item_list.size());
+    for (int64_t first = 0; first == 0 || (indices && first < pg.num_values); first += kPqPart)
+      item_list.push_back(PagePart{static_cast<int32_t>(p), static_cast<int32_t>(first), 1, 0});
+    if (item_list.size() > INT32_MAX) fail(GFPDB_EUNSUPPORTED, "a Parquet read of too many pages");
+    pd[p].n_parts = static_cast<int32_t>(item_list.size()) - pd[p].first_part;
+    if (pd[p].n_parts > 1) {  // a chunk's pages are walked or not by its first one
+      if (pg.chunk != looked_at) {
+        looked_at = pg.chunk;
+        walk = !one_run(file, pg);
+      }
+      if (walk) {
+        pd[p].walked = 1;
+        walk_list.push_back(static_cast<int32_t>(p));
+      }
     }
   }
   while (batch < batches.size()) end_batch();
@@ -669,7 +898,7 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
     const int c = pg.column;
     const bool v2 = pg.type == parquet::PAGE_DATA_V2;
     PageDev& d = pd[p];
-    std::memset(&d, 0, sizeof(d));
+    d.late_from = kPqNever;
     d.body = arena->as<uint8_t>() + chunk_at[pg.chunk] + (pg.data_offset - L.chunks[pg.chunk].begin);
     d.body_len = pg.compressed;
     d.snappy = inflate_at[p] >= 0 ? 1 : 0;
@@ -704,56 +933,87 @@ TupleSetPtr parquet_read(const uint8_t* file, int64_t size, const std::vector<st
   DevStatus* st = status->as<DevStatus>();
   const int64_t np = static_cast<int64_t>(pd.size());
   auto pages_dev = make_buffer((np > 0 ? np : 1) * static_cast<int64_t>(sizeof(PageDev)), s);
-  std::vector<int32_t> all_lists(item_list);
-  all_lists.insert(all_lists.end(), snappy_list.begin(), snappy_list.end());
-  all_lists.insert(all_lists.end(), data_list.begin(), data_list.end());
-  const int64_t nl = static_cast<int64_t>(all_lists.size());
-  auto lists = make_buffer((nl > 0 ? nl : 1) * 4, s);
+  // the parts, then the lists of pages to walk, to inflate and to copy values of
+  const size_t item_bytes = item_list.size() * sizeof(PagePart);
+  std::vector<char> lists_host(item_bytes + (walk_list.size() + snappy_list.size() + data_list.size()) * 4);
+  {
+    char* to = lists_host.data();
+    auto append = [&](const void* from, size_t bytes) {
+      if (bytes > 0) std::memcpy(to, from, bytes);
+      to += bytes;
+    };
+    append(item_list.data(), item_bytes);
+    append(walk_list.data(), walk_list.size() * 4);
+    append(snappy_list.data(), snappy_list.size() * 4);
+    append(data_list.data(), data_list.size() * 4);
+  }
+  auto lists = make_buffer(static_cast<int64_t>(lists_host.size()) + 16, s);
+  PagePart* items = lists->as<PagePart>();
+  int32_t* walk_dev = reinterpret_cast<int32_t*>(lists->as<char>() + item_bytes);
   if (np > 0) GF_CUDA(cudaMemcpyAsync(pages_dev->data(), pd.data(), np * sizeof(PageDev), cudaMemcpyHostToDevice, s));
-  if (nl > 0) GF_CUDA(cudaMemcpyAsync(lists->data(), all_lists.data(), nl * 4, cudaMemcpyHostToDevice, s));
+  if (!lists_host.empty())
+    GF_CUDA(cudaMemcpyAsync(items, lists_host.data(), lists_host.size(), cudaMemcpyHostToDevice, s));
   PageDev* pages = pages_dev->as<PageDev>();
-  const int32_t* snappy_dev = lists->as<int32_t>() + item_list.size();
+  const int32_t* snappy_dev = walk_dev + walk_list.size();
   const int32_t* data_dev = snappy_dev + snappy_list.size();
 
-  const PagePart* items = lists->as<PagePart>();
-  Batch from{};
-  for (const Batch& b : batches) {
-    copy_to(b.span_end);
-    if (copies.s != nullptr) copies.order(copies.s, s);
-    if (b.snappy_end > from.snappy_end) {
-      const int64_t n = static_cast<int64_t>(b.snappy_end - from.snappy_end);
-      ProfScope prof("parquet_snappy_kernel", s);
-      parquet_snappy_kernel<<<grid_parquet(n * 32), 256, 0, s>>>(pages, snappy_dev + from.snappy_end,
-                                                                 static_cast<int32_t>(n), st);
-      after_launch("parquet_snappy_kernel");
-      double bytes = 0;
-      for (size_t k = from.snappy_end; k < b.snappy_end; ++k) bytes += pd[snappy_list[k]].inflated_len;
-      prof.stop(bytes);
+  // the walks, parts and values of the pages of batches (from, to]
+  auto decode = [&](const Batch& from, const Batch& to, bool late) {
+    if (to.walk_end > from.walk_end) {
+      const int64_t n = static_cast<int64_t>(to.walk_end - from.walk_end), most = static_cast<int64_t>(num_sms()) * 16;
+      ProfScope prof("parquet_runs_kernel", s);
+      parquet_runs_kernel<<<static_cast<int>(std::min((n + 3) / 4, most)), 128, 0, s>>>(
+          pages, walk_dev + from.walk_end, static_cast<int32_t>(n), items, late ? -1 : kPqWalkSteps, late ? 1 : 0, st);
+      after_launch("parquet_runs_kernel");
+      prof.stop(0.0);
     }
-    if (b.item_end > from.item_end) {
+    if (to.item_end > from.item_end) {
       ProfScope prof("parquet_pages_kernel", s);
-      const int64_t n = static_cast<int64_t>(b.item_end - from.item_end), most = static_cast<int64_t>(num_sms()) * 8;
+      const int64_t n = static_cast<int64_t>(to.item_end - from.item_end), most = static_cast<int64_t>(num_sms()) * 8;
       parquet_pages_kernel<<<static_cast<int>(std::min(n, most)), kPqThreads, 0, s>>>(
-          pages, static_cast<int32_t>(np), items + from.item_end, n, dicts, st);
+          pages, static_cast<int32_t>(np), items + from.item_end, n, late ? 1 : 0, dicts, st);
       after_launch("parquet_pages_kernel");
       prof.stop(0.0);
     }
     // each data page's values over up to 64 blocks of 256 threads
     int64_t most = 0;
-    for (size_t k = from.data_end; k < b.data_end; ++k) most = std::max<int64_t>(most, L.pages[data_list[k]].num_values);
+    for (size_t k = from.data_end; k < to.data_end; ++k) most = std::max<int64_t>(most, L.pages[data_list[k]].num_values);
     const int gx = static_cast<int>(std::min<int64_t>(64, std::max<int64_t>(1, (most + 255) / 256)));
-    for (size_t at = from.data_end; at < b.data_end; at += 65535) {  // grid y limit
-      const int gy = static_cast<int>(std::min<size_t>(65535, b.data_end - at));
+    for (size_t at = from.data_end; at < to.data_end; at += 65535) {  // grid y limit
+      const int gy = static_cast<int>(std::min<size_t>(65535, to.data_end - at));
       ProfScope prof("parquet_values_kernel", s);
-      parquet_values_kernel<<<dim3(gx, gy), 256, 0, s>>>(pages, data_dev + at, static_cast<int32_t>(at), dicts, st);
+      parquet_values_kernel<<<dim3(gx, gy), 256, 0, s>>>(pages, data_dev + at, static_cast<int32_t>(at), late ? 1 : 0,
+                                                         dicts, st);
       after_launch("parquet_values_kernel");
       prof.stop(0.0);
     }
-    from = b;
+  };
+  Batch from{};
+  for (size_t b = 0; b < batches.size(); ++b) {
+    const Batch& to = batches[b];
+    if (copies.s != nullptr) copies.await(b, s);
+    if (to.snappy_end > from.snappy_end) {
+      const int64_t n = static_cast<int64_t>(to.snappy_end - from.snappy_end);
+      ProfScope prof("parquet_snappy_kernel", s);
+      parquet_snappy_kernel<<<grid_parquet(n * 32), 256, 0, s>>>(pages, snappy_dev + from.snappy_end,
+                                                                 static_cast<int32_t>(n), st);
+      after_launch("parquet_snappy_kernel");
+      double bytes = 0;
+      for (size_t k = from.snappy_end; k < to.snappy_end; ++k) bytes += pd[snappy_list[k]].inflated_len;
+      prof.stop(bytes);
+    }
+    decode(from, to, false);
+    copy_batch(b + 2);
+    from = to;
   }
   DevStatus h;
   GF_CUDA(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
   sync(s);
+  if (h.code == 0 && h.aux[0] != 0) {  // a batch's walks were cut short: the second round
+    decode(Batch{}, batches.back(), true);
+    GF_CUDA(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
+    sync(s);
+  }
   if (h.code != 0)
     fail(h.code, std::string(h.code == GFPDB_EUNSUPPORTED ? "Parquet column with nulls (definition levels)"
                                                          : "malformed Parquet page data") +
