@@ -898,6 +898,7 @@ struct SBShared {
   uint32_t st_range[kSBFastStaged];
   int32_t st_keys[kSBFastStaged], st_tab[kSBFastStaged];
   int32_t nst, ngl, nhash;
+  int32_t group_u[2];  // group column g's dimension is the one that step (2) looks up u-th (-1: another)
 };
 
 // A warp's stacks of rows: after the staged dimensions, and after all.
@@ -907,6 +908,7 @@ struct SBStacks {
   M m2[kSBStack2];
   uint32_t row1[kSBStack1];
   uint32_t row2[kSBStack2];
+  uint32_t idx2[kSBRingDims][kSBStack2];  // the row's place in each dimension that step (2) looks up
   uint8_t part1[kSBStack1];
   uint8_t part2[kSBStack2];
 };
@@ -937,11 +939,17 @@ __device__ __noinline__ M sb_extra_lookups(const SBFactParams& p, const SBShared
   return m;
 }
 
-// The value of group column g for a row that every dimension selects.
-__device__ __forceinline__ uint32_t sb_group_value(const SBFactParams& p, const SBShared& sh, const DevCol* cols,
-                                                   int64_t row, int g) {
+// The value of group column g for the row at `e` of the second stack, which
+// every dimension selects. Its place in a dimension of step (2) comes along on
+// the stack: that foreign key may lie in host memory, and a second read of it
+// took 3% more bytes over the link (247 MB against 241 for 32 queries over 16
+// partitions) and a sector of device memory a row.
+template <typename M>
+__device__ __forceinline__ uint32_t sb_group_value(const SBFactParams& p, const SBShared& sh, const SBStacks<M>& R, int e,
+                                                   const DevCol* cols, int64_t row, int g) {
   const int d = p.fd.group_dim[g], c = p.fd.group_idx[g];
   const SBDimDev& D = p.dims[d];
+  if (sh.group_u[g] >= 0) return static_cast<uint32_t>(__ldg(D.dg[c] + R.idx2[sh.group_u[g]][e]));
   const int64_t key = load_int(cols[p.fd.fk_col[d]], row);
   if (sh.range[d] != 0)
     return static_cast<uint32_t>(__ldg(D.dg[c] + (static_cast<uint64_t>(key) - static_cast<uint64_t>(sh.kmin[d]))));
@@ -970,8 +978,8 @@ __device__ __forceinline__ void sb_direct_groups(const SBFactParams& p, const SB
       vals[a] = x;
     }
   }
-  const uint32_t g0 = p.fd.n_group > 0 ? sb_group_value(p, sh, cols, row, 0) : 0;
-  const uint32_t g1 = p.fd.n_group > 1 ? sb_group_value(p, sh, cols, row, 1) : 0;
+  const uint32_t g0 = p.fd.n_group > 0 ? sb_group_value<M>(p, sh, R, base + lane, cols, row, 0) : 0;
+  const uint32_t g1 = p.fd.n_group > 1 ? sb_group_value<M>(p, sh, R, base + lane, cols, row, 1) : 0;
   const uint64_t slot = sb_group_slot(p, sb_group_key(p.fd.n_group, g0, g1));
   if (slot == UINT64_MAX) return;
   // a query's bit is set once and stays: an old value that shows it is enough
@@ -1002,13 +1010,16 @@ __device__ __forceinline__ void sb_direct_probe(const SBFactParams& p, const SBS
   }
   const DevCol* cols = p.part_cols + static_cast<int64_t>(part) * p.n_cols;
   M q[kSBRingDims];
+  uint32_t at[kSBRingDims];
 #pragma unroll
   for (int u = 0; u < kSBRingDims; ++u) {
     q[u] = u < ndirect ? M(0) : ~M(0);
+    at[u] = 0;
     if (u >= ndirect || m == 0) continue;
     const SBShared::Global& G = sh.gl[u];
     const int32_t fk = __ldg(static_cast<const int32_t*>(cols[G.col].data) + row);
     const uint64_t idx = static_cast<uint64_t>(static_cast<int64_t>(fk) - G.kmin);
+    at[u] = static_cast<uint32_t>(idx);
     if (idx < G.range)
       q[u] = sizeof(M) == 4 ? static_cast<M>(__ldg(reinterpret_cast<const unsigned*>(G.dq) + 2 * idx))
                             : static_cast<M>(__ldg(reinterpret_cast<const unsigned long long*>(G.dq) + idx));
@@ -1021,6 +1032,8 @@ __device__ __forceinline__ void sb_direct_probe(const SBFactParams& p, const SBS
     R.m2[e] = m;
     R.row2[e] = row;
     R.part2[e] = static_cast<uint8_t>(part);
+#pragma unroll
+    for (int u = 0; u < kSBRingDims; ++u) R.idx2[u][e] = at[u];
   }
   t2 += __popc(b);
   __syncwarp();  // also: the first stack's rows are read
@@ -1074,6 +1087,11 @@ __global__ void __launch_bounds__(kSBDirectThreads, kSBDirectBlocks)
       } else {
         ++nh;
       }
+    }
+    for (int g = 0; g < 2; ++g) {
+      sh.group_u[g] = -1;
+      for (int u = 0; u < ngl && u < kSBRingDims; ++u)
+        if (g < p.fd.n_group && sh.gl[u].d == p.fd.group_dim[g]) sh.group_u[g] = u;
     }
     sh.nst = nst;
     sh.ngl = ngl;
@@ -1842,7 +1860,9 @@ void StarBatchState::prepare(cudaStream_t s) {
       in_place[c] = 1;
       if (fk) {
         ++n_in_place_fk;
-        for (const auto& g : spec.group) n_in_place_group_fk += fk_slot[g.dim] == c ? 1 : 0;  // read again for its group
+// more dimensions than step (2) carries: a group's key may be read again
+        if (nd - n_staged > kSBRingDims)
+          for (const auto& g : spec.group) n_in_place_group_fk += fk_slot[g.dim] == c ? 1 : 0;
       } else {
         ++n_in_place_measures;
       }
