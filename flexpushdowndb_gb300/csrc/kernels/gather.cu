@@ -209,37 +209,84 @@ struct DeviceCopyParams {
   int32_t n;
 };
 
-// The whole grid takes one copy after another, 16 bytes a load where both
-// ends are 16-byte aligned, four loads in flight per thread. Columns of 8 to
-// 16 MB: 80 MB of traffic in about 17 us, against 33 us as four copies by
-// cudaMemcpyAsync.
+// Bytes that the source lies behind the target modulo 16.
+__host__ __device__ __forceinline__ unsigned copy_offset(const DeviceCopy& c) {
+  return static_cast<unsigned>(reinterpret_cast<uintptr_t>(c.src) - reinterpret_cast<uintptr_t>(c.dst)) & 15u;
+}
+
+// Lines [t, n) of 16 bytes at dst, every `stride`-th, each from the two aligned
+// source lines that hold its bytes: line i's begin kWord words and `shift` bits
+// behind src16[i].
+template <int kWord>
+__device__ __forceinline__ void copy_shifted(const uint4* src16, uint4* dst, int64_t t, int64_t n, int64_t stride,
+                                             unsigned shift) {
+  constexpr int kU = 4;
+  for (int64_t i = t; i < n; i += kU * stride) {
+    uint4 lo[kU], hi[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (i + u * stride < n) {
+        lo[u] = __ldg(src16 + i + u * stride);
+        hi[u] = __ldg(src16 + i + u * stride + 1);
+      }
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (i + u * stride < n) {
+        const uint32_t w[8] = {lo[u].x, lo[u].y, lo[u].z, lo[u].w, hi[u].x, hi[u].y, hi[u].z, hi[u].w};
+        dst[i + u * stride] = make_uint4(
+            __funnelshift_r(w[kWord], w[kWord + 1], shift), __funnelshift_r(w[kWord + 1], w[kWord + 2], shift),
+            __funnelshift_r(w[kWord + 2], w[kWord + 3], shift), __funnelshift_r(w[kWord + 3], w[kWord + 4], shift));
+      }
+  }
+}
+
+// The whole grid takes one copy after another, 16 bytes a store. kShifted
+// false: the copies whose ends are 16-byte aligned alike, one load a store and
+// four in flight per thread. Columns of 8 to 16 MB: 80 MB of traffic in about
+// 17 us, against 33 us as four copies by cudaMemcpyAsync. True: the others, each
+// line from the two aligned ones around its bytes; 20M int64 values 8 bytes
+// apart from alignment 73 us the call (70 by cudaMemcpyAsync, 155 in 4-byte
+// words), as many int32 values 47 (46 and 88). Apart, because the second
+// needs twice the registers (aligned columns 46 us for 42 in one kernel).
+template <bool kShifted>
 __global__ void __launch_bounds__(256) copy_device_kernel(const __grid_constant__ DeviceCopyParams p) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   for (int k = 0; k < p.n; ++k) {
     const DeviceCopy& c = p.c[k];
-    const bool vec = ((reinterpret_cast<uintptr_t>(c.src) | reinterpret_cast<uintptr_t>(c.dst)) & 15u) == 0;
-    const int64_t n16 = vec ? c.bytes / 16 : 0;
-    const uint4* s4 = static_cast<const uint4*>(c.src);
-    uint4* d4 = static_cast<uint4*>(c.dst);
-    int64_t i = t;
-    for (; i + 3 * stride < n16; i += 4 * stride) {
-      const uint4 a = __ldcs(s4 + i), b = __ldcs(s4 + i + stride), x = __ldcs(s4 + i + 2 * stride),
-                  y = __ldcs(s4 + i + 3 * stride);
-      d4[i] = a;
-      d4[i + stride] = b;
-      d4[i + 2 * stride] = x;
-      d4[i + 3 * stride] = y;
+    const char* src = static_cast<const char*>(c.src);
+    char* dst = static_cast<char*>(c.dst);
+    // whole lines of dst [head, head + 16 n), all of whose source lines lie
+    // within the source; the bytes around them one by one
+    int64_t head = (16 - (reinterpret_cast<uintptr_t>(dst) & 15u)) & 15u;
+    const unsigned off = kShifted ? copy_offset(c) : 0;
+    if (kShifted && head < off) head += 16;  // its first line begins `off` bytes before
+    int64_t n = (c.bytes - head - (kShifted ? 16 - off : 0)) / 16;
+    if (c.bytes < head + 32) head = n = 0;
+    uint4* const d = reinterpret_cast<uint4*>(dst + head);
+    const uint4* const s4 = reinterpret_cast<const uint4*>(src + head - off);
+    if (kShifted) {
+      const unsigned shift = 8 * (off & 3u);
+      switch (off >> 2) {
+        case 0: copy_shifted<0>(s4, d, t, n, stride, shift); break;
+        case 1: copy_shifted<1>(s4, d, t, n, stride, shift); break;
+        case 2: copy_shifted<2>(s4, d, t, n, stride, shift); break;
+        default: copy_shifted<3>(s4, d, t, n, stride, shift); break;
+      }
+    } else {
+      int64_t i = t;
+      for (; i + 3 * stride < n; i += 4 * stride) {
+        const uint4 a = __ldcs(s4 + i), b = __ldcs(s4 + i + stride), x = __ldcs(s4 + i + 2 * stride),
+                    y = __ldcs(s4 + i + 3 * stride);
+        d[i] = a;
+        d[i + stride] = b;
+        d[i + 2 * stride] = x;
+        d[i + 3 * stride] = y;
+      }
+      for (; i < n; i += stride) d[i] = __ldcs(s4 + i);
     }
-    for (; i < n16; i += stride) d4[i] = __ldcs(s4 + i);
-    const bool words = ((reinterpret_cast<uintptr_t>(c.src) | reinterpret_cast<uintptr_t>(c.dst)) & 3u) == 0;
-    const int64_t n4 = words ? c.bytes / 4 : 0;
-    const uint32_t* s1 = static_cast<const uint32_t*>(c.src);
-    uint32_t* d1 = static_cast<uint32_t*>(c.dst);
-    for (int64_t j = n16 * 4 + t; j < n4; j += stride) d1[j] = s1[j];
-    const char* s0 = static_cast<const char*>(c.src);
-    char* d0 = static_cast<char*>(c.dst);
-    for (int64_t j = n4 * 4 + t; j < c.bytes; j += stride) d0[j] = s0[j];
+    for (int64_t j = t; j < head; j += stride) dst[j] = src[j];
+    for (int64_t j = head + 16 * n + t; j < c.bytes; j += stride) dst[j] = src[j];
   }
 }
 
@@ -292,18 +339,25 @@ void copy_h2d(void* dst, const void* src, int64_t bytes, cudaStream_t s) {
 }
 
 void copy_device(const std::vector<DeviceCopy>& copies, cudaStream_t s) {
-  for (size_t at = 0; at < copies.size(); at += kDeviceCopies) {
+  for (const bool shifted : {false, true}) {
     DeviceCopyParams p;
-    p.n = static_cast<int32_t>(std::min(copies.size() - at, static_cast<size_t>(kDeviceCopies)));
+    p.n = 0;
     int64_t most = 0;
-    for (int i = 0; i < p.n; ++i) {
-      p.c[i] = copies[at + i];
-      most = std::max(most, p.c[i].bytes);
+    auto launch = [&] {
+      if (p.n == 0) return;
+      const int64_t blocks = std::min<int64_t>((most / 16 + 1023) / 1024, static_cast<int64_t>(num_sms()) * 8);
+      (shifted ? copy_device_kernel<true> : copy_device_kernel<false>)<<<static_cast<int>(blocks > 0 ? blocks : 1), 256, 0, s>>>(p);
+      after_launch("copy_device_kernel");
+      p.n = 0;
+      most = 0;
+    };
+    for (const DeviceCopy& c : copies) {
+      if (c.bytes <= 0 || (copy_offset(c) != 0) != shifted) continue;
+      p.c[p.n++] = c;
+      most = std::max(most, c.bytes);
+      if (p.n == kDeviceCopies) launch();
     }
-    if (most <= 0) continue;
-    const int64_t blocks = std::min<int64_t>((most / 16 + 1023) / 1024, static_cast<int64_t>(num_sms()) * 8);
-    copy_device_kernel<<<static_cast<int>(blocks > 0 ? blocks : 1), 256, 0, s>>>(p);
-    after_launch("copy_device_kernel");
+    launch();
   }
 }
 
