@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kScanThreads)
     int64_t total;
     const int64_t excl = block_exclusive_sum<kScanThreads>(sum, &total, s_warp);
     if (threadIdx.x < 32) {
-      uint64_t b = lookback_exclusive(tile_status, tile, static_cast<uint64_t>(total), st);
+      uint64_t b = lookback_exclusive<4>(tile_status, tile, static_cast<uint64_t>(total), st);
       if (threadIdx.x == 0) s_base = b;
     }
     __syncthreads();

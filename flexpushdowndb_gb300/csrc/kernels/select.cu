@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(const __grid_consta
     int tile_total;
     const int excl = block_exclusive_sum<kSelThreads>(cnt, &tile_total, s_warp);
     if (threadIdx.x < 32) {
-      const uint64_t b = lookback_exclusive(p.tile_status, tile, static_cast<uint64_t>(tile_total), p.status);
+      const uint64_t b = lookback_exclusive<1>(p.tile_status, tile, static_cast<uint64_t>(tile_total), p.status);
       if (threadIdx.x == 0) s_base = b;
     }
     __syncthreads();
@@ -1106,7 +1106,7 @@ __global__ void __launch_bounds__(kLiteThreads) select_lite_kernel(const __grid_
     int tile_total;
     const int excl = block_exclusive_sum<kLiteThreads>(cnt, &tile_total, s_warp);
     if (threadIdx.x < 32) {
-      const uint64_t b = lookback_exclusive(p.tile_status, tile, static_cast<uint64_t>(tile_total), p.status);
+      const uint64_t b = lookback_exclusive<1>(p.tile_status, tile, static_cast<uint64_t>(tile_total), p.status);
       if (threadIdx.x == 0) s_base = b;
     }
     __syncthreads();
