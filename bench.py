@@ -738,8 +738,8 @@ def _operator_case(args):
         prof = _kernel_profile(_abi.lib(), _abi, fn, args.steps)
         kern = {k: v["ms"] / args.steps for k, v in prof.items()}
         ms = sum(kern.get(k, 0.0) for k in ("shuffle_count_kernel", "shuffle_scan_kernel", "shuffle_scatter_kernel"))
-        # the key and 8 B for the slots, every column read and written once
-        algo = n * (8 + 8 + 2 * (8 + 8 + 4))
+        # the key, a 2-byte slot written and read, every column read and written once
+        algo = n * (8 + 4 + 2 * (8 + 8 + 4))
         print(json.dumps({"case": "shuffle", "rows": n, "slots": args.slots, "kernels_ms": kern, "shuffle_ms": ms,
                           "algorithmic_gbs": algo / (ms * 1e6), "rows_per_s": n / (ms * 1e-3)}))
         return
