@@ -426,6 +426,8 @@ Layout read_layout(const uint8_t* file, int64_t size, const std::vector<std::str
         pg.encoding = h.encoding;
         if (h.compressed < 0 || h.uncompressed < 0 || pg.data_offset + h.compressed > end)
           fail(GFPDB_EINVAL, "Parquet page of '" + c.name + "' runs past its column chunk");
+        if (h.num_values < 0 || h.def_len < 0)
+          fail(GFPDB_EINVAL, "Parquet page of '" + c.name + "' with a negative count");
         pos = pg.data_offset + h.compressed;
         if (h.type == PAGE_INDEX) continue;
         if (h.type == PAGE_DICTIONARY) {
@@ -448,7 +450,8 @@ Layout read_layout(const uint8_t* file, int64_t size, const std::vector<std::str
           if (h.rep_len != 0) fail(GFPDB_EUNSUPPORTED, "repeated Parquet column '" + c.name + "'");
           pg.v2_levels = h.def_len;
           pg.v2_compressed = h.v2_compressed;
-          if (h.def_len > h.compressed) fail(GFPDB_EINVAL, "Parquet page levels exceed the page");
+          if (h.def_len > h.compressed || h.def_len > h.uncompressed)
+            fail(GFPDB_EINVAL, "Parquet page levels exceed the page");
         } else {
           pg.v1_def_levels = c.repetition == 1;
         }
