@@ -862,16 +862,19 @@ __global__ void __launch_bounds__(kSBFactThreads, 3) sb_fact_kernel(const __grid
 //  (2) 32 stacked rows at a time, the direct dimensions in global memory;
 //      survivors go to the second stack;
 //  (3) 32 at a time, the group columns' values (looked up here, for the few
-//      rows that come this far, and not carried along), the group slot, the
-//      measures and the atomic adds.
+//      rows that come this far; what comes along is the row's place in a
+//      dimension of step (2)), the group slot, the measures and the atomic
+//      adds.
 // Stacks, not rings: rows are taken from the top, in no particular order.
 //
-// 59,952,713 rows, 32 queries: 266 us and 76 instructions per 32 rows (369 us
-// and 124 with class bytes for every dimension and the group values looked up
-// and carried in step 1), 69% of the measured copy bandwidth over the 1.24 GB
-// it moves; the wait left is for loads, with 32 warps an SM. Measured slower:
-// the next slice's keys read ahead (275 us, spills), and step (2) done in
-// place without a stack (321 us).
+// 59,952,713 rows, 32 queries: by their ranges 266 (76 instructions per 32
+// rows) to 351 us (the benchmark's queries, 91 instructions; 0.40 of the measured
+// copy bandwidth over the 0.96 GB of keys, 0.55 over the 1.3 GB it moves). The
+// first took 369 us and 124 instructions with class bytes for every dimension
+// and the group values looked up and carried in step 1. The wait left is for
+// loads, with 32 warps an SM. Measured slower, where this took 266: the next
+// slice's keys read ahead (275 us, spills), and step (2) done in place without a
+// stack (321 us).
 constexpr int kSBDirectWarps = 16;
 constexpr int kSBDirectThreads = kSBDirectWarps * 32;
 constexpr int kSBDirectBlocks = 2;  // blocks an SM's registers hold
